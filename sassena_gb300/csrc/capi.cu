@@ -202,6 +202,8 @@ int autotune_engine(std::string& m, Engine& eng, const EngineConfig& base, const
             // the shape the engine resolved (an automatic shape depends on the items, so a
             // choice made on a representative subset must name the shape it timed)
             best.shape = eng.stats().shape;
+            // FP64 form: the automatic choice is the fixed-point kernel, which has no tile shape
+            if (c.precision == PREC_FP64 && !c.shape.q_per_lane) best.shape = PhaseShape{0, 0, 0};
             best.split_atoms = c.split_atoms;
             best.rec_k = c.rec_k;
             any = true;
@@ -231,7 +233,10 @@ int autotune_engine(std::string& m, Engine& eng, const EngineConfig& base, const
             if (eng.prepare(c, items, err) == SASS_OK) all_rec = eng.stats().phase_tiles == 0;
         }
     }
-    std::vector<PhaseShape> shapes = all_rec ? std::vector<PhaseShape>{PhaseShape{0, 0, 0}} : phase_shapes(base.precision);
+    std::vector<PhaseShape> shapes;
+    if (all_rec || base.precision == PREC_FP64) shapes.push_back(PhaseShape{0, 0, 0});
+    if (!all_rec)
+        for (const PhaseShape& sh : phase_shapes(base.precision)) shapes.push_back(sh);
     for (const PhaseShape& sh : shapes)
         for (int sp : {0, 2048, 8192}) {
             EngineConfig c = base;

@@ -416,6 +416,47 @@ cudaError_t launch_long_means(const CorrChunk* chunks, int nchunks, const double
     return cudaGetLastError();
 }
 
+// The last kTail lags of a coherent FP64 shell, summed directly: there the 1/(NF - tau)
+// normalisation multiplies the transforms' rounding by up to NF (30,000 frames: 4e-13 of
+// S(q,0) at the last lag), while a lag has only NF - tau products per series.
+constexpr int kTail = 8;
+__global__ void __launch_bounds__(256) long_tail_kernel(LongFinal a) {
+    const FinalEntry e = a.entries[blockIdx.x];
+    const int nf = e.nf, v1 = a.shell_v[blockIdx.x + 1];
+    double2 acc[kTail];  // acc[k]: lag nf - 1 - k, k + 1 products
+#pragma unroll
+    for (int k = 0; k < kTail; ++k) acc[k] = make_double2(0.0, 0.0);
+    for (int v = a.shell_v[blockIdx.x] + (int)threadIdx.x; v < v1; v += 256) {
+        const double2* s = a.A + (size_t)v * nf;
+        double2 x[kTail], y[kTail];
+#pragma unroll
+        for (int k = 0; k < kTail; ++k) {
+            x[k] = s[k];
+            y[k] = s[nf - kTail + k];
+        }
+#pragma unroll
+        for (int k = 0; k < kTail; ++k)
+#pragma unroll
+            for (int t = 0; t <= k; ++t) acc[k] = cadd(acc[k], cmulc(y[kTail - 1 - k + t], x[t]));
+    }
+    __shared__ double2 part[8][kTail];
+#pragma unroll
+    for (int k = 0; k < kTail; ++k) {
+        for (int o = 16; o; o >>= 1) {
+            acc[k].x += __shfl_down_sync(0xffffffffu, acc[k].x, o);
+            acc[k].y += __shfl_down_sync(0xffffffffu, acc[k].y, o);
+        }
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][k] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < kTail) {
+        double2 z = part[0][threadIdx.x];
+        for (int w = 1; w < 8; ++w) z = cadd(z, part[w][threadIdx.x]);
+        const double f = e.inv_nm / (double)(threadIdx.x + 1);
+        e.fqt[nf - 1 - threadIdx.x] = make_double2(z.x * f, (a.conj_out ? -z.y : z.y) * f);
+    }
+}
+
 cudaError_t launch_long_finalize(const LongFinal& a, cudaStream_t st) {
     if (a.nentries == 0) return cudaSuccess;
     if (!long_ok(a.lg)) return cudaErrorInvalidValue;
@@ -435,7 +476,11 @@ cudaError_t launch_long_finalize(const LongFinal& a, cudaStream_t st) {
         long_final_cols_kernel<<<dim3(kLongC / kLongTile, (unsigned)b.nentries), kLongNT, sm_cols, st>>>(b);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    return cudaSuccess;
+    if (a.A) {
+        long_tail_kernel<<<(unsigned)a.nentries, 256, 0, st>>>(a);
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 cudaError_t launch_to_ff2(const double2* src, size_t n, void* dst, cudaStream_t st) {

@@ -469,7 +469,7 @@ int ensure_rec_layout(SystemState& s, std::string& err) {
 void Engine::release() {
     key_.clear();
     DevBuf* bufs[] = {&blob_,    &bfac_, &amp_, &part_,  &ppart_, &apart_,
-                      &a2part_, &counter_, &err_, &tw64_, &tw32_, &rec_bfac_};
+                      &a2part_, &counter_, &err_, &tw64_, &tw32_, &rec_bfac_, &fxtab_, &fxq_};
     for (DevBuf* b : bufs) b->release();
     hblob_.release();
 }
@@ -512,6 +512,7 @@ static std::vector<uint64_t> prepare_key(const EngineConfig& c, const std::vecto
             p(s.xyz.p);
             p(s.xyz_rec.p);
             p(s.block_class.p);
+            p(s.rec_map.p);
             p(s.cls.p);
             u(s.na_rec);
         }
@@ -641,11 +642,30 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     stats_.rec_k = rec_k_;
     stats_.rec_groups = rgroups.size();
 
+    // ---- FP64 form: the fixed-point phase sum, unless an explicit tile shape asks for the FP64
+    // kernel (or the classes are so many that padding each to 32 atoms would cost more than
+    // it gives: 27 times faster per atom, measured)
+    fx_on_.assign(items.size(), 0);
+    for (size_t i = 0; !f32 && coherent && !cfg.shape.q_per_lane && i < items.size(); ++i) {
+        SystemState& s = *items[i].sys;
+        if (items[i].d_amp_given || s.nclass > 65535) continue;
+        if (!s.rec_map_ok) {
+            const int rc = build_rec_map(s, err);
+            if (rc) return rc;
+        }
+        fx_on_[i] = s.na_rec <= 8 * s.na_pad;
+    }
+
     // atom splits: enough tiles for the persistent grid to balance
     nsplit_.assign(items.size(), 1);
     size_t base_tiles = 0;
+    size_t fx_units = 0;  // warp tiles of the fixed-point kernel without splits
     for (size_t i = 0; i < items.size(); ++i) {
         const WorkItem& it = items[i];
+        if (fx_on_[i]) {
+            fx_units += (it.offs.back() + 31) / 32 * it.sys->nf;
+            continue;
+        }
         size_t groups = 0;
         for (size_t s = 0; s + 1 < it.offs.size(); ++s)
             if (!is_rec(i, s))
@@ -658,7 +678,13 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         int max_split = (int)(items[i].sys->na_pad / shape.atoms);
         if (item_ng[i]) max_split = std::min(max_split, (int)(items[i].sys->na_rec / 128));
         int ns = 1;
-        if (cfg.split_atoms > 0) {
+        if (fx_on_[i]) {
+            // a warp tile runs on its own: split until there are about four for each of the
+            // 24 warps of an SM, with at least 4 blocks of 32 atoms in a slice
+            max_split = std::max(1, (int)(items[i].sys->na_rec / 128));
+            if (cfg.split_atoms > 0) ns = (int)((items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms);
+            else ns = (int)std::min<size_t>(64, ((size_t)sms * 96 + fx_units - 1) / std::max<size_t>(fx_units, 1));
+        } else if (cfg.split_atoms > 0) {
             ns = (int)((items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms);
         } else if (base_tiles < target) {
             ns = (int)((target + base_tiles - 1) / std::max<size_t>(base_tiles, 1));
@@ -793,7 +819,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
             const long long nst = (long long)(s.na_pad / shape.atoms), ns = nsplit_[i];
             // frame tiles outermost: the tiles that read the same frames run together, so
             // the coordinates stream from HBM about once and the other reads hit L2
-            for (size_t f0 = 0; f0 < s.nf; f0 += shape.warps)
+            for (size_t f0 = 0; f0 < s.nf && !fx_on_[i]; f0 += shape.warps)
                 for (size_t sh = 0; sh < nq; ++sh) {
                     if (is_rec(i, sh)) continue;
                     for (size_t v = it.offs[sh]; v < it.offs[sh + 1]; v += per)
@@ -883,6 +909,60 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     nrec_tiles_ = (int)rtiles.size();
     nrec_groups_ = (int)rgroups.size();
     if (nrec_groups_) ECK(rec_bfac_.ensure((size_t)nrec_groups_ * kRecMaxClass * rec_k_ * sizeof(float)));
+
+    // fixed-point tiles: 32 sub-vectors x 8 frames x atom slice, frames outermost (L2 reuse)
+    std::vector<FxSystem> fsys(items.size());
+    std::vector<FxTileDesc> ftiles;
+    fxq_off_.assign(items.size(), 0);
+    size_t fxq_total = 0;
+    for (size_t i = 0; i < items.size(); ++i) {
+        if (!fx_on_[i]) continue;
+        const WorkItem& it = items[i];
+        SystemState& s = *it.sys;
+        fxq_off_[i] = fxq_total;
+        fxq_total += it.offs.back();
+        FxSystem& x = fsys[i];
+        x.xyz = s.xyz.as<float4>();
+        x.map = s.rec_map.as<int>();
+        x.block_info = s.block_class.as<int>();
+        x.cf = it.d_cf;
+        x.qv = it.d_qv;
+        x.out = psys[i].out;
+        x.split_stride = psys[i].split_stride;
+        x.na_pad = (int)s.na_pad;
+        x.nf = (int)s.nf;
+        x.nshell = (int)it.offs.size() - 1;
+        x.nclass = (int)s.nclass;
+        const size_t nv = it.offs.back();
+        const long long nb = (long long)(s.na_rec / 32), ns = nsplit_[i];
+        for (size_t f0 = 0; f0 < s.nf; f0 += 8)
+            for (size_t v = 0; v < nv; v += 32)
+                for (int sp = 0; sp < nsplit_[i]; ++sp) {
+                    FxTileDesc t{};
+                    t.system = (int)i;
+                    t.v0 = (int)v;
+                    t.nv = (int)std::min<size_t>(32, nv - v);
+                    t.f0 = (int)f0;
+                    t.b_begin = (int)(sp * nb / ns);
+                    t.b_end = (int)((sp + 1) * nb / ns);
+                    t.split = sp;
+                    ftiles.push_back(t);
+                }
+    }
+    std::stable_sort(ftiles.begin(), ftiles.end(), [](const FxTileDesc& a, const FxTileDesc& b) {
+        return a.b_end - a.b_begin > b.b_end - b.b_begin;
+    });
+    nfx_tiles_ = (int)ftiles.size();
+    if (nfx_tiles_) {
+        ECK(fxq_.ensure(fxq_total * kFxQBytes));
+        if (!fxtab_.p) {
+            ECK(fxtab_.ensure(kFxTableGlobalBytes));
+            ECK(launch_fx_table(fxtab_.p, 0));
+        }
+        for (size_t i = 0; i < items.size(); ++i)
+            if (fx_on_[i])
+                fsys[i].qw = reinterpret_cast<const uint4*>(fxq_.as<unsigned char>() + fxq_off_[i] * kFxQBytes);
+    }
 
     // ---- correlation chunks and finalisation entries ------------------------------------------
     std::vector<CorrChunk> chunks;
@@ -1042,7 +1122,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     ECK(ppart_.ensure(poff * sizeof(double)));
     ECK(apart_.ensure(slot * sizeof(double2)));
     ECK(a2part_.ensure(slot * sizeof(double)));
-    ECK(counter_.ensure(2 * sizeof(unsigned)));
+    ECK(counter_.ensure(3 * sizeof(unsigned)));
     ECK(err_.ensure(sizeof(unsigned)));
 
     // shared twiddle table at the largest length
@@ -1059,13 +1139,18 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     std::vector<size_t> shell_off(items.size());
     for (size_t i = 0; i < items.size(); ++i) shell_off[i] = push(blob, shell_v[i]);
     size_t o_psys = push(blob, psys), o_tiles = push(blob, tiles);
+    size_t o_ftiles = push(blob, ftiles);
     size_t o_rsys = push(blob, rsys), o_rgroups = push(blob, rgroups), o_rtiles = push(blob, rtiles);
     // CorrSystem.shell_v points into the blob: patch with the final device address
-    ECK(blob_.ensure(blob.size() + 8192 + csys.size() * sizeof(CorrSystem) +
+    ECK(blob_.ensure(blob.size() + 8192 + csys.size() * sizeof(CorrSystem) + fsys.size() * sizeof(FxSystem) +
                      (chunks.size() + lchunks.size()) * sizeof(CorrChunk) +
                      (entries.size() + entries_w.size() + lentries.size()) * sizeof(FinalEntry) + 4096));
-    for (size_t i = 0; i < items.size(); ++i)
-        csys[i].shell_v = reinterpret_cast<const int*>(blob_.as<unsigned char>() + shell_off[i]);
+    item_shell_v_.assign(items.size(), nullptr);
+    for (size_t i = 0; i < items.size(); ++i) {
+        item_shell_v_[i] = reinterpret_cast<const int*>(blob_.as<unsigned char>() + shell_off[i]);
+        csys[i].shell_v = fsys[i].shell_v = item_shell_v_[i];
+    }
+    size_t o_fsys = push(blob, fsys);
     size_t o_csys = push(blob, csys), o_chunks = push(blob, chunks), o_entries = push(blob, entries);
     size_t o_entries_w = push(blob, entries_w);
     size_t o_lchunks = push(blob, lchunks), o_lentries = push(blob, lentries);
@@ -1079,6 +1164,8 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     unsigned char* base = blob_.as<unsigned char>();
     d_psys_ = reinterpret_cast<PhaseSystem*>(base + o_psys);
     d_tiles_ = reinterpret_cast<PhaseTileDesc*>(base + o_tiles);
+    d_fsys_ = reinterpret_cast<FxSystem*>(base + o_fsys);
+    d_ftiles_ = reinterpret_cast<FxTileDesc*>(base + o_ftiles);
     d_rsys_ = reinterpret_cast<RecSystem*>(base + o_rsys);
     d_rgroups_ = reinterpret_cast<RecGroup*>(base + o_rgroups);
     d_rtiles_ = reinterpret_cast<RecTileDesc*>(base + o_rtiles);
@@ -1089,7 +1176,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     d_long_chunks_ = reinterpret_cast<CorrChunk*>(base + o_lchunks);
     d_long_entries_ = reinterpret_cast<FinalEntry*>(base + o_lentries);
     ECK(cudaDeviceSynchronize());
-    stats_.phase_tiles = tiles.size();
+    stats_.phase_tiles = tiles.size() + ftiles.size();
     stats_.rec_tiles = rtiles.size();
     stats_.corr_chunks = chunks.size() + lchunks.size();
     stats_.final_entries = entries.size() + lentries.size();
@@ -1101,9 +1188,10 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
     const bool coherent = cfg_.scattering == 0;
     size_t launches = 0, phase_launches = 0;
     ECK(cudaMemsetAsync(err_.p, 0, sizeof(unsigned), st));
-    ECK(cudaMemsetAsync(counter_.p, 0, 2 * sizeof(unsigned), st));
+    ECK(cudaMemsetAsync(counter_.p, 0, 3 * sizeof(unsigned), st));
     for (int i = 0; i < nitems_; ++i) {
         SystemState& s = *item_sys_[i];
+        if (fx_on_[i]) continue;  // reads the class factors
         ECK(launch_expand_factors(item_cf_[i], (int)s.nclass, (int)item_nq_[i], s.cls.as<int>(), (int)s.na_pad,
                                   cfg_.precision, bfac_.as<unsigned char>() + bfac_off_[i], st));
         ++launches;
@@ -1135,6 +1223,22 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
         pl.err = err_.as<unsigned>();
         if (ntiles_) {
             ECK(launch_phase_sum(pl, st));
+            ++launches;
+            ++phase_launches;
+        }
+        if (nfx_tiles_) {
+            for (int i = 0; i < nitems_; ++i) {
+                if (!fx_on_[i]) continue;
+                ECK(launch_fx_q(item_qv_[i], item_nv_[i], fxq_.as<unsigned char>() + fxq_off_[i] * kFxQBytes, st));
+                ++launches;
+            }
+            FxLaunch fl{};
+            fl.systems = d_fsys_;
+            fl.tiles = d_ftiles_;
+            fl.ntiles = nfx_tiles_;
+            fl.table = fxtab_.p;
+            fl.counter = counter_.as<unsigned>() + 2;
+            ECK(launch_phase_fx(fl, st));
             ++launches;
             ++phase_launches;
         }
@@ -1245,6 +1349,11 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
         lf.a2part = a2part_.as<double>();
         lf.tw = s.tw64.as<double2>();
         lf.Z = long_Z_.as<double2>();
+        if (coherent && !f32) {
+            lf.A = static_cast<const double2*>(item_amp_[li.item]);
+            lf.shell_v = item_shell_v_[li.item];
+            ++launches;
+        }
         ECK(launch_long_finalize(lf, st));
         launches += 2;
     }

@@ -170,6 +170,13 @@ private:
     std::vector<size_t> item_nq_;
     int nphase_systems_ = 0, ntiles_ = 0, nchunks_ = 0, nentries_ = 0;
     int nrec_tiles_ = 0, nrec_groups_ = 0, rec_k_ = 0;
+    // fixed-point phase sum (FP64 form)
+    std::vector<char> fx_on_;
+    std::vector<size_t> fxq_off_;  // sub-vector offset of each item's fixed-point words
+    int nfx_tiles_ = 0;
+    FxSystem* d_fsys_ = nullptr;
+    FxTileDesc* d_ftiles_ = nullptr;
+    DevBuf fxtab_, fxq_;
     RecSystem* d_rsys_ = nullptr;
     RecGroup* d_rgroups_ = nullptr;
     RecTileDesc* d_rtiles_ = nullptr;
@@ -198,6 +205,7 @@ private:
     std::vector<LongBatch> long_batches_;
     std::vector<LongItem> long_items_;
     std::vector<const void*> item_amp_;
+    std::vector<const int*> item_shell_v_;  // device copies of the sub-vector offsets
     std::vector<std::vector<size_t>> item_offs_;
     std::vector<const double*> item_qv_;
     CorrChunk* d_long_chunks_ = nullptr;

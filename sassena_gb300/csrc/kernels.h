@@ -104,6 +104,44 @@ cudaError_t launch_split_reduce_f32(const float2* part, int nsplit, size_t n, fl
                                     cudaStream_t st);
 
 // ---------------------------------------------------------------------------------------
+// Fixed-point phase sum (FP64 form): a warp owns 32 q-vectors of any shells and one frame.
+// ---------------------------------------------------------------------------------------
+struct FxSystem {
+    const float4* xyz;      // [nf][na_pad] staged coordinates
+    const int* map;         // [na_rec] atom of each class-sorted slot (-1: padding)
+    const int* block_info;  // [na_rec / 32] class | padding atoms << 16 of every 32-atom block
+    const double* cf;       // [nshell][nclass] class factors
+    const double* qv;       // [nv][3] sub-vectors
+    const uint4* qw;        // [nv][4] their fixed-point words (launch_fx_q)
+    const int* shell_v;     // [nshell+1] sub-vector offsets of each shell
+    double2* out;           // amplitudes [nv][nf], or split partials [nsplit][nv][nf]
+    size_t split_stride;    // nv * nf
+    int na_pad, nf, nshell, nclass;
+};
+
+struct FxTileDesc {
+    int system;
+    int v0, nv;             // sub-vectors [v0, v0+nv), nv <= 32
+    int f0;                 // first of 8 frames, one per warp
+    int b_begin, b_end;     // 32-atom blocks of the class-sorted slots
+    int split, pad;
+};
+
+struct FxLaunch {
+    const FxSystem* systems;
+    const FxTileDesc* tiles;
+    int ntiles;
+    const void* table;      // launch_fx_table
+    unsigned int* counter;  // work-queue counter, zero before the launch
+};
+
+constexpr size_t kFxQBytes = 64;            // fixed-point words of one sub-vector
+constexpr size_t kFxTableGlobalBytes = 1024 * 16;
+cudaError_t launch_fx_table(void* table, cudaStream_t st);
+cudaError_t launch_fx_q(const double* qv, size_t nv, void* qw, cudaStream_t st);
+cudaError_t launch_phase_fx(const FxLaunch& a, cudaStream_t st);
+
+// ---------------------------------------------------------------------------------------
 // Shell-recurrence phase sum (FP32 form): runs of shells lam_k = lam0 + k dlam along
 // shared base vectors, evaluated with a three-term recurrence over k.
 // ---------------------------------------------------------------------------------------
@@ -292,6 +330,8 @@ struct LongFinal {
     const double* a2part;
     const double2* tw;         // W_L^j, j < L/2, FP64
     double2* Z;                // [nentries][L] scratch
+    const double2* A;          // coherent FP64: amplitudes [nv][nf] and sub-vector offsets
+    const int* shell_v;        //   [nentries+1] for the directly summed last lags (null: none)
 };
 cudaError_t launch_long_finalize(const LongFinal& a, cudaStream_t st);
 // K of a long system: K(k) = sum_{tau<nf} exp(+2 pi i k tau / L) / (nf L (nf - tau)) in the long
