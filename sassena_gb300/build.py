@@ -32,7 +32,7 @@ CXX = os.environ.get("CXX", "g++")
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-ffp-contract=off", "-I" + INCLUDE, "-I" + HOST]
 
 CUDA_SOURCES = [
-    "capi.cu", "engine.cu", "phase_sum.cu", "phase_rec.cu", "phase_fx.cu", "correlate.cu", "peaks.cu", "noalloc.cu", "mlp.cu",
+    "capi.cu", "engine.cu", "phase_sum.cu", "phase_rec.cu", "phase_fx.cu", "phase_grid.cu", "correlate.cu", "peaks.cu", "noalloc.cu", "mlp.cu",
     "cv.cu", "multipole.cu", "align.cu", "corr_long.cu",
 ]
 HOST_SOURCES = []  # filled when the host layer exists (see host_sources())

@@ -76,7 +76,7 @@ std::map<std::string, TuneChoice> g_tune_cache;
 
 // Product-set detection on host sub-vectors (copied from the device when needed).
 int product_of(std::string& m, const double* qv, bool on_device, const std::vector<size_t>& offs,
-               std::vector<double>& lam, int& base);
+               std::vector<double>& lam, int& base, double& umax);
 
 }  // namespace
 
@@ -97,6 +97,7 @@ struct sass_batch {
     int split_atoms = 0, rec_k = 0;
     std::vector<std::vector<double>> lam;  // product structure per system (empty: none)
     std::vector<int> lam_base;
+    std::vector<double> umax;
     std::string msg;
     sass_timing timing{};
     cudaEvent_t ev[kEvents] = {};
@@ -210,15 +211,19 @@ int autotune_engine(std::string& m, Engine& eng, const EngineConfig& base, const
         }
         return SASS_OK;
     };
-    // the recurrence widths are worth timing only where some shells form runs
-    bool product = false;
-    for (const WorkItem& it : items)
-        product = product || (!it.lam.empty() && !arithmetic_runs(it.lam, 3).empty());
+    // product sets: the automatic choice (the gridded kernel where it pays) against the direct
+    // kernel, and the recurrence widths where some shells form runs
+    bool product = false, runs = false;
+    for (const WorkItem& it : items) {
+        product = product || !it.lam.empty();
+        runs = runs || (!it.lam.empty() && !arithmetic_runs(it.lam, 3).empty());
+    }
     int rec_k = -1;
     bool all_rec = false;
     if (base.precision == PREC_FP32 && product) {
-        std::vector<int> ks = {-1};
-        for (int k : rec_shell_counts()) ks.push_back(k);
+        std::vector<int> ks = {-1, 0};
+        if (runs)
+            for (int k : rec_shell_counts()) ks.push_back(k);
         for (int k : ks) {
             EngineConfig c = base;
             c.rec_k = k;
@@ -226,7 +231,7 @@ int autotune_engine(std::string& m, Engine& eng, const EngineConfig& base, const
             if (rc) return rc;
         }
         rec_k = best.rec_k;
-        if (rec_k > 0) {
+        if (rec_k >= 0) {
             EngineConfig c = base;
             c.rec_k = rec_k;
             std::string err;
@@ -258,7 +263,7 @@ int autotune_engine(std::string& m, Engine& eng, const EngineConfig& base, const
 }
 
 int product_of(std::string& m, const double* qv, bool on_device, const std::vector<size_t>& offs,
-               std::vector<double>& lam, int& base) {
+               std::vector<double>& lam, int& base, double& umax) {
     lam.clear();
     base = -1;
     const double* h = qv;
@@ -268,7 +273,7 @@ int product_of(std::string& m, const double* qv, bool on_device, const std::vect
         CK(m, cudaMemcpy(copy.data(), qv, copy.size() * sizeof(double), cudaMemcpyDeviceToHost));
         h = copy.data();
     }
-    detect_product(h, offs, lam, base);
+    detect_product(h, offs, lam, base, umax);
     return SASS_OK;
 }
 
@@ -521,7 +526,7 @@ int sass_compute(sass_plan* p, size_t nq, const size_t* offs, const double* subv
         it.d_qv = d_qv + 3 * offs[i];
         if (want_rec) {
             rc = product_of(p->msg, io_on_device ? d_qv + 3 * offs[i] : subvectors + 3 * offs[i], io_on_device != 0,
-                            it.offs, it.lam, it.lam_base);
+                            it.offs, it.lam, it.lam_base, it.umax);
             if (rc) return rc;
         }
         it.d_cf = d_cf + nclass * i;
@@ -594,7 +599,8 @@ int sass_autotune(sass_plan* p, size_t nq, const size_t* offs, const double* sub
     items[0].d_fq = p->fq.as<double2>();
     items[0].d_fq2 = p->fq2.as<double2>();
     if (p->d.precision == SASS_PRECISION_FP32) {
-        rc = product_of(p->msg, subvectors, false, items[0].offs, items[0].lam, items[0].lam_base);
+        rc = product_of(p->msg, subvectors, false, items[0].offs, items[0].lam, items[0].lam_base,
+                        items[0].umax);
         if (rc) return rc;
     }
     TuneChoice best;
@@ -758,8 +764,9 @@ int sass_batch_create(const sass_plan_desc* desc, size_t nsystems, const sass_sy
         b->offs.emplace_back(s.sub_offsets, s.sub_offsets + s.nq + 1);
         b->lam.emplace_back();
         b->lam_base.push_back(-1);
+        b->umax.push_back(0);
         if (b->d.precision == SASS_PRECISION_FP32 && b->d.scattering == SASS_SCATTERING_ALL)
-            detect_product(s.subvectors, b->offs.back(), b->lam.back(), b->lam_base.back());
+            detect_product(s.subvectors, b->offs.back(), b->lam.back(), b->lam_base.back(), b->umax.back());
         b->nq.push_back(s.nq);
         b->nv.push_back(s.sub_offsets[s.nq]);
         b->qv_off.push_back(qv_n);
@@ -804,6 +811,7 @@ static std::vector<WorkItem> batch_items(sass_batch* b) {
         it.d_qv = b->qv.as<double>() + b->qv_off[i];
         it.lam = b->lam[i];
         it.lam_base = b->lam_base[i];
+        it.umax = b->umax[i];
         it.d_cf = b->cf.as<double>() + b->cf_off[i];
         it.d_fqt = reinterpret_cast<double2*>(b->out.as<double>() + b->fqt_off[i]);
         it.d_fq = reinterpret_cast<double2*>(b->out.as<double>() + b->fq_off[i]);

@@ -619,8 +619,10 @@ __device__ __forceinline__ float centred(float x, float h, float l) {
 
 __global__ void stage_kernel(const float* __restrict__ raw, int nf, int na, int na_pad, double cx,
                              double cy, double cz, int center, float4* __restrict__ xyz,
-                             const int* __restrict__ rec_inv, int na_rec, float4* __restrict__ xyz_rec) {
+                             const int* __restrict__ rec_inv, int na_rec, float4* __restrict__ xyz_rec,
+                             unsigned int* __restrict__ rmax2) {
     const size_t n = (size_t)nf * na_pad;
+    unsigned int far = 0;  // largest |r|^2 as bits: NaN and infinity sort above every number
     // the centre as float pairs hi + lo: x - c is formed by TwoSum in FP32 and rounded once
     // (per coordinate an FP64 subtraction and two conversions made this kernel bound by
     // GB300's narrow FP64 pipe once its input came from device memory)
@@ -643,8 +645,13 @@ __global__ void stage_kernel(const float* __restrict__ raw, int nf, int na, int 
                 r.z = p[2];
             }
             if (xyz_rec) xyz_rec[f * na_rec + rec_inv[j]] = make_float4(r.x, r.y, r.z, 1.f);
+            far = max(far, __float_as_uint(r.x * r.x + r.y * r.y + r.z * r.z) & 0x7fffffffu);
         }
         xyz[idx] = r;
+    }
+    if (rmax2) {
+        far = __reduce_max_sync(0xffffffffu, far);
+        if ((threadIdx.x & 31) == 0 && far > *reinterpret_cast<volatile unsigned int*>(rmax2)) atomicMax(rmax2, far);
     }
 }
 
@@ -1918,10 +1925,10 @@ cudaError_t launch_store_kernel(const double2* tw64, int lg_tw, double2* k64, fl
 
 cudaError_t launch_stage(const float* raw, int nf, int na, int na_pad, double cx, double cy,
                          double cz, int center, float4* xyz, const int* rec_inv, int na_rec,
-                         float4* xyz_rec, cudaStream_t st) {
+                         float4* xyz_rec, unsigned int* rmax2, cudaStream_t st) {
     size_t n = (size_t)nf * na_pad;
     stage_kernel<<<grid_for(n, 256), 256, 0, st>>>(raw, nf, na, na_pad, cx, cy, cz, center, xyz, rec_inv,
-                                                   na_rec, xyz_rec);
+                                                   na_rec, xyz_rec, rmax2);
     return cudaGetLastError();
 }
 

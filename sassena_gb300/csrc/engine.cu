@@ -234,11 +234,28 @@ int stage_system(SystemState& s, const float* coords, bool on_device, int precis
         }
     }
     memcpy(s.center, c, sizeof(c));
+    const bool bounded = precision == PREC_FP32;  // the gridded phase sum needs the extent
+    if (bounded) {
+        ECK(s.rmax_word.ensure(sizeof(unsigned)));
+        ECK(cudaMemsetAsync(s.rmax_word.p, 0, sizeof(unsigned), st));
+    }
     // the class-sorted copy, once it exists for the current classes, is filled in the same pass
     const bool rec = s.rec_ready && s.rec_map_ok;
     ECK(launch_stage(src, (int)s.nf, (int)s.na, (int)s.na_pad, c[0], c[1], c[2], precision == PREC_FP32,
                      s.xyz.as<float4>(), rec ? s.rec_inv.as<int>() : nullptr, (int)s.na_rec,
-                     rec ? s.xyz_rec.as<float4>() : nullptr, st));
+                     rec ? s.xyz_rec.as<float4>() : nullptr, bounded ? s.rmax_word.as<unsigned>() : nullptr, st));
+    s.rmax = 0;
+    if (bounded) {
+        float r2 = 0.f;
+        ECK(cudaMemcpyAsync(&r2, s.rmax_word.p, sizeof(r2), cudaMemcpyDeviceToHost, st));
+        ECK(cudaStreamSynchronize(st));
+        // rounded up to 6 significant bits (and FP32's rounding of r^2), so that descriptors built
+        // for one staging mostly fit the next
+        int e = 0;
+        const double m = std::frexp(std::sqrt((double)r2) * (1.0 + 1e-6), &e);
+        s.rmax = r2 > 0 ? std::ldexp(std::ceil(m * 64.0) / 64.0, e) : (r2 == 0 ? 1e-30 : INFINITY);
+        if (!std::isfinite((double)r2)) s.rmax = INFINITY;
+    }
     ECK(cudaStreamSynchronize(st));
     s.staged = true;
     s.rec_valid = rec;
@@ -320,9 +337,11 @@ int set_system_classes(SystemState& s, const int32_t* cls, bool on_device, cudaS
     return kOk;
 }
 
-bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vector<double>& lam, int& base) {
+bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vector<double>& lam, int& base,
+                    double& umax) {
     lam.clear();
     base = -1;
+    umax = 0;
     const size_t nq = offs.size() - 1;
     if (nq == 0 || !qv) return false;
     const size_t nd = offs[1] - offs[0];
@@ -362,6 +381,7 @@ bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vect
             }
         lam[s] = l;
     }
+    umax = std::sqrt(best);
     return true;
 }
 
@@ -406,6 +426,83 @@ int choose_rec_k(const std::vector<std::vector<std::pair<int, int>>>& runs) {
         }
     }
     return best;
+}
+
+// Gridded phase sum: grid of an item's projections for weight set `set`.
+struct GridShape {
+    double h;    // spacing along a base vector
+    int G, off;  // points; the point of projection 0
+};
+
+GridShape grid_shape(const WorkItem& it, int set) {
+    double lmax = 0;
+    for (double l : it.lam) lmax = std::max(lmax, std::fabs(l));
+    GridShape g{};
+    g.h = 3.14159265358979323846 / (kGridSigma[set] * lmax);
+    const double half = std::ceil(it.sys->rmax * it.umax / g.h) + 1;  // projections round to [-half, half]
+    g.off = half < 1e6 ? (int)half + 2 : 1 << 20;
+    g.G = 2 * g.off + 2;  // six points: 2 below the nearest integer to 3 above it
+    return g;
+}
+
+// Directions of a warp's lanes: 32, and 16 x 2 or 8 x 4 frames for what is left over.
+struct GridLanes {
+    int d0, nd, lgd;
+};
+
+std::vector<GridLanes> grid_lanes(int nd) {
+    std::vector<GridLanes> v;
+    for (int d = 0; d < nd;) {
+        const int rem = nd - d, lgd = rem > 24 ? 5 : (rem > 8 ? 4 : 3), n = std::min(rem, 1 << lgd);
+        v.push_back(GridLanes{d, n, lgd});
+        d += n;
+    }
+    return v;
+}
+
+// Items the gridded kernel takes, the weight set, the largest grid and the frames per warp. In
+// clocks of an SM per 32 (atom, direction, frame): the grid costs 12 and its transforms nq G / 1.5
+// per slice, the recurrence 1.18 (K + 5.5) per group of K equally spaced shells, the direct kernel
+// 4.5 per shell (measured on a GB300 at 10,000 atoms). Below 512 atoms the transforms and the
+// grid's clearing outweigh the atoms. Two CTAs per SM still fill three quarters of the issue
+// slots; grids that leave one are not taken. The finer weight set (more points) is used where it
+// leaves all four CTAs.
+void choose_grid(const std::vector<WorkItem>& items, std::vector<char>& on, int& set, int& points, int& frames) {
+    bool any = false;
+    set = 1;
+    for (size_t i = 0; i < items.size(); ++i) {
+        const WorkItem& it = items[i];
+        const SystemState& s = *it.sys;
+        if (it.lam.size() + 1 != it.offs.size() || it.lam_base < 0 || it.d_amp_given || !(it.umax > 0) ||
+            !(s.rmax > 0) || !std::isfinite(s.rmax) || s.na < 512 || s.nclass > 65535)
+            continue;
+        const int G = grid_shape(it, 0).G;
+        if (G > 4096 || grid_ctas(G, 4) < 2) continue;
+        const int nd = (int)it.offs[1], nq = (int)it.lam.size();
+        double lanes = 0;
+        for (const GridLanes& g : grid_lanes(nd)) lanes += 1 << g.lgd;
+        const double slice = (double)std::min(s.na, kGridMaxSlice);
+        const double grid = ((grid_ctas(G, 4) < 4 ? 15.0 : 12.0) + (double)nq * G / (1.5 * slice)) * lanes / nd;
+        const auto runs = arithmetic_runs(it.lam, 3);
+        double other = 4.5 * nq;
+        if (s.nclass <= (size_t)kRecMaxClass && !runs.empty()) {
+            const int K = choose_rec_k({runs});
+            for (const auto& ae : runs) {
+                const int n = ae.second - ae.first, ng = (n + K - 1) / K;
+                other += ng * 1.18 * rec_group_cost(K) * std::ceil(ng * nd / 32.0) * 32.0 / (ng * nd) - 4.5 * n;
+            }
+        }
+        if (grid > 0.9 * other) continue;
+        on[i] = 1;
+        any = true;
+        if (grid_ctas(grid_shape(it, 1).G, 4) < 4) set = 0;
+    }
+    if (!any) return;
+    for (size_t i = 0; i < items.size(); ++i) {
+        if (!on[i]) continue;
+        points = std::max(points, grid_shape(items[i], set).G);
+        for (const GridLanes& g : grid_lanes((int)items[i].offs[1])) frames = std::max(frames, 32 >> g.lgd);
+    }
 }
 
 // Class-sorted layout for the recurrence kernel: class segments padded to 32 atoms, w = 1
@@ -469,7 +566,7 @@ int ensure_rec_layout(SystemState& s, std::string& err) {
 void Engine::release() {
     key_.clear();
     DevBuf* bufs[] = {&blob_,    &bfac_, &amp_, &part_,  &ppart_, &apart_,
-                      &a2part_, &counter_, &err_, &tw64_, &tw32_, &rec_bfac_, &fxtab_, &fxq_};
+                      &a2part_, &counter_, &err_, &tw64_, &tw32_, &rec_bfac_, &fxtab_, &fxq_, &grid_ws_};
     for (DevBuf* b : bufs) b->release();
     hblob_.release();
 }
@@ -509,6 +606,7 @@ static std::vector<uint64_t> prepare_key(const EngineConfig& c, const std::vecto
             u((uint64_t)s.staged | (uint64_t)s.classes_set << 1 | (uint64_t)s.rec_valid << 2 |
               (uint64_t)s.rec_map_ok << 3 | (uint64_t)s.rec_ready << 4);
             for (int c3 = 0; c3 < 3; ++c3) d(s.center[c3]);
+            d(s.rmax);
             p(s.xyz.p);
             p(s.xyz_rec.p);
             p(s.block_class.p);
@@ -521,6 +619,7 @@ static std::vector<uint64_t> prepare_key(const EngineConfig& c, const std::vecto
         u(it.lam.size());
         for (double l : it.lam) d(l);
         u((uint64_t)(int64_t)it.lam_base);
+        d(it.umax);
         for (const void* q : {(const void*)it.d_qv, (const void*)it.d_cf, (const void*)it.d_fqt,
                               (const void*)it.d_fq, (const void*)it.d_fq2, (const void*)it.d_wsqrt,
                               (const void*)it.d_fqt_w, (const void*)it.d_fq_w, (const void*)it.d_fq2_w,
@@ -588,6 +687,18 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     }
     stats_.shape = shape;
 
+    // ---- gridded phase sum (FP32 form; shells along one direction set, automatic choice) ---------
+    std::vector<char> grid_on(items.size(), 0);
+    grid_points_ = 0;
+    grid_frames_ = 1;
+    grid_set_ = 0;
+    if (f32 && coherent && cfg.rec_k == 0) choose_grid(items, grid_on, grid_set_, grid_points_, grid_frames_);
+    for (size_t i = 0; i < items.size(); ++i)
+        if (grid_on[i]) {
+            const int rc = ensure_rec_layout(*items[i].sys, err);
+            if (rc) return rc;
+        }
+
     // ---- shell-recurrence groups (FP32 form; shells along one direction set) ---------------------
     std::vector<std::vector<char>> rec_on(items.size());
     std::vector<RecGroup> rgroups;
@@ -598,7 +709,8 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         bool any = false;
         for (size_t i = 0; i < items.size(); ++i) {
             const WorkItem& it = items[i];
-            if (it.lam.size() + 1 != it.offs.size() || it.lam_base < 0 || it.sys->nclass > (size_t)kRecMaxClass)
+            if (grid_on[i] || it.lam.size() + 1 != it.offs.size() || it.lam_base < 0 ||
+                it.sys->nclass > (size_t)kRecMaxClass)
                 continue;
             runs[i] = arithmetic_runs(it.lam, 3);
             any = any || !runs[i].empty();
@@ -659,11 +771,15 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     // atom splits: enough tiles for the persistent grid to balance
     nsplit_.assign(items.size(), 1);
     size_t base_tiles = 0;
-    size_t fx_units = 0;  // warp tiles of the fixed-point kernel without splits
+    size_t fx_units = 0, grid_units = 0;  // warp tiles of the fixed-point and gridded kernels without splits
     for (size_t i = 0; i < items.size(); ++i) {
         const WorkItem& it = items[i];
         if (fx_on_[i]) {
             fx_units += (it.offs.back() + 31) / 32 * it.sys->nf;
+            continue;
+        }
+        if (grid_on[i]) {
+            for (const GridLanes& g : grid_lanes((int)it.offs[1])) grid_units += (it.sys->nf * (size_t)(1 << g.lgd) + 31) / 32;
             continue;
         }
         size_t groups = 0;
@@ -684,6 +800,16 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
             max_split = std::max(1, (int)(items[i].sys->na_rec / 128));
             if (cfg.split_atoms > 0) ns = (int)((items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms);
             else ns = (int)std::min<size_t>(64, ((size_t)sms * 96 + fx_units - 1) / std::max<size_t>(fx_units, 1));
+        } else if (grid_on[i]) {
+            // as above, four for each of the CTAs of an SM, with slices of at least 1,024 atoms, since
+            // each pays for its own transform, and at most kGridMaxSlice
+            const size_t nr = items[i].sys->na_rec;
+            max_split = std::max(1, (int)(nr / 128));
+            const size_t want = ((size_t)sms * grid_ctas(grid_points_, grid_frames_) * 4 + grid_units - 1) /
+                                std::max<size_t>(grid_units, 1);
+            size_t n = std::min(want, nr / 1024);
+            if (cfg.split_atoms > 0) n = (items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms;
+            ns = (int)std::max(n, (nr + kGridMaxSlice - 1) / kGridMaxSlice);
         } else if (cfg.split_atoms > 0) {
             ns = (int)((items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms);
         } else if (base_tiles < target) {
@@ -819,7 +945,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
             const long long nst = (long long)(s.na_pad / shape.atoms), ns = nsplit_[i];
             // frame tiles outermost: the tiles that read the same frames run together, so
             // the coordinates stream from HBM about once and the other reads hit L2
-            for (size_t f0 = 0; f0 < s.nf && !fx_on_[i]; f0 += shape.warps)
+            for (size_t f0 = 0; f0 < s.nf && !fx_on_[i] && !grid_on[i]; f0 += shape.warps)
                 for (size_t sh = 0; sh < nq; ++sh) {
                     if (is_rec(i, sh)) continue;
                     for (size_t v = it.offs[sh]; v < it.offs[sh + 1]; v += per)
@@ -962,6 +1088,87 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         for (size_t i = 0; i < items.size(); ++i)
             if (fx_on_[i])
                 fsys[i].qw = reinterpret_cast<const uint4*>(fxq_.as<unsigned char>() + fxq_off_[i] * kFxQBytes);
+    }
+
+    // gridded tiles: directions x frames of a warp's lanes, 8 warps' frames, atom slice
+    std::vector<GridSystem> gsys;
+    std::vector<GridTileDesc> gtiles;
+    std::vector<double> gshells;
+    std::vector<size_t> gitem;
+    size_t gws = 256;  // the weights' coefficients first
+    grid_table_ = 0;
+    for (size_t i = 0; i < items.size(); ++i) {
+        if (!grid_on[i]) continue;
+        const WorkItem& it = items[i];
+        SystemState& s = *it.sys;
+        const GridShape gs = grid_shape(it, grid_set_);
+        GridSystem g{};
+        g.xyzw = s.xyz_rec.as<float4>();
+        g.block_class = s.block_class.as<int>();
+        g.cf = it.d_cf;
+        g.dirs = it.d_qv + 3 * it.offs[it.lam_base];
+        g.out_f32 = psys[i].out_f32;
+        g.split_stride = psys[i].split_stride;
+        g.inv_h = 1.0 / gs.h;
+        g.na_rec = (int)s.na_rec;
+        g.nf = (int)s.nf;
+        g.nd = (int)it.offs[1];
+        g.nclass = (int)s.nclass;
+        g.nq = (int)it.lam.size();
+        g.G = gs.G;
+        g.off = gs.off;
+        g.shell_off = (int)gshells.size();
+        for (double l : it.lam) gshells.push_back(l * gs.h * 0.15915494309189533577);
+        for (double l : it.lam) gshells.push_back(1.0 / grid_deconvolution(grid_set_, l * gs.h));
+        const int nk = (g.nq + kGridShellChunk - 1) / kGridShellChunk * kGridShellChunk;
+        const int np = (g.off + 2 + 15) / 16 * 16, sidx = (int)gsys.size();
+        grid_table_ = std::max(grid_table_, nk * np);
+        // offsets for now; patched with the buffer's address below
+        auto take = [&](size_t bytes) {
+            const size_t o = gws;
+            gws += (bytes + 255) & ~(size_t)255;
+            return o;
+        };
+        g.tw = reinterpret_cast<float2*>(take((size_t)nk * np * sizeof(float2)));
+        g.facs = reinterpret_cast<float*>(take((size_t)g.nclass * g.nq * sizeof(float)));
+        g.gw = reinterpret_cast<float*>(take((size_t)(g.nclass + 1) * sizeof(float)));
+        g.konst = reinterpret_cast<int*>(take(sizeof(int)));
+        const long long nb = (long long)(s.na_rec / 32), ns = nsplit_[i];
+        g.slice_atoms = (int)((nb + ns - 1) / ns) * 32;
+        gsys.push_back(g);
+        for (const GridLanes& gl : grid_lanes(g.nd))
+            for (int f0 = 0; f0 < g.nf; f0 += 256 >> gl.lgd)
+                for (int sp = 0; sp < nsplit_[i]; ++sp) {
+                    GridTileDesc t{};
+                    t.system = sidx;
+                    t.d0 = gl.d0;
+                    t.nd = gl.nd;
+                    t.lgd = gl.lgd;
+                    t.f0 = f0;
+                    t.b_begin = (int)(sp * nb / ns);
+                    t.b_end = (int)((sp + 1) * nb / ns);
+                    t.split = sp;
+                    gtiles.push_back(t);
+                }
+        stats_.rec_shells += it.lam.size();
+    }
+    // longest first; then frames together, so that their coordinates are read from HBM about once
+    std::stable_sort(gtiles.begin(), gtiles.end(), [](const GridTileDesc& a, const GridTileDesc& b) {
+        const int ca = a.b_end - a.b_begin, cb = b.b_end - b.b_begin;
+        if (ca != cb) return ca > cb;
+        return a.system != b.system ? a.system < b.system : a.f0 < b.f0;
+    });
+    ngrid_tiles_ = (int)gtiles.size();
+    ngrid_systems_ = (int)gsys.size();
+    if (ngrid_tiles_) {
+        ECK(grid_ws_.ensure(gws));
+        auto at = [&](void* off) { return grid_ws_.as<unsigned char>() + (size_t)(uintptr_t)off; };
+        for (GridSystem& g : gsys) {
+            g.tw = reinterpret_cast<float2*>(at(g.tw));
+            g.facs = reinterpret_cast<float*>(at(g.facs));
+            g.gw = reinterpret_cast<float*>(at(g.gw));
+            g.konst = reinterpret_cast<int*>(at(g.konst));
+        }
     }
 
     // ---- correlation chunks and finalisation entries ------------------------------------------
@@ -1122,7 +1329,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     ECK(ppart_.ensure(poff * sizeof(double)));
     ECK(apart_.ensure(slot * sizeof(double2)));
     ECK(a2part_.ensure(slot * sizeof(double)));
-    ECK(counter_.ensure(3 * sizeof(unsigned)));
+    ECK(counter_.ensure(4 * sizeof(unsigned)));
     ECK(err_.ensure(sizeof(unsigned)));
 
     // shared twiddle table at the largest length
@@ -1140,6 +1347,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     for (size_t i = 0; i < items.size(); ++i) shell_off[i] = push(blob, shell_v[i]);
     size_t o_psys = push(blob, psys), o_tiles = push(blob, tiles);
     size_t o_ftiles = push(blob, ftiles);
+    size_t o_gsys = push(blob, gsys), o_gtiles = push(blob, gtiles), o_gshells = push(blob, gshells);
     size_t o_rsys = push(blob, rsys), o_rgroups = push(blob, rgroups), o_rtiles = push(blob, rtiles);
     // CorrSystem.shell_v points into the blob: patch with the final device address
     ECK(blob_.ensure(blob.size() + 8192 + csys.size() * sizeof(CorrSystem) + fsys.size() * sizeof(FxSystem) +
@@ -1164,6 +1372,9 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     unsigned char* base = blob_.as<unsigned char>();
     d_psys_ = reinterpret_cast<PhaseSystem*>(base + o_psys);
     d_tiles_ = reinterpret_cast<PhaseTileDesc*>(base + o_tiles);
+    d_gsys_ = reinterpret_cast<GridSystem*>(base + o_gsys);
+    d_gtiles_ = reinterpret_cast<GridTileDesc*>(base + o_gtiles);
+    d_gshells_ = reinterpret_cast<double*>(base + o_gshells);
     d_fsys_ = reinterpret_cast<FxSystem*>(base + o_fsys);
     d_ftiles_ = reinterpret_cast<FxTileDesc*>(base + o_ftiles);
     d_rsys_ = reinterpret_cast<RecSystem*>(base + o_rsys);
@@ -1177,7 +1388,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     d_long_entries_ = reinterpret_cast<FinalEntry*>(base + o_lentries);
     ECK(cudaDeviceSynchronize());
     stats_.phase_tiles = tiles.size() + ftiles.size();
-    stats_.rec_tiles = rtiles.size();
+    stats_.rec_tiles = rtiles.size() + gtiles.size();
     stats_.corr_chunks = chunks.size() + lchunks.size();
     stats_.final_entries = entries.size() + lentries.size();
     return kOk;
@@ -1188,7 +1399,7 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
     const bool coherent = cfg_.scattering == 0;
     size_t launches = 0, phase_launches = 0;
     ECK(cudaMemsetAsync(err_.p, 0, sizeof(unsigned), st));
-    ECK(cudaMemsetAsync(counter_.p, 0, 3 * sizeof(unsigned), st));
+    ECK(cudaMemsetAsync(counter_.p, 0, 4 * sizeof(unsigned), st));
     for (int i = 0; i < nitems_; ++i) {
         SystemState& s = *item_sys_[i];
         if (fx_on_[i]) continue;  // reads the class factors
@@ -1209,6 +1420,18 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
         rl.err = err_.as<unsigned>();
         ECK(launch_rec_factors(rl, nrec_groups_, st));
         ECK(launch_phase_rec(rl, st));
+        launches += 2;
+        ++phase_launches;
+    }
+    if (coherent && ngrid_tiles_) {
+        ECK(launch_grid_tables(d_gsys_, ngrid_systems_, grid_table_, d_gshells_, grid_set_, grid_ws_.as<float2>(), st));
+        GridLaunch gl{};
+        gl.systems = d_gsys_;
+        gl.tiles = d_gtiles_;
+        gl.ntiles = ngrid_tiles_;
+        gl.counter = counter_.as<unsigned>() + 3;
+        gl.coef = grid_ws_.as<float2>();
+        ECK(launch_phase_grid(gl, grid_points_, grid_frames_, st));
         launches += 2;
         ++phase_launches;
     }

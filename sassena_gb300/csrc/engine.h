@@ -45,6 +45,10 @@ struct SystemState {
     size_t na = 0, nf = 0, na_pad = 0, nclass = 0;
     int lg = 0;  // padded FFT length 2^lg >= 2 nf
     double center[3] = {0, 0, 0};
+    // FP32 form: bound on |r| of the staged frames (rounded up to 6 bits; 0: not known, infinite:
+    // some coordinate is not finite)
+    double rmax = 0;
+    DevBuf rmax_word;
     DevBuf raw, xyz, cls, tw64, tw32, k64, k32;
     DevBuf twff, kff;  // long series: float-float twiddles [L/2] and store kernel [L] (16 B each)
     bool staged = false, classes_set = false;
@@ -87,6 +91,7 @@ struct WorkItem {
     // shell s (see detect_product); empty: general sub-vectors
     std::vector<double> lam;
     int lam_base = -1;
+    double umax = 0;  // length of the longest base vector
     const double* d_cf = nullptr;  // [nq][nclass]
     double2* d_fqt = nullptr;      // [nq][nf]
     double2* d_fq = nullptr;       // [nq]
@@ -133,7 +138,9 @@ void drop_prefetch(SystemState& s);
 // Whether shells [0, nq) of host sub-vectors qv (offsets offs) are multiples of one base
 // set: equal counts per shell and qv[offs[s] + d] = lam[s] * qv[offs[base] + d] within
 // 1e-12 of the shell's largest sub-vector. Fills lam and base on success.
-bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vector<double>& lam, int& base);
+// `umax` is the length of the longest base vector.
+bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vector<double>& lam, int& base,
+                    double& umax);
 // Maximal runs [a, e) of at least min_len shells whose lam lies on a line within
 // 2.5e-7 of the run's largest |lam| (float-rounded linear scans qualify).
 std::vector<std::pair<int, int>> arithmetic_runs(const std::vector<double>& lam, int min_len);
@@ -173,6 +180,12 @@ private:
     // fixed-point phase sum (FP64 form)
     std::vector<char> fx_on_;
     std::vector<size_t> fxq_off_;  // sub-vector offset of each item's fixed-point words
+    // gridded phase sum (FP32 form)
+    int ngrid_tiles_ = 0, ngrid_systems_ = 0, grid_points_ = 0, grid_frames_ = 1, grid_set_ = 0, grid_table_ = 0;
+    GridSystem* d_gsys_ = nullptr;
+    GridTileDesc* d_gtiles_ = nullptr;
+    double* d_gshells_ = nullptr;
+    DevBuf grid_ws_;
     int nfx_tiles_ = 0;
     FxSystem* d_fsys_ = nullptr;
     FxTileDesc* d_ftiles_ = nullptr;

@@ -197,6 +197,56 @@ cudaError_t launch_permute_stage(const float4* src, int na_pad_src, const int* m
                                  float4* dst, cudaStream_t st);
 
 // ---------------------------------------------------------------------------------------
+// Gridded phase sum (FP32 form): all shells of a direction from one grid of its projections.
+// ---------------------------------------------------------------------------------------
+struct GridSystem {
+    const float4* xyzw;       // class-sorted coordinates [nf][na_rec], w = 0 for padding atoms
+    const int* block_class;   // [na_rec / 32] class | padding atoms << 16
+    const double* cf;         // [nq][nclass] class factors
+    const double* dirs;       // [nd][3] base vectors
+    float2* out_f32;          // FP32 amplitudes [nv][nf] (one split), or FP32 split partials
+    size_t split_stride;      // nv * nf
+    double inv_h;             // 1 / grid spacing (along a base vector)
+    // filled by launch_grid_tables
+    float2* tw;               // [nq / 8 rounded up][off + 2 rounded up to 16][8]
+    float* facs;              // [nclass][nq]
+    float* gw;                // [nclass + 1]
+    int* konst;
+    int na_rec, nf, nd, nclass, nq;
+    int G, off;               // grid points; the point of projection 0
+    int shell_off;            // of the system's [2][nq] shell constants
+    int slice_atoms;          // most atoms of a tile
+};
+
+struct GridTileDesc {
+    int system;
+    int d0, nd, lgd;          // directions [d0, d0+nd), nd <= 2^lgd (32, 16 or 8)
+    int f0;                   // 8 units of 32 / 2^lgd frames
+    int b_begin, b_end;       // 32-atom blocks (not empty)
+    int split;
+};
+
+struct GridLaunch {
+    const GridSystem* systems;
+    const GridTileDesc* tiles;
+    int ntiles;
+    unsigned int* counter;    // work-queue counter, zero before the launch
+    const float2* coef;       // [9] weight coefficients (launch_grid_tables)
+    int grid_bytes, ring_bytes;  // set by launch_phase_grid
+};
+
+constexpr int kGridShellChunk = 8;
+constexpr size_t kGridMaxSlice = 4096;        // atoms per tile: the unit of the integer grid grows with them
+constexpr double kGridSigma[2] = {3.0, 4.0};  // grid points per half period at the largest shell, per weight set
+// D(l) of the weights `set`; CTAs per SM for that many grid points and staged frames (0: too many)
+double grid_deconvolution(int set, double l);
+int grid_ctas(int grid_points, int ring_frames);
+// shells: per system [nq] lam_k h / 2 pi, then [nq] 1 / D(lam_k h)
+cudaError_t launch_grid_tables(const GridSystem* systems, int nsys, int max_points, const double* shells, int set,
+                               float2* coef, cudaStream_t st);
+cudaError_t launch_phase_grid(GridLaunch a, int grid_points, int ring_frames, cudaStream_t st);
+
+// ---------------------------------------------------------------------------------------
 // Correlation, store and orientational average
 // ---------------------------------------------------------------------------------------
 enum DspType { DSP_AUTOCORRELATE = 0, DSP_SQUARE = 1, DSP_PLAIN = 2 };
@@ -348,9 +398,10 @@ cudaError_t launch_store_kernel(const double2* tw64, int lg_tw, double2* k64, fl
 // Staging: raw frame-major float [nf][na][3] -> float4 [nf][na_pad] (minus centre); with
 // xyz_rec, also the class-sorted copy xyz_rec[f][rec_inv[j]] = (x, y, z, 1). `raw` may be
 // host memory the device reads in place.
+// With `rmax2` (zeroed by the caller) also the largest |r|^2 of the staged frames, as float bits.
 cudaError_t launch_stage(const float* raw, int nf, int na, int na_pad, double cx, double cy,
                          double cz, int center, float4* xyz, const int* rec_inv, int na_rec,
-                         float4* xyz_rec, cudaStream_t st);
+                         float4* xyz_rec, unsigned int* rmax2, cudaStream_t st);
 // b[s][j] = class_factors[s][cls[j]] (0 for padding atoms), float or double output.
 cudaError_t launch_expand_factors(const double* class_factors, int nclass, int nshell,
                                   const int* cls, int na_pad, int precision, void* b,
