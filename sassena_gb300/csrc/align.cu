@@ -41,22 +41,22 @@ __global__ void pp_promote_kernel(const float* __restrict__ in, size_t n, double
 
 // com[f] = sum_i m_i r_i / sum_i m_i over the list, r_i = base[f * stride + 3 idx[i]]
 // (idx NULL: i), summed in list order without fused multiply-adds, as the reference's loop
-// (center_of_mass.cpp:160-264). One CTA per 32 frames, one frame per lane: tiles of 32 list
-// entries x 32 frames are loaded cooperatively (consecutive threads read consecutive atoms of a
-// frame) and turned into the products m_i r_i in shared memory; then warp w runs accumulator w
-// (m, x, y, z) with lane = frame through the tile in list order.
-constexpr int kComFrames = 32, kComTile = 32, kComThreads = 128;
+// (center_of_mass.cpp:160-264). The sums of a frame are chains of dependent FP64 adds, and GB300's
+// FP64 pipe takes a warp instruction in about 19 clocks however many lanes it has. So one warp
+// runs the four chains (m, x, y, z) of 8 frames in its 32 lanes, and the other warps turn the next
+// tile of 64 list entries x 8 frames into products meanwhile (a warp per accumulator with 32
+// frames a CTA kept 8 SMs busy for 256 frames of 10,000 atoms and took 1.29 ms).
+constexpr int kComFrames = 8, kComTile = 64, kComThreads = 128;
 
 __global__ void __launch_bounds__(kComThreads) pp_com_kernel(const double* __restrict__ base, size_t stride,
                                                              const size_t* __restrict__ idx,
                                                              const double* __restrict__ mass, size_t n, int nf,
                                                              double* __restrict__ com) {
-    __shared__ double S[4][kComTile][kComFrames + 1];
+    __shared__ double S[2][kComTile][32 + 1];  // [entry][accumulator * 8 + frame]
     const int f0 = blockIdx.x * kComFrames, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double acc = 0.0;
-    for (size_t i0 = 0; i0 < n; i0 += kComTile) {
-        for (int t = threadIdx.x; t < kComTile * kComFrames; t += kComThreads) {
-            const int e = t % kComTile, fl = t / kComTile;
+    auto products = [&](size_t i0, int buf, int first, int step) {
+        for (int t = first; t < kComTile * kComFrames; t += step) {
+            const int e = t % kComTile, fl = t / kComTile;  // consecutive threads read consecutive atoms
             const size_t i = i0 + e;
             double mi = 0.0, px = 0.0, py = 0.0, pz = 0.0;
             if (i < n && f0 + fl < nf) {
@@ -67,29 +67,36 @@ __global__ void __launch_bounds__(kComThreads) pp_com_kernel(const double* __res
                 py = __dmul_rn(r[1], mi);
                 pz = __dmul_rn(r[2], mi);
             }
-            S[0][e][fl] = mi;
-            S[1][e][fl] = px;
-            S[2][e][fl] = py;
-            S[3][e][fl] = pz;
+            double* o = &S[buf][e][fl];
+            o[0] = mi;
+            o[8] = px;
+            o[16] = py;
+            o[24] = pz;
         }
-        __syncthreads();
-        const int cnt = (int)min((size_t)kComTile, n - i0);
-        for (int e = 0; e < cnt; ++e) acc = __dadd_rn(acc, S[warp][e][lane]);
+    };
+    double acc = 0.0;
+    products(0, 0, threadIdx.x, kComThreads);
+    __syncthreads();
+    for (size_t i0 = 0; i0 < n; i0 += kComTile) {
+        const int buf = (int)(i0 / kComTile) & 1, cnt = (int)min((size_t)kComTile, n - i0);
+        if (warp == 0) {
+#pragma unroll 8
+            for (int e = 0; e < cnt; ++e) acc = __dadd_rn(acc, S[buf][e][lane]);
+        } else if (i0 + kComTile < n) {
+            products(i0 + kComTile, buf ^ 1, threadIdx.x - 32, kComThreads - 32);
+        }
         __syncthreads();
     }
-    S[warp][0][lane] = acc;  // totals: m, x, y, z of frame f0 + lane
-    __syncthreads();
-    const int f = f0 + lane;
-    if (warp == 0 && f < nf) {
-        double* o = com + 3 * (size_t)f;
-        const double m = S[0][0][lane];
-        if (n == 0) {
-            o[0] = o[1] = o[2] = 0.0;
-        } else {
-            o[0] = __ddiv_rn(S[1][0][lane], m);
-            o[1] = __ddiv_rn(S[2][0][lane], m);
-            o[2] = __ddiv_rn(S[3][0][lane], m);
-        }
+    if (warp) return;
+    // lanes 0 .. 7 gather m, x, y, z of frame f0 + lane
+    const int fl = lane & 7;
+    const double m = __shfl_sync(0xffffffffu, acc, fl), x = __shfl_sync(0xffffffffu, acc, 8 + fl),
+                 y = __shfl_sync(0xffffffffu, acc, 16 + fl), z = __shfl_sync(0xffffffffu, acc, 24 + fl);
+    if (lane < kComFrames && f0 + lane < nf) {
+        double* o = com + 3 * (size_t)(f0 + lane);
+        o[0] = n ? __ddiv_rn(x, m) : 0.0;
+        o[1] = n ? __ddiv_rn(y, m) : 0.0;
+        o[2] = n ? __ddiv_rn(z, m) : 0.0;
     }
 }
 
@@ -145,58 +152,66 @@ __global__ void pp_gather_kernel(const double* __restrict__ W, size_t nsys, cons
 }
 
 // K[f] = sum_i m_i (u_i v_i^T), u_i = R_i - ref, v_i = C[f][i] - pos[f] (center_of_mass.cpp:79-98),
-// R_i = reference[i] or (NULL) C[f][i]; each element m_i * (u_r * v_c), summed in order. Layout as
-// pp_com_kernel: tiles of 16 entries x 32 frames of the nine products in shared memory, then warp w
-// runs elements w, w + 4, w + 8 of K with lane = frame.
-constexpr int kKmatTile = 16;
+// R_i = reference[i] or (NULL) C[f][i]; each element m_i * (u_r * v_c), summed in order. As
+// pp_com_kernel: warp 0 runs the nine chains of FB frames in 9 FB lanes, the other warps form the
+// products of the next 64 entries (256 frames of 10,000 atoms: 4.8 ms with 32 frames a CTA).
+constexpr int kKmatTile = 64, kKmatThreads = 32 + 6 * 32;
 
-__global__ void __launch_bounds__(kComThreads) pp_kmat_kernel(const double* __restrict__ C, const double* __restrict__ ref_xyz,
-                                                              const double* __restrict__ mass, size_t n, int nf,
-                                                              const double* __restrict__ pos, const double* __restrict__ ref,
-                                                              int ref_one, double* __restrict__ K) {
-    __shared__ double S[9][kKmatTile][kComFrames + 1];
-    const int f0 = blockIdx.x * kComFrames, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (size_t i0 = 0; i0 < n; i0 += kKmatTile) {
-        for (int t = threadIdx.x; t < kKmatTile * kComFrames; t += kComThreads) {
-            const int e = t % kKmatTile, fl = t / kKmatTile;
+template <int FB>
+__global__ void __launch_bounds__(kKmatThreads) pp_kmat_kernel(const double* __restrict__ C, const double* __restrict__ ref_xyz,
+                                                               const double* __restrict__ mass, size_t n, int nf,
+                                                               const double* __restrict__ pos, const double* __restrict__ ref,
+                                                               int ref_one, double* __restrict__ K) {
+    __shared__ double S[2][kKmatTile][9 * FB + 1 - (FB & 1)];  // an odd row length: no bank conflicts
+    const int f0 = blockIdx.x * FB, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto products = [&](size_t i0, int buf, int first, int step) {
+        for (int t = first; t < kKmatTile * FB; t += step) {
+            const int e = t % kKmatTile, fl = t / kKmatTile, f = f0 + fl;
             const size_t i = i0 + e;
-            const int f = f0 + fl;
-            double tv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            if (i < n && f < nf) {
-                const double* cf = C + ((size_t)f * n + i) * 3;
-                const double* rr = ref_xyz ? ref_xyz + 3 * i : cf;
-                const double* pf = pos + 3 * (size_t)f;
-                const double* qf = ref + 3 * (size_t)(ref_one ? 0 : f);
-                const double mi = mass[i];
-                double u[3], v[3];
-                for (int d = 0; d < 3; ++d) {
-                    v[d] = __dsub_rn(cf[d], pf[d]);
-                    u[d] = __dsub_rn(rr[d], qf[d]);
-                }
-                for (int r = 0; r < 3; ++r)
-                    for (int c = 0; c < 3; ++c) tv[3 * r + c] = __dmul_rn(mi, __dmul_rn(u[r], v[c]));
+            if (i >= n || f >= nf) continue;
+            const double* cf = C + ((size_t)f * n + i) * 3;
+            const double* rr = ref_xyz ? ref_xyz + 3 * i : cf;
+            const double* pf = pos + 3 * (size_t)f;
+            const double* qf = ref + 3 * (size_t)(ref_one ? 0 : f);
+            const double mi = mass[i];
+            double u[3], v[3];
+            for (int d = 0; d < 3; ++d) {
+                v[d] = __dsub_rn(cf[d], pf[d]);
+                u[d] = __dsub_rn(rr[d], qf[d]);
             }
-#pragma unroll
-            for (int q = 0; q < 9; ++q) S[q][e][fl] = tv[q];
+            for (int r = 0; r < 3; ++r)
+                for (int c = 0; c < 3; ++c) S[buf][e][fl * 9 + 3 * r + c] = __dmul_rn(mi, __dmul_rn(u[r], v[c]));
         }
-        __syncthreads();
-        const int cnt = (int)min((size_t)kKmatTile, n - i0);
-        for (int e = 0; e < cnt; ++e)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int q = warp + 4 * k;
-                if (q < 9) acc[k] = __dadd_rn(acc[k], S[q][e][lane]);
-            }
+    };
+    double acc = 0.0;
+    products(0, 0, threadIdx.x, kKmatThreads);
+    __syncthreads();
+    const bool chain = lane < 9 * FB && f0 + lane / 9 < nf;
+    for (size_t i0 = 0; i0 < n; i0 += kKmatTile) {
+        const int buf = (int)(i0 / kKmatTile) & 1, cnt = (int)min((size_t)kKmatTile, n - i0);
+        if (warp == 0) {
+            if (chain)
+#pragma unroll 8
+                for (int e = 0; e < cnt; ++e) acc = __dadd_rn(acc, S[buf][e][lane]);
+        } else if (i0 + kKmatTile < n) {
+            products(i0 + kKmatTile, buf ^ 1, threadIdx.x - 32, kKmatThreads - 32);
+        }
         __syncthreads();
     }
-    const int f = f0 + lane;
-    if (f < nf)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int q = warp + 4 * k;
-            if (q < 9) K[9 * (size_t)f + q] = acc[k];
-        }
+    if (warp == 0 && chain) K[9 * (size_t)f0 + lane] = acc;
+}
+
+// Frames per CTA: a CTA's FP64 time per entry is about 19 + 14 FB clocks (one add, 24 FB products
+// in full warps), over as many CTAs as share an SM.
+void launch_kmat(const double* C, const double* ref_xyz, const double* mass, size_t n, int nf, const double* pos,
+                 const double* ref, int ref_one, double* K, cudaStream_t st) {
+    const int sms = current_sms();
+    int best = 1;
+    auto cost = [&](int fb) { return ((nf + fb - 1) / fb + sms - 1) / sms * (19 + 14 * fb); };
+    for (int fb = 2; fb <= 3; ++fb)
+        if (cost(fb) < cost(best)) best = fb;
+    auto k = best == 1 ? pp_kmat_kernel<1> : (best == 2 ? pp_kmat_kernel<2> : pp_kmat_kernel<3>);
+    k<<<(unsigned)((nf + best - 1) / best), kKmatThreads, 0, st>>>(C, ref_xyz, mass, n, nf, pos, ref, ref_one, K);
 }
 
 // C[f][i] = R[f] (C[f][i] - pos[f]) + ref (center_of_mass.cpp:114-128; ublas prod order).
@@ -450,7 +465,7 @@ extern "C" int sass_stage_frames_prepass(sass_plan* p, const float* frames, size
     double* C = p->pp_C.as<double>();
     const int nfi = (int)nf;
     const unsigned gf = (unsigned)((nf + kPerFrameThreads - 1) / kPerFrameThreads);
-    const unsigned gw = (unsigned)((nf + 31) / 32);  // the ordered sums: one CTA per 32 frames
+    const unsigned gw = (unsigned)((nf + kComFrames - 1) / kComFrames);  // the ordered sums
     auto L = [&](size_t off) { return reinterpret_cast<const size_t*>(dl + off); };
     auto D = [&](size_t off) { return reinterpret_cast<const double*>(dl + off); };
     std::vector<double> hK(nf * 9), hR(nf * 9);
@@ -497,8 +512,7 @@ extern "C" int sass_stage_frames_prepass(sass_plan* p, const float* frames, size
                         pp_com_kernel<<<1, kComThreads, 0, st>>>(D(o.refxyz), 0, nullptr, D(o.rmass), nref, 1, va);
                     else
                         pp_com_kernel<<<gw, kComThreads, 0, st>>>(C, nref * 3, nullptr, D(o.rmass), nref, nfi, va);
-                    pp_kmat_kernel<<<gw, kComThreads, 0, st>>>(C, ref_one ? D(o.refxyz) : nullptr, D(o.rmass),
-                                                                     nref, nfi, vb, va, ref_one, vK);
+                    launch_kmat(C, ref_one ? D(o.refxyz) : nullptr, D(o.rmass), nref, nfi, vb, va, ref_one, vK, st);
                     PCK(cudaGetLastError());
                     PCK(cudaMemcpyAsync(hK.data(), vK, nf * 9 * sizeof(double), cudaMemcpyDeviceToHost, st));
                     PCK(cudaStreamSynchronize(st));
