@@ -45,16 +45,35 @@ __global__ void pp_promote_kernel(const float* __restrict__ in, size_t n, double
 // FP64 pipe takes a warp instruction in about 19 clocks however many lanes it has. So one warp
 // runs the four chains (m, x, y, z) of 8 frames in its 32 lanes, and the other warps turn the next
 // tile of 64 list entries x 8 frames into products meanwhile (a warp per accumulator with 32
-// frames a CTA kept 8 SMs busy for 256 frames of 10,000 atoms and took 1.29 ms).
-constexpr int kComFrames = 8, kComTile = 64, kComThreads = 128;
+// frames a CTA kept 8 SMs busy for 256 frames of 10,000 atoms: 1.29 ms, now 0.42).
+constexpr int kComFrames = 8, kComTile = 64, kComThreads = 32 + 8 * 32;
 
-__global__ void __launch_bounds__(kComThreads) pp_com_kernel(const double* __restrict__ base, size_t stride,
-                                                             const size_t* __restrict__ idx,
-                                                             const double* __restrict__ mass, size_t n, int nf,
-                                                             double* __restrict__ com) {
+struct ComJob {
+    const double* base;
+    size_t stride;
+    const size_t* idx;
+    const double* mass;
+    size_t n;
+    int nf;
+    double* com;
+};
+
+// Two lists in one launch (second.nf = 0: one): a chain waits about 80 clocks for each add, 0.4 ms
+// for 10,000 entries, whatever else runs.
+__global__ void __launch_bounds__(kComThreads) pp_com_kernel(const ComJob first_job, const ComJob second, int first_blocks) {
+    const bool one = (int)blockIdx.x < first_blocks;
+    const ComJob& jb = one ? first_job : second;
+    const double* __restrict__ base = jb.base;
+    const size_t stride = jb.stride, n = jb.n;
+    const size_t* __restrict__ idx = jb.idx;
+    const double* __restrict__ mass = jb.mass;
+    const int nf = jb.nf;
+    double* __restrict__ com = jb.com;
     __shared__ double S[2][kComTile][32 + 1];  // [entry][accumulator * 8 + frame]
-    const int f0 = blockIdx.x * kComFrames, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int f0 = ((int)blockIdx.x - (one ? 0 : first_blocks)) * kComFrames, warp = threadIdx.x >> 5,
+              lane = threadIdx.x & 31;
     auto products = [&](size_t i0, int buf, int first, int step) {
+#pragma unroll 2
         for (int t = first; t < kComTile * kComFrames; t += step) {
             const int e = t % kComTile, fl = t / kComTile;  // consecutive threads read consecutive atoms
             const size_t i = i0 + e;
@@ -98,6 +117,11 @@ __global__ void __launch_bounds__(kComThreads) pp_com_kernel(const double* __res
         o[1] = n ? __ddiv_rn(y, m) : 0.0;
         o[2] = n ? __ddiv_rn(z, m) : 0.0;
     }
+}
+
+void launch_com(const ComJob& a, const ComJob& b, cudaStream_t st) {
+    const int na = (a.nf + kComFrames - 1) / kComFrames, nb = (b.nf + kComFrames - 1) / kComFrames;
+    pp_com_kernel<<<(unsigned)(na + nb), kComThreads, 0, st>>>(a, b, na);
 }
 
 // Per-frame translation vectors. a, b: [nf][3] or one row broadcast (a_one, b_one).
@@ -154,7 +178,8 @@ __global__ void pp_gather_kernel(const double* __restrict__ W, size_t nsys, cons
 // K[f] = sum_i m_i (u_i v_i^T), u_i = R_i - ref, v_i = C[f][i] - pos[f] (center_of_mass.cpp:79-98),
 // R_i = reference[i] or (NULL) C[f][i]; each element m_i * (u_r * v_c), summed in order. As
 // pp_com_kernel: warp 0 runs the nine chains of FB frames in 9 FB lanes, the other warps form the
-// products of the next 64 entries (256 frames of 10,000 atoms: 4.8 ms with 32 frames a CTA).
+// products of the next 64 entries (256 frames of 10,000 atoms: 4.8 ms with 32 frames a CTA, now
+// 0.45).
 constexpr int kKmatTile = 64, kKmatThreads = 32 + 6 * 32;
 
 template <int FB>
@@ -465,7 +490,6 @@ extern "C" int sass_stage_frames_prepass(sass_plan* p, const float* frames, size
     double* C = p->pp_C.as<double>();
     const int nfi = (int)nf;
     const unsigned gf = (unsigned)((nf + kPerFrameThreads - 1) / kPerFrameThreads);
-    const unsigned gw = (unsigned)((nf + kComFrames - 1) / kComFrames);  // the ordered sums
     auto L = [&](size_t off) { return reinterpret_cast<const size_t*>(dl + off); };
     auto D = [&](size_t off) { return reinterpret_cast<const double*>(dl + off); };
     std::vector<double> hK(nf * 9), hR(nf * 9);
@@ -476,26 +500,22 @@ extern "C" int sass_stage_frames_prepass(sass_plan* p, const float* frames, size
         const size_t nsel = q.nselection, nref = q.nreference;
         // centre of mass of the reference structure -> va ([1][3] when it is constant)
         const bool ref_one = q.reference != nullptr;
-        auto com_ref = [&](double* out) {
-            if (ref_one)
-                pp_com_kernel<<<1, kComThreads, 0, st>>>(D(o.refxyz), 0, nullptr, D(o.rmass), nref, 1, out);
-            else
-                pp_com_kernel<<<gw, kComThreads, 0, st>>>(W, nsys * 3, L(o.ref), D(o.rmass), nref, nfi, out);
-        };
+        const ComJob none{};
+        const ComJob com_ref = ref_one ? ComJob{D(o.refxyz), 0, nullptr, D(o.rmass), nref, 1, va}
+                                       : ComJob{W, nsys * 3, L(o.ref), D(o.rmass), nref, nfi, va};
         switch (q.type) {
             case SASS_STEP_CENTER:
-                com_ref(va);
+                launch_com(com_ref, none, st);
                 pp_combine_kernel<<<gf, kPerFrameThreads, 0, st>>>(va, ref_one, nullptr, 0, 0, nfi, vt);
                 if (nsel) pp_translate_kernel<<<grid_for(nf * nsel, 256), 256, 0, st>>>(W, nsys, L(o.sel), nsel, nfi, vt);
                 break;
             case SASS_STEP_FITTRANS:
-                com_ref(va);
-                pp_com_kernel<<<gw, kComThreads, 0, st>>>(W, nsys * 3, L(o.sel), D(o.smass), nsel, nfi, vb);
+                launch_com(com_ref, ComJob{W, nsys * 3, L(o.sel), D(o.smass), nsel, nfi, vb}, st);
                 pp_combine_kernel<<<gf, kPerFrameThreads, 0, st>>>(va, ref_one, vb, 0, 1, nfi, vt);
                 if (nsel) pp_translate_kernel<<<grid_for(nf * nsel, 256), 256, 0, st>>>(W, nsys, L(o.sel), nsel, nfi, vt);
                 break;
             case SASS_STEP_MOTION:
-                com_ref(va);
+                launch_com(com_ref, none, st);
                 if (nsel)
                     pp_motion_kernel<<<grid_for(nf * nsel, 256), 256, 0, st>>>(W, nsys, L(o.sel), nsel, nfi, va, ref_one,
                                                                               D(o.trans));
@@ -503,15 +523,12 @@ extern "C" int sass_stage_frames_prepass(sass_plan* p, const float* frames, size
             default: {  // FITROTTRANS, FITROT
                 const bool rot_only = q.type == SASS_STEP_FITROT;
                 if (rot_only)  // centre of mass of the moved atoms before the fit
-                    pp_com_kernel<<<gw, kComThreads, 0, st>>>(W, nsys * 3, L(o.sel), D(o.smass), nsel, nfi, vc);
+                    launch_com(ComJob{W, nsys * 3, L(o.sel), D(o.smass), nsel, nfi, vc}, none, st);
                 if (nref) {
                     pp_gather_kernel<<<grid_for(nf * nref * 3, 256), 256, 0, st>>>(W, nsys, L(o.ref), nref, nfi, C);
                     // pos: the copy's centre; ref: the reference structure's (the copy itself when instant)
-                    pp_com_kernel<<<gw, kComThreads, 0, st>>>(C, nref * 3, nullptr, D(o.rmass), nref, nfi, vb);
-                    if (ref_one)
-                        pp_com_kernel<<<1, kComThreads, 0, st>>>(D(o.refxyz), 0, nullptr, D(o.rmass), nref, 1, va);
-                    else
-                        pp_com_kernel<<<gw, kComThreads, 0, st>>>(C, nref * 3, nullptr, D(o.rmass), nref, nfi, va);
+                    launch_com(ComJob{C, nref * 3, nullptr, D(o.rmass), nref, nfi, vb},
+                               ref_one ? com_ref : ComJob{C, nref * 3, nullptr, D(o.rmass), nref, nfi, va}, st);
                     launch_kmat(C, ref_one ? D(o.refxyz) : nullptr, D(o.rmass), nref, nfi, vb, va, ref_one, vK, st);
                     PCK(cudaGetLastError());
                     PCK(cudaMemcpyAsync(hK.data(), vK, nf * 9 * sizeof(double), cudaMemcpyDeviceToHost, st));
