@@ -158,6 +158,95 @@ __device__ void forward_tile(Smem& s, int n) {
     __syncthreads();
 }
 
+// ---- forward only (inference, quadrature) ----------------------------------------------------
+// Shared memory of a CTA that keeps nothing for a backward pass: 47 KB, four CTAs per SM where
+// the training layout (200 KB) left one.
+struct SmemF {
+    float w1[H * 4], b1[H], b2[H], w3[H], b3, pad0[3];
+    float x[TB * 4], y[TB], ypart[NT / 32][TB];
+    __nv_bfloat16 w2[H * HP];  // read once, into the fragments
+    __nv_bfloat16 h1[TB * HP];
+};
+
+// The layer-2 operand of warp w: columns j in [32 w, 32 w + 32) for every k, in registers.
+struct FragB {
+    uint32_t b[4][8][2];
+};
+
+__device__ void load_weights(SmemF& s, const __nv_bfloat16* __restrict__ w, FragB& f) {
+    for (int i = threadIdx.x; i < H * 4; i += NT) s.w1[i] = bf(w, OW1 + i);
+    for (int i = threadIdx.x; i < H * H; i += NT) s.w2[i / H * HP + i % H] = w[OW2 + i];
+    for (int i = threadIdx.x; i < H; i += NT) {
+        s.b1[i] = bf(w, OB1 + i);
+        s.b2[i] = bf(w, OB2 + i);
+        s.w3[i] = bf(w, OW3 + i);
+    }
+    if (threadIdx.x == 0) s.b3 = bf(w, OB3);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+            const __nv_bfloat16* b = s.w2 + (size_t)(32 * warp + 8 * nt + g) * HP + 16 * ks + 2 * t;
+            f.b[nt][ks][0] = ld2(b);
+            f.b[nt][ks][1] = ld2(b + 8);
+        }
+}
+
+// As the training forward, with the same operations in the same order (the same bits).
+__device__ __forceinline__ void forward_tile(SmemF& s, const FragB& f, int n) {
+    const int j = threadIdx.x, warp = j >> 5, lane = j & 31, g = lane >> 2, t = lane & 3;
+    {
+        const float4 w1 = *reinterpret_cast<const float4*>(s.w1 + j * 4);
+        const float b1 = s.b1[j];
+#pragma unroll 4
+        for (int b = 0; b < TB; ++b) {
+            const float4 x = *reinterpret_cast<const float4*>(s.x + b * 4);
+            const float z = fmaf(w1.w, x.w, fmaf(w1.z, x.z, fmaf(w1.y, x.y, fmaf(w1.x, x.x, b1))));
+            s.h1[b * HP + j] = __float2bfloat16_rn(b < n ? tanhf(z) : 0.f);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+        float d[4][4];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d[nt][e] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+            const __nv_bfloat16* a = s.h1 + (size_t)(16 * mt + g) * HP + 16 * ks + 2 * t;
+            const uint32_t a0 = ld2(a), a1 = ld2(a + 8 * HP), a2 = ld2(a + 8), a3 = ld2(a + 8 * HP + 8);
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) mma_bf16(d[nt], a0, a1, a2, a3, f.b[nt][ks][0], f.b[nt][ks][1]);
+        }
+        float yp[2] = {0.f, 0.f};  // rows g, g + 8
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int jj = 32 * warp + 8 * nt + 2 * t + (e & 1);
+                yp[e >> 1] = fmaf(s.w3[jj], tanhf(d[nt][e] + s.b2[jj]), yp[e >> 1]);
+            }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float v = yp[r];
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (t == 0) s.ypart[warp][16 * mt + g + 8 * r] = v;
+        }
+    }
+    __syncthreads();
+    if (j < TB) {
+        float y = s.b3;
+        for (int w = 0; w < NT / 32; ++w) y += s.ypart[w][j];
+        s.y[j] = y;
+    }
+    __syncthreads();
+}
+
 }  // namespace
 
 __global__ void __launch_bounds__(NT) mlp_train_kernel(const __nv_bfloat16* __restrict__ w,
@@ -286,57 +375,68 @@ __global__ void mlp_adam_kernel(float* __restrict__ master, __nv_bfloat16* __res
     }
 }
 
-__global__ void __launch_bounds__(NT) mlp_forward_kernel(const __nv_bfloat16* __restrict__ w,
-                                                         const float* __restrict__ X, int n, float* __restrict__ Y) {
+__global__ void __launch_bounds__(NT, 4) mlp_forward_kernel(const __nv_bfloat16* __restrict__ w,
+                                                            const float* __restrict__ X, int n, float* __restrict__ Y) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-    load_weights(s, w, false);
-    __syncthreads();
+    SmemF& s = *reinterpret_cast<SmemF*>(smem_raw);
+    FragB f;
+    load_weights(s, w, f);
     const int ntiles = (n + TB - 1) / TB;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int b0 = tile * TB, nb = min(TB, n - b0);
         for (int i = threadIdx.x; i < TB * 4; i += NT) s.x[i] = (i / 4) < nb ? X[(size_t)b0 * 4 + i] : 0.f;
         __syncthreads();
-        forward_tile(s, nb);
+        forward_tile(s, f, nb);
         if (threadIdx.x < nb) Y[b0 + threadIdx.x] = s.y[threadIdx.x];
         __syncthreads();
     }
 }
 
-// Mean of g = exp(y * y_std + y_mean) over a spherical-Fibonacci set of P points on
-// each shell: gbar[s] (FP64). One CTA per (shell, chunk of points); per-CTA FP64
-// partials are added with atomics (fixed count per shell, order-independent to ~1e-16).
-__global__ void __launch_bounds__(NT) mlp_sphere_kernel(const __nv_bfloat16* __restrict__ w,
-                                                        const double* __restrict__ qlen, int nshell, int P,
-                                                        int chunks, float q_mid, float q_half, float y_mean,
-                                                        float y_std, double* __restrict__ part) {
+// The spherical-Fibonacci set: P unit vectors, the same for every shell (FP64 sines are slow on
+// GB300, and each shell's tiles recomputed them).
+__global__ void mlp_points_kernel(int P, float* __restrict__ pts) {
+    const double golden = 3.14159265358979323846 * (3.0 - 2.23606797749978969641);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
+        const double z = 1.0 - 2.0 * (i + 0.5) / P;
+        const double r = sqrt(fmax(0.0, 1.0 - z * z));
+        double sn, cs;
+        sincos(golden * (i + 0.5), &sn, &cs);
+        pts[3 * (size_t)i] = (float)(r * cs);
+        pts[3 * (size_t)i + 1] = (float)(r * sn);
+        pts[3 * (size_t)i + 2] = (float)z;
+    }
+}
+
+// Mean of g = exp(y * y_std + y_mean) over the spherical-Fibonacci set of P points on each
+// shell: gbar[s] (FP64). One CTA per (shell, chunk of points), partials added in chunk order.
+// Bound by the tanh evaluations (256 per point, about 22 instructions each) and the latency
+// between a tile's three barriers, which four CTAs per SM hide: 24 shells x 32,768 points take
+// 0.25 ms (1.53 ms with the training kernel's layout and each tile's points computed in FP64).
+__global__ void __launch_bounds__(NT, 4) mlp_sphere_kernel(const __nv_bfloat16* __restrict__ w,
+                                                           const double* __restrict__ qlen,
+                                                           const float* __restrict__ pts, int nshell, int P,
+                                                           int chunks, float q_mid, float q_half, float y_mean,
+                                                           float y_std, double* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
+    SmemF& s = *reinterpret_cast<SmemF*>(smem_raw);
     __shared__ double red[NT / 32];
-    load_weights(s, w, false);
-    __syncthreads();
+    FragB f;
+    load_weights(s, w, f);
     const int sh = blockIdx.x / chunks, c = blockIdx.x % chunks;
     const int per = (P + chunks - 1) / chunks, p0 = c * per, p1 = min(P, p0 + per);
     const float sq = (float)((qlen[sh] - q_mid) / q_half);
-    const double golden = 3.14159265358979323846 * (3.0 - 2.23606797749978969641);
     double acc = 0.0;
     for (int b0 = p0; b0 < p1; b0 += TB) {
         const int nb = min(TB, p1 - b0);
-        if (threadIdx.x < TB) {
-            const int i = b0 + threadIdx.x;
-            const double z = 1.0 - 2.0 * (i + 0.5) / P;
-            const double r = sqrt(fmax(0.0, 1.0 - z * z));
-            double sn, cs;
-            sincos(golden * (i + 0.5), &sn, &cs);
-            s.x[threadIdx.x * 4 + 0] = (float)(r * cs);
-            s.x[threadIdx.x * 4 + 1] = (float)(r * sn);
-            s.x[threadIdx.x * 4 + 2] = (float)z;
-            s.x[threadIdx.x * 4 + 3] = sq;
+        if (threadIdx.x < 3 * TB) {
+            const int b = threadIdx.x / 3;
+            s.x[b * 4 + threadIdx.x % 3] = b < nb ? pts[3 * (size_t)b0 + threadIdx.x] : 0.f;
+        } else {
+            s.x[(threadIdx.x - 3 * TB) * 4 + 3] = sq;
         }
         __syncthreads();
-        forward_tile(s, nb);
+        forward_tile(s, f, nb);
         if (threadIdx.x < nb) acc += exp((double)s.y[threadIdx.x] * y_std + y_mean);
-        __syncthreads();
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -371,7 +471,7 @@ __global__ void scale_series_kernel(T2* __restrict__ A, const double* __restrict
     }
 }
 
-size_t mlp_smem_bytes(bool) { return sizeof(Smem); }
+size_t mlp_smem_bytes(bool train) { return train ? sizeof(Smem) : sizeof(SmemF); }
 
 size_t mlp_train_scratch_bytes(int sms) {
     return (size_t)std::max(sms, 1) * ((size_t)kMlpParams * sizeof(float) + sizeof(double));
@@ -408,12 +508,11 @@ cudaError_t launch_mlp_forward(const __nv_bfloat16* w, const float* X, int n, fl
     return cudaGetLastError();
 }
 
-static int sphere_chunks(int nshell, int P, int sms) {
-    return max(1, min((P + 1023) / 1024, (max(sms, 1) * 4 + nshell - 1) / nshell));
-}
+// Chunks per shell: one wave of four CTAs per SM, at least 256 points each.
+static int sphere_chunks(int nshell, int P, int sms) { return max(1, min((P + 255) / 256, max(sms, 1) * 4 / nshell)); }
 
 size_t mlp_sphere_scratch_bytes(int nshell, int P, int sms) {
-    return (size_t)nshell * sphere_chunks(nshell, P, sms) * sizeof(double);
+    return (size_t)nshell * sphere_chunks(nshell, P, sms) * sizeof(double) + (size_t)P * 3 * sizeof(float);
 }
 
 cudaError_t launch_mlp_sphere(const __nv_bfloat16* w, const double* qlen, int nshell, int P, float q_mid,
@@ -423,7 +522,9 @@ cudaError_t launch_mlp_sphere(const __nv_bfloat16* w, const double* qlen, int ns
     cudaError_t e = cudaFuncSetAttribute(mlp_sphere_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     const int chunks = sphere_chunks(nshell, P, sms);
-    mlp_sphere_kernel<<<nshell * chunks, NT, sm, st>>>(w, qlen, nshell, P, chunks, q_mid, q_half, y_mean, y_std,
+    float* pts = reinterpret_cast<float*>(scratch + (size_t)nshell * chunks);
+    mlp_points_kernel<<<grid_blocks((size_t)P, 128, 8), 128, 0, st>>>(P, pts);
+    mlp_sphere_kernel<<<nshell * chunks, NT, sm, st>>>(w, qlen, pts, nshell, P, chunks, q_mid, q_half, y_mean, y_std,
                                                        scratch);
     mlp_sphere_reduce_kernel<<<(nshell + 127) / 128, 128, 0, st>>>(scratch, nshell, chunks, P, gbar);
     return cudaGetLastError();
