@@ -680,6 +680,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         lg_min_ = std::min(lg_min_, it.sys->lg);
         nf_max_ = std::max(nf_max_, (int)it.sys->nf);
     }
+    self_fx_ = !coherent && self_fx_supported(cfg.precision, cfg.dsp, lg_min_, lg_max_);
     PhaseShape shape = cfg.shape.q_per_lane ? cfg.shape : default_shape(cfg.precision, min_nm);
     if (coherent && !phase_shape_supported(cfg.precision, shape)) {
         err = "phase tile shape not instantiated";
@@ -1040,8 +1041,14 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     std::vector<FxSystem> fsys(items.size());
     std::vector<FxTileDesc> ftiles;
     fxq_off_.assign(items.size(), 0);
+    fx_self_item_.assign(items.size(), 0);
     size_t fxq_total = 0;
     for (size_t i = 0; i < items.size(); ++i) {
+        fx_self_item_[i] = self_fx_ && !long_item[i];
+        if (fx_self_item_[i]) {
+            fxq_off_[i] = fxq_total;
+            fxq_total += items[i].offs.back();
+        }
         if (!fx_on_[i]) continue;
         const WorkItem& it = items[i];
         SystemState& s = *it.sys;
@@ -1079,15 +1086,15 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         return a.b_end - a.b_begin > b.b_end - b.b_begin;
     });
     nfx_tiles_ = (int)ftiles.size();
-    if (nfx_tiles_) {
+    if (fxq_total) {
         ECK(fxq_.ensure(fxq_total * kFxQBytes));
         if (!fxtab_.p) {
             ECK(fxtab_.ensure(kFxTableGlobalBytes));
             ECK(launch_fx_table(fxtab_.p, 0));
         }
         for (size_t i = 0; i < items.size(); ++i)
-            if (fx_on_[i])
-                fsys[i].qw = reinterpret_cast<const uint4*>(fxq_.as<unsigned char>() + fxq_off_[i] * kFxQBytes);
+            fsys[i].qw = csys[i].qw =
+                reinterpret_cast<const uint4*>(fxq_.as<unsigned char>() + fxq_off_[i] * kFxQBytes);
     }
 
     // gridded tiles: directions x frames of a warp's lanes, 8 warps' frames, atom slice
@@ -1185,7 +1192,9 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
             weighted_ = true;
             item_wsqrt_[i] = items[i].d_wsqrt;
         }
-    const size_t per_shell = std::max<size_t>(1, ((size_t)sms * 8 + total_shells - 1) / total_shells);
+    // (the fixed-point incoherent kernel runs one CTA per SM: two waves of them)
+    const size_t per_shell = self_fx_ ? std::max<size_t>(1, (size_t)sms * 2 / total_shells)
+                                      : std::max<size_t>(1, ((size_t)sms * 8 + total_shells - 1) / total_shells);
     size_t poff = 0;
     int slot = 0;
     for (size_t i = 0; i < items.size(); ++i) {
@@ -1495,7 +1504,17 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
     cl.apart = apart_.as<double2>();
     cl.a2part = a2part_.as<double>();
     cl.err = err_.as<unsigned>();
-    ECK(coherent ? launch_corr_accumulate(cl, st) : launch_self_accumulate(cl, st));
+    if (self_fx_) {
+        for (int i = 0; i < nitems_; ++i) {
+            if (fx_self_item_[i] == 0) continue;
+            ECK(launch_fx_q(item_qv_[i], item_offs_[i].back(), fxq_.as<unsigned char>() + fxq_off_[i] * kFxQBytes, st));
+            ++launches;
+        }
+        cl.fx_table = fxtab_.p;
+        ECK(launch_self_fx(cl, st));
+    } else {
+        ECK(coherent ? launch_corr_accumulate(cl, st) : launch_self_accumulate(cl, st));
+    }
     ++launches;
     for (const LongItem& li : long_items_) {
         SystemState& s = *item_sys_[li.item];

@@ -178,7 +178,7 @@ private:
     int nphase_systems_ = 0, ntiles_ = 0, nchunks_ = 0, nentries_ = 0;
     int nrec_tiles_ = 0, nrec_groups_ = 0, rec_k_ = 0;
     // fixed-point phase sum (FP64 form)
-    std::vector<char> fx_on_;
+    std::vector<char> fx_on_, fx_self_item_;
     std::vector<size_t> fxq_off_;  // sub-vector offset of each item's fixed-point words
     // gridded phase sum (FP32 form)
     int ngrid_tiles_ = 0, ngrid_systems_ = 0, grid_points_ = 0, grid_frames_ = 1, grid_set_ = 0, grid_table_ = 0;
@@ -186,6 +186,7 @@ private:
     GridTileDesc* d_gtiles_ = nullptr;
     double* d_gshells_ = nullptr;
     DevBuf grid_ws_;
+    bool self_fx_ = false;         // fixed-point incoherent autocorrelation
     int nfx_tiles_ = 0;
     FxSystem* d_fsys_ = nullptr;
     FxTileDesc* d_ftiles_ = nullptr;

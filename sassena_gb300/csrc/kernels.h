@@ -260,6 +260,7 @@ struct CorrSystem {
     const int* shell_v;     // [nshell+1] sub-vector offsets of each shell
     const void* kbr;        // [L] bit-reversed store kernel: float2 (FP32) or double2 (FP64)
     const float4* qrev;     // FP32 form: sub-vectors in revolutions (q / 2 pi) [nv]
+    const uint4* qw;        // fixed-point form: the sub-vectors' words (launch_fx_q)
     double cx, cy, cz;      // frame centre (FP32 form) for the plain-dsp phase restore
     int nf, lg, na_pad;
 };
@@ -291,10 +292,15 @@ struct CorrLaunch {
     double2* apart;         // [nslot]
     double* a2part;         // [nslot]
     unsigned int* err;
+    const void* fx_table;   // fixed-point form: launch_fx_table
 };
 
 cudaError_t launch_corr_accumulate(const CorrLaunch& a, cudaStream_t st);  // coherent
 cudaError_t launch_self_accumulate(const CorrLaunch& a, cudaStream_t st);  // incoherent
+// Incoherent autocorrelation of the FP64 form in fixed point (padded lengths 64 .. 256, one length
+// per launch). Few large chunks: a CTA fills an SM.
+bool self_fx_supported(int precision, int dsp, int lg_min, int lg_max);
+cudaError_t launch_self_fx(const CorrLaunch& a, cudaStream_t st);
 
 // Per-shell finalisation entry.
 struct FinalEntry {

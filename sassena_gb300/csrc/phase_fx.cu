@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "fx.cuh"
 #include "kernels.h"
 
 namespace sassgpu {
@@ -39,12 +40,10 @@ namespace sassgpu {
 namespace {
 
 constexpr int kFxWarps = 24;           // one CTA per SM
-constexpr int kFxTable = 1024;         // grid angles per revolution
 constexpr int kFxFold = 4;             // blocks of 32 atoms per fold: 2^62 in units of 2^-55
 constexpr int kFxTableBytes = kFxTable * 128;
 constexpr int kFxRecord = 32 * 48;     // a block's records: integers, floats, residuals
 constexpr int kFxSmem = kFxTableBytes + kFxWarps * kFxRecord;
-constexpr unsigned kFxBig = 0x49800000u;  // float bits of 2^20
 
 // (cos, sin)(2 pi i / 1024) in units of 2^-55: Taylor series in 2^-62 on the first octant.
 __global__ void fx_table_kernel(longlong2* __restrict__ out) {
@@ -117,28 +116,6 @@ __global__ void fx_q_kernel(const double* __restrict__ qv, size_t nv, uint4* __r
             out[4 * v + 3].x = 1u;  // every writer stores the same value; cleared before the launch
         }
     }
-}
-
-struct FxQ {
-    unsigned w1[3], w2[3];  // Q in units of 2^-(33 + E) (integer part, 64 bits)
-    float w0[3];            // its next 32 bits, times 2^-32
-    unsigned hi0, lo0;      // minus the phase of the coordinates' offset 2^31
-};
-
-// Q at block exponent E (coordinates below 2^E): the 2^-96 words shifted down by 31 - E.
-__device__ __forceinline__ void fx_shift_q(const uint4* __restrict__ t, int E, FxQ& q) {
-    const int s = 31 - E;  // 11 .. 31
-    unsigned long long p0 = 0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const uint4 w = __ldg(t + c);
-        q.w0[c] = __uint2float_rn(__funnelshift_r(w.x, w.y, s)) * 2.3283064365386963e-10f;
-        q.w1[c] = __funnelshift_r(w.y, w.z, s);
-        q.w2[c] = __funnelshift_r(w.z, w.w, s);
-        p0 -= (((unsigned long long)q.w2[c] << 32) | q.w1[c]) << 31;
-    }
-    q.hi0 = (unsigned)(p0 >> 32);
-    q.lo0 = (unsigned)p0;
 }
 
 struct FxSums {
