@@ -419,13 +419,16 @@ cudaError_t launch_long_means(const CorrChunk* chunks, int nchunks, const double
 // The last kTail lags of a coherent FP64 shell, summed directly: there the 1/(NF - tau)
 // normalisation multiplies the transforms' rounding by up to NF (30,000 frames: 4e-13 of
 // S(q,0) at the last lag), while a lag has only NF - tau products per series.
-constexpr int kTail = 8;
+constexpr int kTail = kTailLags;
 __global__ void __launch_bounds__(256) long_tail_kernel(LongFinal a) {
     const FinalEntry e = a.entries[blockIdx.x];
     const int nf = e.nf, v1 = a.shell_v[blockIdx.x + 1];
     double2 acc[kTail];  // acc[k]: lag nf - 1 - k, k + 1 products
 #pragma unroll
     for (int k = 0; k < kTail; ++k) acc[k] = make_double2(0.0, 0.0);
+    int bad = 0;  // where a series is not finite, no lag is
+    for (int s = e.slot_begin + (int)threadIdx.x; s < e.slot_end; s += 256)
+        bad |= !isfinite(a.apart[s].x) || !isfinite(a.apart[s].y);
     for (int v = a.shell_v[blockIdx.x] + (int)threadIdx.x; v < v1; v += 256) {
         const double2* s = a.A + (size_t)v * nf;
         double2 x[kTail], y[kTail];
@@ -448,11 +451,11 @@ __global__ void __launch_bounds__(256) long_tail_kernel(LongFinal a) {
         }
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][k] = acc[k];
     }
-    __syncthreads();
+    bad = __syncthreads_or(bad);
     if (threadIdx.x < kTail) {
         double2 z = part[0][threadIdx.x];
         for (int w = 1; w < 8; ++w) z = cadd(z, part[w][threadIdx.x]);
-        const double f = e.inv_nm / (double)(threadIdx.x + 1);
+        const double f = (bad ? nan("") : 1.0) * e.inv_nm / (double)(threadIdx.x + 1);
         e.fqt[nf - 1 - threadIdx.x] = make_double2(z.x * f, (a.conj_out ? -z.y : z.y) * f);
     }
 }

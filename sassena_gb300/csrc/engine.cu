@@ -1181,6 +1181,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     // ---- correlation chunks and finalisation entries ------------------------------------------
     std::vector<CorrChunk> chunks;
     std::vector<FinalEntry> entries, entries_w;
+    std::vector<TailEntry> tails, tails_w;
     weighted_ = false;
     item_wsqrt_.assign(items.size(), nullptr);
     for (size_t i = 0; i < items.size(); ++i)
@@ -1197,6 +1198,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
                                       : std::max<size_t>(1, ((size_t)sms * 8 + total_shells - 1) / total_shells);
     size_t poff = 0;
     int slot = 0;
+    tails_ = false;
     for (size_t i = 0; i < items.size(); ++i) {
         if (long_item[i]) continue;
         const WorkItem& it = items[i];
@@ -1215,6 +1217,14 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
             e.fq = it.d_fq + sh;
             e.fq2 = it.d_fq2 + sh;
             e.f32pair = corr_writes_f32_pairs(cfg.precision, cfg.dsp, lg_max_) ? 1 : 0;
+            // from 128 frames on: below, the transforms' rounding stays under FP32's own
+            TailEntry tail{};
+            if (f32 && coherent && autoc && s.nf >= 128) {
+                tail.A = static_cast<const float2*>(item_amp_[i]) + it.offs[sh] * s.nf;
+                tail.nv = it.offs[sh + 1] - it.offs[sh];
+                tails_ = true;
+            }
+            tails.push_back(tail);
             const size_t units = coherent ? it.offs[sh + 1] - it.offs[sh] : s.na;
             const size_t g = std::min(per_shell, units);
             const size_t len = (units + g - 1) / g;
@@ -1237,6 +1247,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
                 ew.fq = it.d_fq_w + sh;
                 ew.fq2 = it.d_fq2_w + sh;
                 entries_w.push_back(ew);
+                tails_w.push_back(tail);
             }
         }
     }
@@ -1361,7 +1372,8 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     // CorrSystem.shell_v points into the blob: patch with the final device address
     ECK(blob_.ensure(blob.size() + 8192 + csys.size() * sizeof(CorrSystem) + fsys.size() * sizeof(FxSystem) +
                      (chunks.size() + lchunks.size()) * sizeof(CorrChunk) +
-                     (entries.size() + entries_w.size() + lentries.size()) * sizeof(FinalEntry) + 4096));
+                     (entries.size() + entries_w.size() + lentries.size()) * sizeof(FinalEntry) +
+                     (tails.size() + tails_w.size()) * sizeof(TailEntry) + 4096));
     item_shell_v_.assign(items.size(), nullptr);
     for (size_t i = 0; i < items.size(); ++i) {
         item_shell_v_[i] = reinterpret_cast<const int*>(blob_.as<unsigned char>() + shell_off[i]);
@@ -1370,6 +1382,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     size_t o_fsys = push(blob, fsys);
     size_t o_csys = push(blob, csys), o_chunks = push(blob, chunks), o_entries = push(blob, entries);
     size_t o_entries_w = push(blob, entries_w);
+    size_t o_tails = push(blob, tails), o_tails_w = push(blob, tails_w);
     size_t o_lchunks = push(blob, lchunks), o_lentries = push(blob, lentries);
     if (blob.size() > blob_.bytes) {
         err = "descriptor blob sizing";
@@ -1393,6 +1406,8 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     d_chunks_ = reinterpret_cast<CorrChunk*>(base + o_chunks);
     d_entries_ = reinterpret_cast<FinalEntry*>(base + o_entries);
     d_entries_w_ = reinterpret_cast<FinalEntry*>(base + o_entries_w);
+    d_tails_ = tails_ ? reinterpret_cast<TailEntry*>(base + o_tails) : nullptr;
+    d_tails_w_ = tails_ ? reinterpret_cast<TailEntry*>(base + o_tails_w) : nullptr;
     d_long_chunks_ = reinterpret_cast<CorrChunk*>(base + o_lchunks);
     d_long_entries_ = reinterpret_cast<FinalEntry*>(base + o_lentries);
     ECK(cudaDeviceSynchronize());
@@ -1572,6 +1587,7 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
     fl.conj_out = cfg_.dsp == DSP_AUTOCORRELATE && cfg_.method == 1;
     fl.entries = d_entries_;
     fl.nentries = nentries_;
+    fl.tails = d_tails_;
     fl.lg_max = lg_max_;
     fl.ppart = ppart_.as<double>();
     fl.apart = apart_.as<double2>();
@@ -1611,6 +1627,7 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
         ECK(launch_corr_accumulate(cl, st));
         FinalLaunch fw = fl;
         fw.entries = d_entries_w_;
+        fw.tails = d_tails_w_;
         int nw = 0;
         for (int i = 0; i < nitems_; ++i)
             if (item_wsqrt_[i]) nw += (int)item_nq_[i];

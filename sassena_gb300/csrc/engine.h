@@ -176,6 +176,7 @@ private:
     std::vector<SystemState*> item_sys_;
     std::vector<size_t> item_nq_;
     int nphase_systems_ = 0, ntiles_ = 0, nchunks_ = 0, nentries_ = 0;
+    bool tails_ = false;
     int nrec_tiles_ = 0, nrec_groups_ = 0, rec_k_ = 0;
     // fixed-point phase sum (FP64 form)
     std::vector<char> fx_on_, fx_self_item_;
@@ -203,6 +204,7 @@ private:
     CorrChunk* d_chunks_ = nullptr;
     FinalEntry* d_entries_ = nullptr;
     FinalEntry* d_entries_w_ = nullptr;  // weighted outputs (same slots)
+    TailEntry *d_tails_ = nullptr, *d_tails_w_ = nullptr;  // one per entry
     std::vector<const double*> item_wsqrt_;
     bool weighted_ = false;
     int tw_lg_ = 0;

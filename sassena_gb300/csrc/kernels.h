@@ -315,6 +315,14 @@ struct FinalEntry {
     double2* fq2;
 };
 
+// FP32 form: the series [nv][nf] of a shell whose last kTailLags lags are summed directly
+// (A nullptr: they come from the transforms like the others).
+constexpr int kTailLags = 8;
+struct TailEntry {
+    const float2* A;
+    size_t nv;
+};
+
 struct FinalLaunch {
     int dsp, conj_out;
     const FinalEntry* entries;
@@ -324,6 +332,7 @@ struct FinalLaunch {
     const double2* apart;
     const double* a2part;
     const double2* tw;         // [L_max/2] FP64
+    const TailEntry* tails;    // one per entry, or nullptr: none
 };
 cudaError_t launch_finalize(const FinalLaunch& a, cudaStream_t st);
 

@@ -315,13 +315,18 @@ __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const
         const float bmax = hi ? __uint_as_float(hi) : 1.f;
         const int konst = !differs && (!hi || bmax <= 16.f * __uint_as_float(lo));
         // units per weight of 1: no sum of slice_atoms atoms reaches 2^31, no weight 2^22
-        const float scale = fminf(2.0e9f / (kGridPeak * (float)s.slice_atoms), 4.0e6f / kGridPeak);
+        // times a power of two, so that the factors' products with it are exact: a rounding of
+        // the scale is common to all atoms and counts four times in fq2
+        const double most = fmin(2.0e9 / (kGridPeak * s.slice_atoms), 4.0e6 / kGridPeak);
+        int ex;
+        frexp(most / (konst ? bmax : 1.f), &ex);
+        const double scale = ldexp(1.0, ex - 1);
         if (threadIdx.x == 0) {
             *s.konst = konst;
-            s.gw[s.nclass] = konst ? bmax / scale : 1.f / scale;
+            s.gw[s.nclass] = (float)(1.0 / scale);
         }
         for (int c = threadIdx.x; c < s.nclass; c += blockDim.x)
-            s.gw[c] = konst ? fminf(fmaxf((float)s.cf[c] / bmax, -1.f), 1.f) * scale : scale;
+            s.gw[c] = (float)((konst ? (double)fminf(fmaxf((float)s.cf[c], -bmax), bmax) : 1.0) * scale);
     }
 }
 
