@@ -15,10 +15,9 @@
 //
 // GB300 layout.
 //   sphere: the sum over atoms is, for one frame and one l, a product of the matrix
-//     b_j(q) j_l(|q| r_j) [q x atom] with conj(Y_l^m(j)) [atom x m]. A basis kernel writes both
-//     factors for a batch of frames to HBM (every Y_l^m once, not once per q); a tiled
-//     contraction kernel stages atom tiles of both in shared memory and accumulates every
-//     (q, m) output of one (frame, l) in FP64.
+//     b_j(q) j_l(|q| r_j) [q x atom] with conj(Y_l^m(j)) [atom x m]. Basis kernels write both
+//     factors for a batch of frames to HBM (every Y_l^m with m >= 0 once, not once per q, in
+//     fixed point); a contraction kernel sums every (q, m) output of one (frame, l) in integers.
 //   cylinder: one CTA per (q, frame) stages, for a tile of atoms, J_n(q_r r) for every
 //     order n <= 2L, cos(n phi), sin(n phi) and b exp(i s z q_z) in shared memory; threads
 //     then own orders n and accumulate sum_j X_j J_n cos(n phi_j) and ... sin(n phi_j);
@@ -45,7 +44,6 @@ namespace sassgpu {
 namespace {
 
 constexpr int kMpMaxL = 40;  // largest major moment (sphere) / half order (cylinder)
-constexpr int kMpTileAtoms = 32;
 
 // ---------------------------------------------------------------------------------------
 // coordinate representations
@@ -122,26 +120,33 @@ __global__ void mp_convert_kernel(const float4* __restrict__ xyz, int na_pad, in
 // ---------------------------------------------------------------------------------------
 // special functions (FP64)
 // ---------------------------------------------------------------------------------------
-// b * j_l(x) for l = 0..L written to out[l * stride]. Divisions are hoisted (1/x once):
-// GB300's FP64 pipe makes every division or square root a dozen FMAs.
-__device__ void sph_bessel_row(int L, double x, double b, double* out, size_t stride) {
+// Per CTA in shared memory: 2 n + 1 and 1 / (2 n + 1), 1 / n (a conversion or a division holds the
+// FP64 pipe as long as one or a dozen FMAs).
+constexpr int kJlTab = kMpMaxL + 48;
+struct JlTab {
+    double odd[kJlTab], iodd[kJlTab], inv[kJlTab];
+};
+
+// b * j_l(x) for l = 0..L written to out[l * stride].
+__device__ void sph_bessel_row(int L, double x, double b, double* out, size_t stride, const JlTab& t) {
     if (x == 0) {
         out[0] = b;
         for (int l = 1; l <= L; ++l) out[l * stride] = 0;
         return;
     }
     if (x < 0.5) {  // power series
-        double xl = 1;
-        const double x2 = x * x;
+        double xl = b;
+        const double x2 = -0.5 * x * x;
         for (int l = 0; l <= L; ++l) {
-            if (l > 0) xl *= x / (2 * l + 1);
+            if (l > 0) xl *= x * t.iodd[l];
             double term = 1, sum = 1;
             for (int k = 1; k < 40; ++k) {
-                term *= -x2 / (2.0 * k * (2 * l + 2 * k + 1));
+                term *= x2 * t.inv[k] * t.iodd[l + k];
                 sum += term;
-                if (fabs(term) < 1e-18 * fabs(sum)) break;
+                // below 2^-60 of the sum
+                if ((__double2hiint(term) & 0x7fffffff) + (60 << 20) < (__double2hiint(sum) & 0x7fffffff)) break;
             }
-            out[l * stride] = b * xl * sum;
+            out[l * stride] = xl * sum;
         }
         return;
     }
@@ -150,26 +155,32 @@ __device__ void sph_bessel_row(int L, double x, double b, double* out, size_t st
     sincos(x, &sx, &cx);
     const double j0 = sx * ix, j1 = (sx * ix - cx) * ix;
     if (x > L) {  // upward recurrence, stable for every l < x
-        double jm = j0, jc = j1;
-        out[0] = b * j0;
-        if (L >= 1) out[stride] = b * j1;
+        double jm = b * j0, jc = b * j1;
+        out[0] = jm;
+        if (L >= 1) out[stride] = jc;
         for (int l = 1; l < L; ++l) {
-            const double jn = (2 * l + 1) * ix * jc - jm;
-            out[(l + 1) * stride] = b * jn;
+            const double jn = t.odd[l] * ix * jc - jm;
+            out[(l + 1) * stride] = jn;
             jm = jc;
             jc = jn;
         }
         return;
     }
-    // Miller's downward recurrence from order L + 32, normalised by j_0 or j_1
-    const int N = L + 32;
+    // Miller's downward recurrence, normalised by j_0 or j_1. It starts at the order N where
+    // the ratios j_n / j_{n-1} < x / (2 n + 1 - x) (n > L >= x) have multiplied to 2^-32: the
+    // square of that is what the start at (1, 0) leaves of the second solution.
+    int N = L;
+    for (float p = 1.f, xf = (float)x; p > 2.3e-10f && N < L + 32;) {
+        ++N;
+        p *= __fdividef(xf, (float)(2 * N + 1) - xf);
+    }
     double fp = 0, f = 1e-250;
     for (int n = N; n >= 1; --n) {
-        const double fm = (2 * n + 1) * ix * f - fp;
+        const double fm = t.odd[n] * ix * f - fp;
         fp = f;
         f = fm;
         if (n - 1 <= L) out[(n - 1) * stride] = f;
-        if (fabs(f) > 1e200) {
+        if ((__double2hiint(f) & 0x7fffffff) > 0x69800000) {  // 2^665
             for (int l = n - 1; l <= L; ++l) out[l * stride] *= 1e-200;
             fp *= 1e-200;
             f *= 1e-200;
@@ -179,60 +190,111 @@ __device__ void sph_bessel_row(int L, double x, double b, double* out, size_t st
     for (int l = 0; l <= L; ++l) out[l * stride] *= scale;
 }
 
-// Coefficients of the normalised associated Legendre recurrences, per (l, m) with m <= l:
-//   cf[(l (l + 1)) / 2 + m] = (a_lm, b_lm), a = sqrt((4l^2 - 1)/(l^2 - m^2)),
-//   b = sqrt(((l-1)^2 - m^2)/(4 (l-1)^2 - 1)) (l >= m + 2); the seeds per m:
-//   sd[m] = (-sqrt((2m + 1)/(2m)), sqrt(2m + 3)).
-__global__ void ylm_coeff_kernel(int L, double2* cf, double2* sd) {
+// The normalised associated Legendre functions as P_l^m = g_lm y_lm with
+//   y_lm = al_lm x y_{l-1,m} - y_{l-2,m}, y_mm = P_mm, y_{m+1,m} = x P_mm
+// (two FP64 instructions a step instead of three; the factors g_lm, 0.1 to 2, are applied to the
+// sums over atoms): from P_l = a_l (x P_{l-1} - b_l P_{l-2}), a = sqrt((4l^2 - 1)/(l^2 - m^2)),
+// b = sqrt(((l-1)^2 - m^2)/(4 (l-1)^2 - 1)), g_l = a_l b_l g_{l-2} and al_l = a_l g_{l-1} / g_l.
+// Per (l, m) with m <= l, i = (l (l + 1)) / 2 + m: al[i], g[i], and ex[i] with |y_lm| < 2^ex from
+// |P_l^m| <= sqrt((2l + 1) / 4 pi); the seeds per m: sd[m] = -sqrt((2m + 1)/(2m)).
+struct MpLegendre {
+    double *al, *g, *sd;
+    int* ex;
+};
+__host__ __device__ inline size_t legendre_bytes(int L) {
+    return (size_t)((L + 1) * (L + 2) + L + 1) * sizeof(double) + (size_t)(L + 1) * (L + 2) / 2 * sizeof(int);
+}
+__host__ __device__ inline MpLegendre legendre_at(void* p, int L) {
+    MpLegendre t;
     const int n = (L + 1) * (L + 2) / 2;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int l = 0;
-        while ((l + 1) * (l + 2) / 2 <= i) ++l;
-        const int m = i - l * (l + 1) / 2;
-        double a = 0, bb = 0;
-        if (l >= m + 2) {
-            a = sqrt((4.0 * l * l - 1) / ((double)l * l - (double)m * m));
-            bb = sqrt((((double)l - 1) * (l - 1) - (double)m * m) / (4.0 * (l - 1) * (l - 1) - 1));
+    t.al = static_cast<double*>(p);
+    t.g = t.al + n;
+    t.sd = t.g + n;
+    t.ex = reinterpret_cast<int*>(t.sd + L + 1);
+    return t;
+}
+__global__ void ylm_coeff_kernel(int L, MpLegendre t) {
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m <= L; m += gridDim.x * blockDim.x) {
+        t.sd[m] = m > 0 ? -sqrt((2.0 * m + 1) / (2.0 * m)) : 0.0;
+        double g2 = 1, g1 = sqrt(2.0 * m + 3);
+        for (int l = m; l <= L; ++l) {
+            const int i = l * (l + 1) / 2 + m;
+            double g = l == m ? 1.0 : g1, al = 1.0;
+            if (l >= m + 2) {
+                const double a = sqrt((4.0 * l * l - 1) / ((double)l * l - (double)m * m));
+                const double b = sqrt((((double)l - 1) * (l - 1) - (double)m * m) / (4.0 * (l - 1) * (l - 1) - 1));
+                g = a * b * g2;
+                al = a * g1 / g;
+                g2 = g1;
+                g1 = g;
+            }
+            t.al[i] = al;
+            t.g[i] = g;
+            t.ex[i] = (int)ceil(log2(sqrt((2.0 * l + 1) / (4 * 3.14159265358979323846)) / g * 1.0000001));
         }
-        cf[i] = make_double2(a, bb);
-        if (l == m) sd[m] = make_double2(m > 0 ? -sqrt((2.0 * m + 1) / (2.0 * m)) : 0.0, sqrt(2.0 * m + 3));
     }
 }
 
-// conj(Y_l^m(theta, phi)) for the requested moments (idx[l (2L+1) + L + m] -> moment, or -1)
-// written to out[k * stride]; m outer, l inner, so the Legendre recurrence carries two values.
-// e^{i m phi} by rotation (m multiplications of e^{i phi}).
-__device__ void conj_ylm_row(int L, double theta, double phi, const int* __restrict__ idx, const double2* cf,
-                             const double2* sd, double2* out, size_t stride) {
+// Fixed-point numbers of the sphere's contraction: v = (h 2^29 + l) 2^(E - 57), |v| < 2^E, l in
+// [-2^28, 2^28).
+__device__ __forceinline__ long long mp_fixed(double v, int E) {
+    const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+    const unsigned long long m =
+        ((((unsigned long long)((hi & 0xfffff) | (e ? 0x100000 : 0))) << 32) | (unsigned)__double2loint(v)) << 4;
+    const long long t = (long long)(m >> min(max(E + 1022 - e, 0), 63));
+    const long long sg = (long long)(hi >> 31);
+    return (t ^ sg) - sg;
+}
+__device__ __forceinline__ int2 mp_split(long long t) {
+    const int h = (int)((t + (1ll << 28)) >> 29);
+    return make_int2(h, (int)((unsigned)t - ((unsigned)h << 29)));
+}
+// a b + c. Written out: of the forms of a sum of products this one keeps both integer pipes busy
+// (the contraction 1.12 ms; 1.38 as the compiler takes plain C).
+__device__ __forceinline__ long long mp_wide(int a, int b, long long c) {
+    long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+// a b / 2^57
+__device__ __forceinline__ long long mp_mul(int2 a, int2 b) {
+    const long long x = (long long)a.x * b.y + (long long)a.y * b.x + (1ll << 27);
+    return 2 * (long long)a.x * b.x + (x >> 28);
+}
+// conj(Y_l^m(theta, phi)) / g_lm, m >= 0, for the requested pairs (idx[l (L+1) + m] -> pair, or -1)
+// written to out[k * stride] as fixed-point words (re, im); m outer, l inner, so the Legendre
+// recurrence carries two values. e^{i m phi} by rotation (m multiplications of e^{i phi}); its
+// products with the Legendre functions are integers (the FP64 pipe is the bound here).
+__device__ void conj_ylm_row(int L, double theta, double phi, const int* __restrict__ idx,
+                             const MpLegendre& t, int4* out, size_t stride) {
     const double x = cos(theta), s = sqrt((1 - x) * (1 + x));
     double pmm = sqrt(1.0 / (4 * 3.14159265358979323846));
-    const int W = 2 * L + 1;
     double s1, c1;
     sincos(phi, &s1, &c1);
     double cm = 1.0, sm = 0.0;
     for (int m = 0; m <= L; ++m) {
         if (m > 0) {
-            pmm = sd[m].x * s * pmm;
+            pmm = t.sd[m] * s * pmm;
             const double cn = cm * c1 - sm * s1;
             sm = sm * c1 + cm * s1;
             cm = cn;
         }
+        // |cos m phi| may be rounded above 1: 2^E = 1 + 2^-56 here
+        const int2 ci = mp_split(min(max(mp_fixed(cm, 1) << 1, -(1ll << 57)), 1ll << 57));
+        const int2 si = mp_split(min(max(mp_fixed(sm, 1) << 1, -(1ll << 57)), 1ll << 57));
         auto emit = [&](int l, double P) {
-            const int kp = idx[l * W + L + m];
-            if (kp >= 0) out[kp * stride] = make_double2(P * cm, -P * sm);
-            if (m > 0) {
-                const int kn = idx[l * W + L - m];
-                const double v = (m & 1) ? -P : P;  // conj(Y_l^{-m}) = (-1)^m Pbar e^{i m phi}
-                if (kn >= 0) out[kn * stride] = make_double2(v * cm, v * sm);
-            }
+            const int k = idx[l * (L + 1) + m];
+            if (k < 0) return;
+            const int2 pi = mp_split(mp_fixed(P, t.ex[l * (l + 1) / 2 + m]));
+            const int2 re = mp_split(mp_mul(pi, ci)), im = mp_split(-mp_mul(pi, si));
+            out[k * stride] = make_int4(re.x, re.y, im.x, im.y);
         };
         emit(m, pmm);
         if (m < L) {
-            double p2 = pmm, p1 = sd[m].y * x * pmm;
+            double p2 = pmm, p1 = x * pmm;
             emit(m + 1, p1);
             for (int l = m + 2; l <= L; ++l) {
-                const double2 ab = cf[l * (l + 1) / 2 + m];
-                const double p = ab.x * (x * p1 - ab.y * p2);
+                const double p = t.al[l * (l + 1) / 2 + m] * x * p1 - p2;
                 emit(l, p);
                 p2 = p1;
                 p1 = p;
@@ -324,118 +386,231 @@ struct MpSphereBasis {
     const int* cls;     // [na_pad] (-1 padding)
     const double* cf;   // [nq][nclass]
     const double* qlen; // [nq]
-    const int* idx;     // [(L+1)(2L+1)]
-    const double2* ycf; // Legendre coefficients [(L+1)(L+2)/2] and seeds [L+1] (ylm_coeff_kernel)
-    const double2* ysd;
+    const int* idx;     // [L+1][L+1]: pair (l, m >= 0) or -1
+    void* legendre;     // tables of ylm_coeff_kernel
     double* Jb;         // [nfb][nq][L+1][na_pad]  b_j(q) j_l(|q| r_j)
-    double2* Yc;        // [nfb][nmom][na_pad]     conj(Y_l^m(j))
-    int na_pad, nclass, nq, L, nmom, f0, nfb;
+    unsigned* jmax;     // [nfb][nq][L+1] largest |Jb| of the row, its upper half's bits
+    int4* Yc;           // [nfb][npair][na_pad]    conj(Y_l^m(j)) / g_lm, m >= 0, in fixed point
+    int na_pad, nclass, nq, L, npair, f0, nfb;
 };
 
-// conj(Y_l^m) of every (frame, atom) of the batch; the coefficient tables live in shared memory.
+// conj(Y_l^m) / g_lm of every (frame, atom) of the batch; the tables live in shared memory. Also
+// clears jmax for the kernel that follows.
 __global__ void __launch_bounds__(128) mp_ylm_kernel(MpSphereBasis a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    double2* cf = reinterpret_cast<double2*>(smem);
+    const MpLegendre from = legendre_at(a.legendre, a.L), t = legendre_at(smem, a.L);
     const int ncf = (a.L + 1) * (a.L + 2) / 2;
-    double2* sd = cf + ncf;
-    for (int i = threadIdx.x; i < ncf; i += blockDim.x) cf[i] = a.ycf[i];
-    for (int i = threadIdx.x; i <= a.L; i += blockDim.x) sd[i] = a.ysd[i];
+    for (int i = threadIdx.x; i < ncf; i += blockDim.x) {
+        t.al[i] = from.al[i];
+        t.ex[i] = from.ex[i];
+    }
+    for (int i = threadIdx.x; i <= a.L; i += blockDim.x) t.sd[i] = from.sd[i];
     __syncthreads();
-    const size_t n = (size_t)a.nfb * a.na_pad;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t n = (size_t)a.nfb * a.na_pad, n0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.L + 1); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+    for (size_t i = n0; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int fl = (int)(i / a.na_pad), j = (int)(i - (size_t)fl * a.na_pad);
         const float4 c = a.sph[(size_t)(a.f0 + fl) * a.na_pad + j];
-        conj_ylm_row(a.L, (double)c.z, (double)c.y, a.idx, cf, sd, a.Yc + (size_t)fl * a.nmom * a.na_pad + j,
-                     a.na_pad);
+        conj_ylm_row(a.L, (double)c.z, (double)c.y, a.idx, t, a.Yc + (size_t)fl * a.npair * a.na_pad + j, a.na_pad);
     }
 }
 
-// b_j(q) j_l(|q| r_j) of every (frame, q, atom) of the batch.
+// b_j(q) j_l(|q| r_j) of every (frame, q, atom) of the batch, and each row's largest magnitude.
 __global__ void __launch_bounds__(128) mp_jl_kernel(MpSphereBasis a) {
-    const size_t n = (size_t)a.nfb * a.nq * a.na_pad;
+    __shared__ JlTab t;
+    for (int i = threadIdx.x; i < kJlTab; i += blockDim.x) {
+        t.odd[i] = 2 * i + 1;
+        t.iodd[i] = 1.0 / (2 * i + 1);
+        t.inv[i] = i ? 1.0 / i : 0.0;
+    }
+    __syncthreads();
+    const size_t n = (size_t)a.nfb * a.nq * a.na_pad;  // na_pad is a multiple of 32: a warp has one row
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t fq = i / a.na_pad;
         const int j = (int)(i - fq * a.na_pad), fl = (int)(fq / a.nq), q = (int)(fq - (size_t)fl * a.nq);
         const float4 c = a.sph[(size_t)(a.f0 + fl) * a.na_pad + j];
         const int cl = (int)c.w;  // atoms sit in radius order; w carries the class (-1: padding)
         const double b = cl >= 0 ? a.cf[(size_t)q * a.nclass + cl] : 0.0;
-        sph_bessel_row(a.L, a.qlen[q] * (double)c.x, b, a.Jb + (fq * (a.L + 1)) * a.na_pad + j, a.na_pad);
+        double* row = a.Jb + (fq * (a.L + 1)) * a.na_pad + j;
+        sph_bessel_row(a.L, a.qlen[q] * (double)c.x, b, row, a.na_pad, t);
+        __syncwarp();
+        for (int l = 0; l <= a.L; ++l) {
+            const unsigned mx =
+                __reduce_max_sync(0xffffffffu, (unsigned)__double2hiint(row[(size_t)l * a.na_pad]) & 0x7fffffffu);
+            if ((threadIdx.x & 31) == 0) atomicMax(a.jmax + fq * (a.L + 1) + l, mx);
+        }
     }
 }
 
 struct MpSphereContract {
     const double* Jb;
-    const double2* Yc;
-    const int* perm;    // moments grouped by l
-    const int* gl;      // [ngroups] l of the group
-    const int* gstart;  // [ngroups] first entry in perm
-    const int* gcount;  // [ngroups]
-    double2* A;         // [nq][nmom][nf]
-    int na_pad, na, nq, L, nmom, nf, f0;
+    const unsigned* jmax;
+    const int4* Yc;
+    void* legendre;
+    const int4* groups;  // [ngroups] (l, first pair, pairs (at most 8), 0): pairs of one l, consecutive
+    const int* pmom;     // [npair + 1] first entry of each pair in pout
+    const int* pout;     // moments of the pairs, 2 moment + (m < 0)
+    const int* pm;       // [npair] m of the pair
+    double2* A;          // [nq][nmom][nf]
+    int na_pad, na, nq, L, nmom, npair, nf, f0;
 };
 
-constexpr int kContractThreads = 256, kContractOutputs = 4;
+constexpr int kSumWarps = 8, kSumTile = 256;  // atoms of a tile
+static_assert(kSumTile == kSumWarps * 32, "a thread converts one atom of a tile");
 
-__global__ void __launch_bounds__(kContractThreads) mp_sphere_contract_kernel(MpSphereContract a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int g = blockIdx.x, fl = blockIdx.y;
-    const int l = a.gl[g], k0 = a.gstart[g], cnt = a.gcount[g];
-    const int nout = a.nq * cnt;
-    const int obase = blockIdx.z * kContractThreads * kContractOutputs;
-    if (obase >= nout) return;
-    double* Js = reinterpret_cast<double*>(smem);                    // [nq][T]
-    double2* Ys = reinterpret_cast<double2*>(Js + (size_t)a.nq * kMpTileAtoms);  // [cnt][T]
-    double2 acc[kContractOutputs];
-#pragma unroll
-    for (int r = 0; r < kContractOutputs; ++r) acc[r] = make_double2(0.0, 0.0);
-    const double* jrow = a.Jb + (size_t)fl * a.nq * (a.L + 1) * a.na_pad;
-    const double2* yrow = a.Yc + (size_t)fl * a.nmom * a.na_pad;
-    const int jend = (a.na + kMpTileAtoms - 1) / kMpTileAtoms * kMpTileAtoms;  // <= na_pad
-    for (int j0 = 0; j0 < jend; j0 += kMpTileAtoms) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < a.nq * kMpTileAtoms; t += kContractThreads) {
-            const int q = t / kMpTileAtoms, jj = t - q * kMpTileAtoms;
-            Js[t] = jrow[((size_t)q * (a.L + 1) + l) * a.na_pad + j0 + jj];
+__device__ __forceinline__ void mp_cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// sum_j b_j(q) j_l(|q| r_j) conj(Y_l^m(j)) of one frame, up to 8 pairs (l, m) and QB q-vectors, in
+// integers: the FP64 pipe takes 19 clocks of an SM per warp FMA, a product of 58-bit numbers as
+// three 32 x 32 -> 64-bit multiplications about 1.7 each. J gets the exponent of its row's largest
+// value, Y that of its bound, so that both keep 57 bits below it; the low halves' product, below
+// 2^-58 of the largest, is left out. Only m >= 0 is summed: b_j j_l is real, so the sum for -m is
+// (-1)^m times the conjugate. A lane is an atom, a warp a pair (or, of fewer pairs than warps, a
+// pair and a part of the atoms): Y is read once, straight from memory; the tile's J words are
+// shared. QB x 2 sums of two words each stay in registers; before they could overflow (62-bit
+// products, 56 atoms a lane) they are added over the lanes by 26-bit pieces and go to FP64.
+// 5,000 atoms, 64 frames, 10 q, 441 moments: 6.7 ms before, 1.1 here.
+template <int QB>
+__global__ void __launch_bounds__(kSumWarps * 32, 2) mp_sphere_sum_kernel(MpSphereContract a) {
+    __shared__ int2 Js[QB][kSumTile];
+    __shared__ __align__(16) double raw[QB][kSumTile];  // the next tile
+    __shared__ int rowe[QB];
+    __shared__ double part[kSumWarps][2 * QB];
+    const int4 grp = a.groups[blockIdx.x];
+    const int l = grp.x, cnt = grp.z, fl = blockIdx.y, q0 = blockIdx.z * QB, nqb = min(QB, a.nq - q0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double* jrow = a.Jb + (((size_t)fl * a.nq + q0) * (a.L + 1) + l) * a.na_pad;
+    const size_t qstep = (size_t)(a.L + 1) * a.na_pad;
+    const int jend = (a.na + 31) & ~31;  // <= na_pad; b_j = 0 past na
+    if (threadIdx.x < nqb) {
+        const unsigned mx = a.jmax[((size_t)fl * a.nq + q0 + threadIdx.x) * (a.L + 1) + l];
+        rowe[threadIdx.x] = mx >= 0x7ff00000u ? 4096 : max((int)(mx >> 20), 1) - 1022;  // 4096: not finite
+    }
+    auto fetch = [&](int j0) {  // two atoms a thread and row
+        for (int i = threadIdx.x; i < nqb * (kSumTile / 2); i += kSumWarps * 32) {
+            const int q = i / (kSumTile / 2), j = i % (kSumTile / 2) * 2;
+            if (j0 + j < jend) mp_cp_async16(&raw[q][j], jrow + q * qstep + j0 + j);
         }
-        for (int t = threadIdx.x; t < cnt * kMpTileAtoms; t += kContractThreads) {
-            const int kk = t / kMpTileAtoms, jj = t - kk * kMpTileAtoms;
-            Ys[t] = yrow[(size_t)a.perm[k0 + kk] * a.na_pad + j0 + jj];
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    // atoms in parts: 8 / cnt warps share a pair
+    const int aw = cnt > 4 ? 1 : cnt > 2 ? 2 : cnt > 1 ? 4 : 8;
+    const int k = warp % cnt, g = warp / cnt;
+    const bool live = g < aw;
+    const int4* y = a.Yc + ((size_t)fl * a.npair + grp.y + k) * a.na_pad + g * 32 + lane;
+    long long rh[QB], rx[QB], ih[QB], ix[QB];
+#pragma unroll
+    for (int q = 0; q < QB; ++q) rh[q] = rx[q] = ih[q] = ix[q] = 0;
+    double total = 0.0;  // of the output this lane holds: 2 q (+ 1: imaginary part)
+    int n = 0;
+    auto flush = [&]() {
+        int p0 = 0, p1 = 0, p2 = 0;
+        auto take = [&](long long h, int o) {
+            const int s0 = __reduce_add_sync(0xffffffffu, (int)h & 0x3ffffff);
+            const int s1 = __reduce_add_sync(0xffffffffu, (int)(h >> 26) & 0x3ffffff);
+            const int s2 = __reduce_add_sync(0xffffffffu, (int)(h >> 52));
+            if (lane == o) {
+                p0 = s0;
+                p1 = s1;
+                p2 = s2;
+            }
+        };
+#pragma unroll
+        for (int q = 0; q < QB; ++q) {
+            take(rh[q] + ((rx[q] + (1 << 28)) >> 29), 2 * q);
+            take(ih[q] + ((ix[q] + (1 << 28)) >> 29), 2 * q + 1);
+            rh[q] = rx[q] = ih[q] = ix[q] = 0;
+        }
+        total += fma((double)p2, 4503599627370496.0, fma((double)p1, 67108864.0, (double)p0));
+        n = 0;
+    };
+    const int4 zero = make_int4(0, 0, 0, 0);
+    int4 yv = live && g * 32 < jend ? *y : zero;
+    for (int j0 = 0; j0 < jend; j0 += kSumTile) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // raw is here; the exponents; the previous tile has been read
+#pragma unroll
+        for (int q = 0; q < QB; ++q) {
+            int2 w = make_int2(0, 0);
+            if (q < nqb && j0 + (int)threadIdx.x < jend) w = mp_split(mp_fixed(raw[q][threadIdx.x], rowe[q]));
+            Js[q][threadIdx.x] = w;
         }
         __syncthreads();
+        if (j0 + kSumTile < jend) fetch(j0 + kSumTile);
+        if (!live) continue;
+        for (int c = g * 32; c < kSumTile && j0 + c < jend; c += aw * 32) {
+            const int4 v = yv;
+            y += aw * 32;
+            yv = j0 + c + aw * 32 < jend ? *y : zero;
 #pragma unroll
-        for (int r = 0; r < kContractOutputs; ++r) {
-            const int o = obase + threadIdx.x + r * kContractThreads;
-            if (o < nout) {
-                const int q = o / cnt, kk = o - q * cnt;
-                const double* jq = Js + q * kMpTileAtoms;
-                const double2* yk = Ys + kk * kMpTileAtoms;
-                double2 s = acc[r];
-                for (int jj = 0; jj < kMpTileAtoms; ++jj) {
-                    s.x = fma(jq[jj], yk[jj].x, s.x);
-                    s.y = fma(jq[jj], yk[jj].y, s.y);
-                }
-                acc[r] = s;
+            for (int q = 0; q < QB; ++q) {
+                const int2 w = Js[q][c + lane];
+                rh[q] += mp_wide(w.x, v.x, 0);
+                rx[q] += mp_wide(w.x, v.y, mp_wide(w.y, v.x, 0));
+                ih[q] += mp_wide(w.x, v.z, 0);
+                ix[q] += mp_wide(w.x, v.w, mp_wide(w.y, v.z, 0));
+            }
+            ++n;
+        }
+        if (n > 48) {
+            flush();
+        } else if (n & 8 || n > 16) {  // the cross products' sums (2^57 each) into the high ones
+#pragma unroll
+            for (int q = 0; q < QB; ++q) {
+                rh[q] += rx[q] >> 29;
+                rx[q] &= (1 << 29) - 1;
+                ih[q] += ix[q] >> 29;
+                ix[q] &= (1 << 29) - 1;
             }
         }
     }
+    if (live) {
+        flush();
+        if (lane < 2 * QB) part[warp][lane] = total;
+    }
+    __syncthreads();
     // times 4 pi i^l
     const double f4 = 4 * 3.14159265358979323846;
-#pragma unroll
-    for (int r = 0; r < kContractOutputs; ++r) {
-        const int o = obase + threadIdx.x + r * kContractThreads;
-        if (o < nout) {
-            const int q = o / cnt, kk = o - q * cnt, mom = a.perm[k0 + kk];
-            double2 v = acc[r], w;
+    for (int o = threadIdx.x; o < cnt * nqb; o += kSumWarps * 32) {
+        const int q = o / cnt, kk = o - q * cnt, pair = grp.y + kk;
+        double2 v = make_double2(0.0, 0.0);
+        for (int w = kk; w < aw * cnt; w += cnt) {
+            v.x += part[w][2 * q];
+            v.y += part[w][2 * q + 1];
+        }
+        const double f = rowe[q] == 4096 ? nan("") : f4;
+        const MpLegendre lt = legendre_at(a.legendre, a.L);
+        const int i0 = l * (l + 1) / 2 + a.pm[pair], e = rowe[q] + lt.ex[i0] - 56;
+        v = make_double2(f * lt.g[i0] * scalbn(v.x, e), f * lt.g[i0] * scalbn(v.y, e));
+        for (int i = a.pmom[pair]; i < a.pmom[pair + 1]; ++i) {
+            const int out = a.pout[i];
+            double2 u = v;
+            if (out & 1) u = (a.pm[pair] & 1) ? make_double2(-v.x, v.y) : make_double2(v.x, -v.y);
+            double2 w;
             switch (l & 3) {
-                case 0: w = make_double2(v.x, v.y); break;
-                case 1: w = make_double2(-v.y, v.x); break;
-                case 2: w = make_double2(-v.x, -v.y); break;
-                default: w = make_double2(v.y, -v.x); break;
+                case 0: w = make_double2(u.x, u.y); break;
+                case 1: w = make_double2(-u.y, u.x); break;
+                case 2: w = make_double2(-u.x, -u.y); break;
+                default: w = make_double2(u.y, -u.x); break;
             }
-            a.A[((size_t)q * a.nmom + mom) * a.nf + a.f0 + fl] = make_double2(f4 * w.x, f4 * w.y);
+            a.A[((size_t)(q0 + q) * a.nmom + (out >> 1)) * a.nf + a.f0 + fl] = w;
         }
     }
 }
+
+template <int QB>
+cudaError_t launch_sphere_sum(int qb, const MpSphereContract& a, dim3 grid, cudaStream_t st) {
+    if (qb < QB) {
+        if constexpr (QB > 1) return launch_sphere_sum<QB - 1>(qb, a, grid, st);
+    }
+    mp_sphere_sum_kernel<QB><<<grid, kSumWarps * 32, 0, st>>>(a);
+    return cudaGetLastError();
+}
+constexpr int kSumQ = 10;  // q-vectors of a CTA, at most: their sums fill the registers
 
 // ---------------------------------------------------------------------------------------
 // cylinder
@@ -666,22 +841,33 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             to_cylinder(px, py, pz, qin[3 * i], qin[3 * i + 1], qin[3 * i + 2]);
         }
     }
-    // sphere: lookup (l, m) -> moment and moments grouped by l
-    const int W = 2 * L + 1;
-    std::vector<int> idx((size_t)(L + 1) * W, -1), perm, gl, gstart, gcount;
+    // sphere: the pairs (l, |m|) of the moments, in order of l, each with its moments (2 moment +
+    // (m < 0)), and groups of at most 8 pairs of one l
+    std::vector<int> idx((size_t)(L + 1) * (L + 1), -1), pmom, pout, pm;
+    std::vector<int4> groups;
     if (!cyl) {
-        for (size_t k = 0; k < nmom; ++k) idx[moments[2 * k] * W + L + moments[2 * k + 1]] = (int)k;
-        for (int l = 0; l <= L; ++l) {
-            const int start = (int)perm.size();
-            for (size_t k = 0; k < nmom; ++k)
-                if (moments[2 * k] == l) perm.push_back((int)k);
-            if ((int)perm.size() > start) {
-                gl.push_back(l);
-                gstart.push_back(start);
-                gcount.push_back((int)perm.size() - start);
-            }
+        std::vector<std::vector<int>> at((size_t)(L + 1) * (L + 1));
+        for (size_t k = 0; k < nmom; ++k) {
+            const int l = moments[2 * k], m = moments[2 * k + 1];
+            at[(size_t)l * (L + 1) + std::abs(m)].push_back((int)(2 * k) + (m < 0));
         }
+        for (int l = 0; l <= L; ++l) {
+            const int first = (int)pm.size();
+            for (int m = 0; m <= l; ++m) {
+                const std::vector<int>& v = at[(size_t)l * (L + 1) + m];
+                if (v.empty()) continue;
+                idx[l * (L + 1) + m] = (int)pm.size();
+                pm.push_back(m);
+                pmom.push_back((int)pout.size());
+                pout.insert(pout.end(), v.begin(), v.end());
+            }
+            for (int p0 = first; p0 < (int)pm.size(); p0 += 8)
+                groups.push_back(make_int4(l, p0, std::min(8, (int)pm.size() - p0), 0));
+        }
+        pmom.push_back((int)pout.size());
+        std::reverse(groups.begin(), groups.end());  // whole groups first
     }
+    const size_t npair = pm.size();
     // one packed upload of every small input (16-byte aligned pieces)
     std::vector<unsigned char> blob;
     auto put = [&](const void* h, size_t bytes) {
@@ -694,10 +880,10 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
     const size_t o_cf = put(class_factors, nq * nclass * sizeof(double));
     const size_t o_mom = put(moments, nmom * 2 * sizeof(int32_t));
     const size_t o_idx = put(idx.data(), idx.size() * sizeof(int));
-    const size_t o_perm = put(perm.data(), perm.size() * sizeof(int));
-    const size_t o_gl = put(gl.data(), gl.size() * sizeof(int));
-    const size_t o_gs = put(gstart.data(), gstart.size() * sizeof(int));
-    const size_t o_gc = put(gcount.data(), gcount.size() * sizeof(int));
+    const size_t o_groups = put(groups.data(), groups.size() * sizeof(int4));
+    const size_t o_pmom = put(pmom.data(), pmom.size() * sizeof(int));
+    const size_t o_pout = put(pout.data(), pout.size() * sizeof(int));
+    const size_t o_pm = put(pm.data(), pm.size() * sizeof(int));
     MCK(p->mp_in.ensure(blob.size()));
     MCK(p->mp_amp.ensure(nq * nmom * nf * sizeof(double2)));
     MCK(p->mp_out.ensure(nq * (nf + 2) * sizeof(double2)));
@@ -754,23 +940,18 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
         size_t free_b = 0, total_b = 0;
         MCK(cudaMemGetInfo(&free_b, &total_b));
         const size_t budget = std::max<size_t>((size_t)1 << 28, std::min<size_t>((size_t)16 << 30, free_b / 4));
-        const size_t per_frame = na_pad * (nq * (L + 1) * sizeof(double) + nmom * sizeof(double2));
+        const size_t per_frame = na_pad * (nq * (L + 1) * sizeof(double) + npair * sizeof(int4));
         const size_t nfb = std::max<size_t>(1, std::min<size_t>({nf, budget / per_frame, (size_t)65535}));  // grid y
-        const int ncf = (L + 1) * (L + 2) / 2;
-        MCK(p->mp_ycf.ensure((size_t)(ncf + L + 1) * sizeof(double2)));
-        ylm_coeff_kernel<<<(ncf + 127) / 128, 128, 0, st>>>(L, p->mp_ycf.as<double2>(), p->mp_ycf.as<double2>() + ncf);
+        const size_t ysm = legendre_bytes(L);
+        const size_t jmax_bytes = nfb * nq * (L + 1) * sizeof(unsigned);
+        MCK(p->mp_ycf.ensure((ysm + 15) / 16 * 16 + jmax_bytes));
+        ylm_coeff_kernel<<<1, 64, 0, st>>>(L, legendre_at(p->mp_ycf.p, L));
         MCK(cudaGetLastError());
         ++launches;
-        const size_t ysm = (size_t)(ncf + L + 1) * sizeof(double2);
         MCK(p->mp_Jb.ensure(nfb * nq * (L + 1) * na_pad * sizeof(double)));
-        MCK(p->mp_Yc.ensure(nfb * nmom * na_pad * sizeof(double2)));
-        int maxcnt = 0;
-        for (int c : gcount) maxcnt = std::max(maxcnt, c);
-        const size_t csm = nq * kMpTileAtoms * sizeof(double) + (size_t)maxcnt * kMpTileAtoms * sizeof(double2);
-        if (csm > 48 * 1024)
-            MCK(cudaFuncSetAttribute(mp_sphere_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
-        const int zchunks = (int)((nq * maxcnt + kContractThreads * kContractOutputs - 1) /
-                                  (kContractThreads * kContractOutputs));
+        MCK(p->mp_Yc.ensure(nfb * npair * na_pad * sizeof(int4)));
+        // q-vectors of a CTA: as even as they go
+        const size_t nqc = (nq + kSumQ - 1) / kSumQ, qb = (nq + nqc - 1) / nqc;
         for (size_t f0 = 0; f0 < nf; f0 += nfb) {
             const int nb = (int)std::min(nfb, nf - f0);
             MpSphereBasis ba{};
@@ -779,41 +960,42 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ba.cf = d_cf;
             ba.qlen = reinterpret_cast<const double*>(dptr(o_qin));
             ba.idx = reinterpret_cast<const int*>(dptr(o_idx));
-            ba.ycf = p->mp_ycf.as<double2>();
-            ba.ysd = p->mp_ycf.as<double2>() + ncf;
+            ba.legendre = p->mp_ycf.p;
+            ba.jmax = reinterpret_cast<unsigned*>(p->mp_ycf.as<unsigned char>() + (ysm + 15) / 16 * 16);
             ba.Jb = p->mp_Jb.as<double>();
-            ba.Yc = p->mp_Yc.as<double2>();
+            ba.Yc = p->mp_Yc.as<int4>();
             ba.na_pad = (int)na_pad;
             ba.nclass = (int)nclass;
             ba.nq = (int)nq;
             ba.L = L;
-            ba.nmom = (int)nmom;
+            ba.npair = (int)npair;
             ba.f0 = (int)f0;
             ba.nfb = nb;
             const size_t ny = (size_t)nb * na_pad, nj = ny * nq;
             mp_ylm_kernel<<<grid_blocks(ny, 128, 64), 128, ysm, st>>>(ba);
             MCK(cudaGetLastError());
-            mp_jl_kernel<<<grid_blocks(nj, 128, 64), 128, 0, st>>>(ba);
+            mp_jl_kernel<<<grid_blocks(nj, 128, 16), 128, 0, st>>>(ba);
             MCK(cudaGetLastError());
             ++launches;
             MpSphereContract ca{};
             ca.Jb = p->mp_Jb.as<double>();
-            ca.Yc = p->mp_Yc.as<double2>();
-            ca.perm = reinterpret_cast<const int*>(dptr(o_perm));
-            ca.gl = reinterpret_cast<const int*>(dptr(o_gl));
-            ca.gstart = reinterpret_cast<const int*>(dptr(o_gs));
-            ca.gcount = reinterpret_cast<const int*>(dptr(o_gc));
+            ca.jmax = ba.jmax;
+            ca.Yc = p->mp_Yc.as<int4>();
+            ca.legendre = p->mp_ycf.p;
+            ca.groups = reinterpret_cast<const int4*>(dptr(o_groups));
+            ca.pmom = reinterpret_cast<const int*>(dptr(o_pmom));
+            ca.pout = reinterpret_cast<const int*>(dptr(o_pout));
+            ca.pm = reinterpret_cast<const int*>(dptr(o_pm));
             ca.A = p->mp_amp.as<double2>();
             ca.na_pad = (int)na_pad;
             ca.na = (int)s.na;
             ca.nq = (int)nq;
             ca.L = L;
             ca.nmom = (int)nmom;
+            ca.npair = (int)npair;
             ca.nf = (int)nf;
             ca.f0 = (int)f0;
-            dim3 grid((unsigned)gl.size(), (unsigned)nb, (unsigned)zchunks);
-            mp_sphere_contract_kernel<<<grid, kContractThreads, csm, st>>>(ca);
-            MCK(cudaGetLastError());
+            MCK(launch_sphere_sum<kSumQ>((int)qb, ca, dim3((unsigned)groups.size(), (unsigned)nb, (unsigned)nqc), st));
             launches += 2;
         }
     } else {
