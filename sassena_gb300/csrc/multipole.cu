@@ -18,10 +18,10 @@
 //     b_j(q) j_l(|q| r_j) [q x atom] with conj(Y_l^m(j)) [atom x m]. Basis kernels write both
 //     factors for a batch of frames to HBM (every Y_l^m with m >= 0 once, not once per q, in
 //     fixed point); a contraction kernel sums every (q, m) output of one (frame, l) in integers.
-//   cylinder: one CTA per (q, frame) stages, for a tile of atoms, J_n(q_r r) for every
-//     order n <= 2L, cos(n phi), sin(n phi) and b exp(i s z q_z) in shared memory; threads
-//     then own orders n and accumulate sum_j X_j J_n cos(n phi_j) and ... sin(n phi_j);
-//     each moment is formed from them with cos(n phi_q), sin(n phi_q).
+//   cylinder: basis kernels write J_n(q_r r) for every order n <= 2L, X = b exp(i s z q_z), and
+//     cos(n phi), sin(n phi) of a batch of frames; a contraction kernel sums X_j J_n cos(n phi_j)
+//     and ... sin(n phi_j) over atoms in integers; each moment is formed from them with
+//     cos(n phi_q), sin(n phi_q).
 // The special functions are this project's own FP64 implementations (Boost, which the
 // reference calls, is not used): spherical Bessel functions by power series, upward
 // recurrence where stable or Miller's downward recurrence; normalised associated Legendre
@@ -261,6 +261,11 @@ __device__ __forceinline__ long long mp_mul(int2 a, int2 b) {
     const long long x = (long long)a.x * b.y + (long long)a.y * b.x + (1ll << 27);
     return 2 * (long long)a.x * b.x + (x >> 28);
 }
+// |v| <= 1 (or rounded above it) in units of 2^-57
+__device__ __forceinline__ int2 mp_unit(double v) {
+    return mp_split(min(max(mp_fixed(v, 1) << 1, -(1ll << 57)), 1ll << 57));
+}
+
 // conj(Y_l^m(theta, phi)) / g_lm, m >= 0, for the requested pairs (idx[l (L+1) + m] -> pair, or -1)
 // written to out[k * stride] as fixed-point words (re, im); m outer, l inner, so the Legendre
 // recurrence carries two values. e^{i m phi} by rotation (m multiplications of e^{i phi}); its
@@ -279,9 +284,7 @@ __device__ void conj_ylm_row(int L, double theta, double phi, const int* __restr
             sm = sm * c1 + cm * s1;
             cm = cn;
         }
-        // |cos m phi| may be rounded above 1: 2^E = 1 + 2^-56 here
-        const int2 ci = mp_split(min(max(mp_fixed(cm, 1) << 1, -(1ll << 57)), 1ll << 57));
-        const int2 si = mp_split(min(max(mp_fixed(sm, 1) << 1, -(1ll << 57)), 1ll << 57));
+        const int2 ci = mp_unit(cm), si = mp_unit(sm);
         auto emit = [&](int l, double P) {
             const int k = idx[l * (L + 1) + m];
             if (k < 0) return;
@@ -303,78 +306,103 @@ __device__ void conj_ylm_row(int L, double theta, double phi, const int* __restr
     }
 }
 
-// J_0(x), J_1(x) for x >= 25 by Hankel's asymptotic expansion (cos, sin of x - pi/4 and
-// x - 3 pi/4 formed from cos x, sin x).
+// Coefficients of Hankel's expansions: A_k(nu) = prod_{i <= k} (4 nu^2 - (2 i - 1)^2) / (8 i); P has
+// (-1)^j A_2j, Q (-1)^j A_2j+1, in powers of 1/x^2. From x = 25 on, twenty terms reach 3e-17.
+struct HankelCoef {
+    double p[2][10], q[2][10];
+    constexpr HankelCoef() : p{}, q{} {
+        for (int nu = 0; nu < 2; ++nu) {
+            double a = 1;
+            for (int k = 0; k < 20; ++k) {
+                if (k > 0) a *= (4.0 * nu * nu - (2.0 * k - 1) * (2.0 * k - 1)) / (8.0 * k);
+                const double v = (k / 2) % 2 ? -a : a;
+                if (k % 2) q[nu][k / 2] = v;
+                else p[nu][k / 2] = v;
+            }
+        }
+    }
+};
+__constant__ HankelCoef kHankel;
+
+// J_0(x), J_1(x) for x >= 25 (cos, sin of x - pi/4 and x - 3 pi/4 formed from cos x, sin x).
 __device__ void bessel01_asymptotic(double x, double& j0, double& j1) {
-    double P0 = 1, Q0 = 0, P1 = 1, Q1 = 0;
+    const double ix = 1.0 / x, i2 = ix * ix;
+    double P[2], Q[2];
+#pragma unroll
     for (int nu = 0; nu < 2; ++nu) {
-        const double mu = 4.0 * nu * nu;
-        double a = 1, P = 1, Q = 0;
-        const double i8x = 1.0 / (8.0 * x);
-        for (int k = 1; k < 60; ++k) {
-            const double next = a * (mu - (2.0 * k - 1) * (2.0 * k - 1)) * i8x / k;
-            if (fabs(next) > fabs(a) && k > 2) break;
-            a = next;
-            if (k & 1) Q += (((k - 1) / 2) & 1 ? -a : a);
-            else P += ((k / 2) & 1 ? -a : a);
-            if (fabs(a) < 1e-18) break;
+        P[nu] = kHankel.p[nu][9];
+        Q[nu] = kHankel.q[nu][9];
+#pragma unroll
+        for (int k = 8; k >= 0; --k) {
+            P[nu] = fma(P[nu], i2, kHankel.p[nu][k]);
+            Q[nu] = fma(Q[nu], i2, kHankel.q[nu][k]);
         }
-        if (nu == 0) {
-            P0 = P;
-            Q0 = Q;
-        } else {
-            P1 = P;
-            Q1 = Q;
-        }
+        Q[nu] *= ix;
     }
     double s, c;
     sincos(x, &s, &c);
-    const double h = 0.70710678118654752440, amp = sqrt(2.0 / (3.14159265358979323846 * x));
-    j0 = amp * (P0 * h * (c + s) - Q0 * h * (s - c));
-    j1 = amp * (P1 * h * (s - c) + Q1 * h * (s + c));
+    const double amp = sqrt(ix * (1.0 / 3.14159265358979323846));  // sqrt(2 / (pi x)) sqrt(1/2)
+    j0 = amp * (P[0] * (c + s) - Q[0] * (s - c));
+    j1 = amp * (P[1] * (s - c) + Q[1] * (s + c));
 }
 
-// J_n(x), n = 0..N, written to out[n * stride].
-__device__ void cyl_bessel_row(int N, double x, double* out, int stride) {
+// J_n(x), n = 0..N, written to out[n * stride]; num[n] = n as FP64.
+constexpr int kJnExtra = 72, kJnTab = 2 * kMpMaxL + kJnExtra + 2;
+__device__ void cyl_bessel_row(int N, double x, double* out, size_t stride, const double* num) {
     if (x == 0) {
         out[0] = 1;
         for (int n = 1; n <= N; ++n) out[n * stride] = 0;
         return;
     }
+    if (!(x > 0)) {  // not a number
+        for (int n = 0; n <= N; ++n) out[n * stride] = x;
+        return;
+    }
+    const double ix2 = 2.0 / x;
     if (x >= 25 && x > N) {
-        double j0, j1;
-        bessel01_asymptotic(x, j0, j1);
-        out[0] = j0;
-        if (N >= 1) out[stride] = j1;
-        double jm = j0, jc = j1;
-        const double ix2 = 2.0 / x;
+        double jm, jc;
+        bessel01_asymptotic(x, jm, jc);
+        out[0] = jm;
+        if (N >= 1) out[stride] = jc;
         for (int n = 1; n < N; ++n) {
-            const double jn = n * ix2 * jc - jm;
+            const double jn = num[n] * ix2 * jc - jm;
             out[(n + 1) * stride] = jn;
             jm = jc;
             jc = jn;
         }
         return;
     }
-    const double top = fmax((double)N, x);
-    int M = (int)(top + 20 + 2 * sqrt(top + 10));
+    // Miller's downward recurrence from M, normalised by J_0 + 2 sum J_2k = 1. Ratios J_n / J_{n-1}
+    // are below x / (n + sqrt(n^2 - x^2)) for n > x; M is where those from x on have multiplied to
+    // 2^-58 (the sum's rest) and those above N to 2^-32 (its square: the second solution).
+    int M = (int)x;
+    const int cap = max(N, M) + kJnExtra;
+    for (float pa = 1.f, pb = 1.f, xf = (float)x; M < cap && (M < N || pa > 3e-18f || pb > 2.3e-10f);) {
+        ++M;
+        const float nf = (float)M, r = fminf(__fdividef(xf, nf + sqrtf(fmaxf(nf * nf - xf * xf, 0.f))), 1.f);
+        pa *= r;
+        if (M > N) pb *= r;
+    }
     M += M & 1;
-    const double ix2 = 2.0 / x;
     double fp = 0, f = 1e-250, norm = 0;
-    for (int n = M; n >= 1; --n) {
-        const double fm = n * ix2 * f - fp;
+    auto step = [&](int n) {  // f_n to f_{n-1}
+        const double fm = num[n] * ix2 * f - fp;
         fp = f;
         f = fm;
         if (n - 1 <= N) out[(n - 1) * stride] = f;
-        if (((n - 1) & 1) == 0) norm += (n - 1 == 0 ? 1.0 : 2.0) * f;
-        if (fabs(f) > 1e200) {
+        if ((__double2hiint(f) & 0x7fffffff) > 0x69800000) {  // 2^665
             for (int k = n - 1; k <= N; ++k) out[k * stride] *= 1e-200;
             fp *= 1e-200;
             f *= 1e-200;
             norm *= 1e-200;
         }
+    };
+    for (int n = M; n > 0; n -= 2) {
+        step(n);
+        step(n - 1);
+        norm += f;
     }
-    const double inorm = 1.0 / norm;
+    const double inorm = 1.0 / (2 * norm - f);
     for (int n = 0; n <= N; ++n) out[n * stride] *= inorm;
 }
 
@@ -617,130 +645,237 @@ constexpr int kSumQ = 10;  // q-vectors of a CTA, at most: their sums fill the r
 // ---------------------------------------------------------------------------------------
 struct MpCylinder {
     const float4* cyl;   // [nf][na_pad] (r, phi, z, class), atoms in order of frame-0 radius
-    const int* cls;
     const double* cf;    // [nq][nclass]
     const double* qcyl;  // [nq][3] (q_r, phi_q, q_z)
+    double* Jb;          // [nfb][nq][N+3][na_pad]: J_n(q_r r), then real and imaginary part of X
+    unsigned* jmax;      // [nfb][nq][N+3] largest magnitude of the row, its upper half's bits
+    int4* Tc;            // [nfb][nn][na_pad] cos(n phi), sin(n phi) in fixed point
+    const int* ns;       // [nn] the orders that the moments need
+    const int* nmom0;    // [nn + 1] first entry of each order in nout
+    const int* nout;     // [nmom] the moments of the orders
     const int* mom;      // [nmom][2]
     double2* A;          // [nq][nmom][nf]
-    int na_pad, na, nclass, nq, N, nmom, nf;
-    int f0;              // first frame of the launch (blockIdx.y counts from it)
+    int na_pad, na, nclass, nq, N, nn, nmom, nf, f0, nfb;
 };
 
-// One CTA per (frame, block of kCylQB q-vectors), kCylThreads threads, tiles of kCylTA atoms.
-// Per tile, threads [0, QB TA) evaluate one (q, atom) pair each: the Bessel row J_n(q_r r) and
-// X = b e^{i s z q_z}; threads [QB TA, QB TA + TA) evaluate cos(n phi), sin(n phi) of one atom
-// (shared by the block's q-vectors). Then every thread owns (q, order, cos|sin) sums.
-constexpr int kCylQB = 3, kCylTA = 32, kCylThreads = 128;
-static_assert(kCylQB * kCylTA + kCylTA <= kCylThreads, "tile roles exceed the CTA");
-
-__global__ void __launch_bounds__(kCylThreads) mp_cylinder_kernel(MpCylinder a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int f = a.f0 + blockIdx.y, q0 = blockIdx.x * kCylQB, nqb = min(kCylQB, a.nq - q0);
-    const int N = a.N, W = N + 1, ntask = nqb * 2 * W;
-    double* Jn = reinterpret_cast<double*>(smem);                         // [QB][W][TA]
-    double* cn = Jn + (size_t)kCylQB * W * kCylTA;                          // [W][TA]
-    double* sn = cn + (size_t)W * kCylTA;                                   // [W][TA]
-    double2* X = reinterpret_cast<double2*>(sn + (size_t)W * kCylTA);      // [QB][TA]
-    constexpr int NPT = (kCylQB * 2 * (2 * kMpMaxL + 1) + kCylThreads - 1) / kCylThreads;
-    double2 acc[NPT];
-#pragma unroll
-    for (int k = 0; k < NPT; ++k) acc[k] = make_double2(0.0, 0.0);
-    const float4* row = a.cyl + (size_t)f * a.na_pad;
-    const int tid = threadIdx.x;
-    for (int j0 = 0; j0 < a.na; j0 += kCylTA) {
-        __syncthreads();
-        if (tid < kCylQB * kCylTA) {
-            const int qq = tid / kCylTA, jj = tid - qq * kCylTA, j = j0 + jj;
-            double* jrow = Jn + (size_t)qq * W * kCylTA + jj;
-            if (qq < nqb && j < a.na) {
-                const int q = q0 + qq;
-                const double qr = a.qcyl[3 * q], qz = a.qcyl[3 * q + 2];
-                const float4 c = row[j];
-                const double r = c.x, z = c.z;
-                const int cl = (int)c.w;  // atoms sit in radius order; w carries the class
-                const double b = cl >= 0 ? a.cf[(size_t)q * a.nclass + cl] : 0.0;
-                double sgn = 1.0;  // parallel_sign, multipole_scatter_device.cpp:944-948
-                if (z != 0 && qz != 0) sgn = (z * qz) / (fabs(z) * fabs(qz));
-                double es, ec;
-                sincos(sgn * z * qz, &es, &ec);
-                X[qq * kCylTA + jj] = make_double2(b * ec, b * es);
-                cyl_bessel_row(N, r * qr, jrow, kCylTA);
-            } else {
-                X[qq * kCylTA + jj] = make_double2(0.0, 0.0);
-                for (int n = 0; n <= N; ++n) jrow[n * kCylTA] = 0;
-            }
-        } else if (tid < kCylQB * kCylTA + kCylTA) {
-            const int jj = tid - kCylQB * kCylTA, j = j0 + jj;
-            double cp = 1, sp = 0, s1 = 0, c1 = 1;  // cos, sin of n phi by rotation
-            if (j < a.na) sincos((double)row[j].y, &s1, &c1);
-            for (int n = 0; n <= N; ++n) {
-                cn[n * kCylTA + jj] = cp;
-                sn[n * kCylTA + jj] = sp;
+// cos(n phi), sin(n phi) of every (frame, atom) of the batch by rotation, n ascending. Also clears
+// jmax for the kernel that follows.
+__global__ void __launch_bounds__(128) mp_angle_kernel(MpCylinder a) {
+    const size_t n = (size_t)a.nfb * a.na_pad, n0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.N + 3); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+    for (size_t i = n0; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const int fl = (int)(i / a.na_pad), j = (int)(i - (size_t)fl * a.na_pad);
+        double s1, c1, cp = 1, sp = 0;
+        sincos((double)a.cyl[(size_t)(a.f0 + fl) * a.na_pad + j].y, &s1, &c1);
+        int4* out = a.Tc + (size_t)fl * a.nn * a.na_pad + j;
+        for (int k = 0, at = 0; k < a.nn; ++k) {
+            for (const int order = a.ns[k]; at < order; ++at) {
                 const double cq = cp * c1 - sp * s1;
                 sp = sp * c1 + cp * s1;
                 cp = cq;
             }
+            const int2 c = mp_unit(cp), s = mp_unit(sp);
+            out[(size_t)k * a.na_pad] = make_int4(c.x, c.y, s.x, s.y);
         }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < NPT; ++k) {
-            const int t = tid + k * kCylThreads;
-            if (t < ntask) {
-                const int qq = t / (2 * W), rem = t - qq * 2 * W, n = rem >> 1;
-                const double* jv = Jn + ((size_t)qq * W + n) * kCylTA;
-                const double* tr = ((rem & 1) ? sn : cn) + (size_t)n * kCylTA;
-                const double2* x = X + qq * kCylTA;
-                double2 sacc = acc[k];
-                for (int jj = 0; jj < kCylTA; ++jj) {
-                    const double w = jv[jj] * tr[jj];
-                    sacc.x = fma(x[jj].x, w, sacc.x);
-                    sacc.y = fma(x[jj].y, w, sacc.y);
-                }
-                acc[k] = sacc;
-            }
-        }
-    }
-    __syncthreads();
-    double2* Sv = reinterpret_cast<double2*>(smem);  // [QB][W][cos, sin]
-#pragma unroll
-    for (int k = 0; k < NPT; ++k) {
-        const int t = tid + k * kCylThreads;
-        if (t < ntask) Sv[t] = acc[k];
-    }
-    __syncthreads();
-    const double norm = sqrt(2 * 3.14159265358979323846), h = 0.70710678118654752440;
-    for (int idx = tid; idx < nqb * a.nmom; idx += kCylThreads) {
-        const int qq = idx / a.nmom, k = idx - qq * a.nmom, q = q0 + qq;
-        const double qphi = a.qcyl[3 * q + 1];
-        const double2* S2 = Sv + (size_t)qq * 2 * W;
-        const int l = a.mom[2 * k], m = a.mom[2 * k + 1];
-        double2 v;
-        if (l == 0 && m == 0) {
-            v = S2[0];
-        } else {
-            const int n = m < 2 ? 2 * l : 2 * l - 1;
-            double snq, cnq;
-            sincos(n * qphi, &snq, &cnq);
-            const double2 C = S2[2 * n], S = S2[2 * n + 1];
-            double2 t;  // sum_j X_j J_n cos / sin (n (phi_j - phi_q))
-            if (m == 0 || m == 2) t = make_double2(cnq * C.x + snq * S.x, cnq * C.y + snq * S.y);
-            else t = make_double2(cnq * S.x - snq * C.x, cnq * S.y - snq * C.y);
-            if (m < 2) {
-                const double c = h * 2.0 * ((l & 1) ? -1.0 : 1.0);
-                v = make_double2(c * t.x, c * t.y);
-            } else {  // times i sqrt(1/2) 2 (-1)^(l-1)
-                const double c = h * 2.0 * (((l - 1) & 1) ? -1.0 : 1.0);
-                v = make_double2(-c * t.y, c * t.x);
-            }
-        }
-        a.A[((size_t)q * a.nmom + k) * a.nf + f] = make_double2(norm * v.x, norm * v.y);
     }
 }
 
-size_t cylinder_smem(int N) {
-    const size_t W = (size_t)N + 1;
-    const size_t tiles = (size_t)(kCylQB + 2) * W * kCylTA * sizeof(double) + (size_t)kCylQB * kCylTA * sizeof(double2);
-    return std::max(tiles, (size_t)kCylQB * 2 * W * sizeof(double2));
+// J_n(q_r r), n <= N, and X = b e^{i s z q_z} of every (frame, q, atom) of the batch, and each row's
+// largest magnitude. Bound by the FP64 pipe: atoms in order of radius, so that a warp takes one
+// branch; about 260 FP64 instructions a row of 41 orders.
+__global__ void __launch_bounds__(128) mp_jn_kernel(MpCylinder a) {
+    __shared__ double num[kJnTab];
+    for (int i = threadIdx.x; i < kJnTab; i += blockDim.x) num[i] = i;
+    __syncthreads();
+    const size_t n = (size_t)a.nfb * a.nq * a.na_pad;  // na_pad is a multiple of 32: a warp has one row
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t fq = i / a.na_pad;
+        const int j = (int)(i - fq * a.na_pad), fl = (int)(fq / a.nq), q = (int)(fq - (size_t)fl * a.nq);
+        const float4 c = a.cyl[(size_t)(a.f0 + fl) * a.na_pad + j];
+        const int cl = (int)c.w;  // atoms sit in radius order; w carries the class (-1: padding)
+        const double b = cl >= 0 ? a.cf[(size_t)q * a.nclass + cl] : 0.0;
+        const double qr = a.qcyl[3 * q], qz = a.qcyl[3 * q + 2], z = c.z;
+        double sgn = 1.0;  // parallel_sign, multipole_scatter_device.cpp:944-948
+        if (z != 0 && qz != 0) sgn = (z * qz) / (fabs(z) * fabs(qz));
+        double es, ec;
+        sincos(sgn * z * qz, &es, &ec);
+        double* row = a.Jb + (fq * (a.N + 3)) * a.na_pad + j;
+        row[(size_t)(a.N + 1) * a.na_pad] = b * ec;
+        row[(size_t)(a.N + 2) * a.na_pad] = b * es;
+        cyl_bessel_row(a.N, (double)c.x * qr, row, a.na_pad, num);
+        __syncwarp();
+        for (int l = 0; l < a.N + 3; ++l) {
+            const unsigned mx =
+                __reduce_max_sync(0xffffffffu, (unsigned)__double2hiint(row[(size_t)l * a.na_pad]) & 0x7fffffffu);
+            if ((threadIdx.x & 31) == 0) atomicMax(a.jmax + fq * (a.N + 3) + l, mx);
+        }
+    }
+}
+
+// sum_j X_j J_n(j) (cos, sin)(n phi_j) of one frame for up to 8 orders n and QB q-vectors, in integers
+// as mp_sphere_sum_kernel sums: a lane is an atom, a warp an order (or a part of one's atoms). The
+// tile's X words are shared; J and the angles are read once, straight from memory. X J is one
+// 58-bit product more, taken before the four sums' (18 of the 32-bit multiplications per J, 12 of
+// them in the sums). 5,000 atoms, 64 frames, 10 q, 41 orders: 8.0 ms with the basis before, 2.8 now
+// (1.0 here, 1.6 the Bessel rows).
+template <int QB>
+__global__ void __launch_bounds__(kSumWarps * 32, 2) mp_cylinder_sum_kernel(MpCylinder a) {
+    __shared__ int4 Xs[QB][kSumTile];
+    __shared__ int jexp[kSumWarps][QB], xexp[QB];
+    __shared__ double part[kSumWarps][4 * QB];
+    const int fl = blockIdx.y, q0 = blockIdx.z * QB, nqb = min(QB, a.nq - q0);
+    const int k0 = blockIdx.x * kSumWarps, cnt = min(kSumWarps, a.nn - k0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t qstep = (size_t)(a.N + 3) * a.na_pad;
+    const double* rows = a.Jb + ((size_t)fl * a.nq + q0) * qstep;
+    const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q0) * (a.N + 3);
+    const int jend = (a.na + 31) & ~31;  // <= na_pad; b_j = 0 past na
+    auto exponent = [](unsigned m) { return m >= 0x7ff00000u ? 4096 : max((int)(m >> 20), 1) - 1022; };
+    for (int i = threadIdx.x; i < cnt * nqb; i += kSumWarps * 32)
+        jexp[i / nqb][i % nqb] = exponent(mx[(size_t)(i % nqb) * (a.N + 3) + a.ns[k0 + i / nqb]]);
+    if (threadIdx.x < nqb)
+        xexp[threadIdx.x] = exponent(max(mx[(size_t)threadIdx.x * (a.N + 3) + a.N + 1],
+                                         mx[(size_t)threadIdx.x * (a.N + 3) + a.N + 2]));
+    __syncthreads();
+    const int aw = cnt > 4 ? 1 : cnt > 2 ? 2 : cnt > 1 ? 4 : 8;
+    const int k = warp % cnt, g = warp / cnt, order = a.ns[k0 + k];
+    const bool live = g < aw;
+    const int4* t = a.Tc + ((size_t)fl * a.nn + k0 + k) * a.na_pad + g * 32 + lane;
+    const double* jn = rows + (size_t)order * a.na_pad + g * 32 + lane;
+    int je[QB];
+#pragma unroll
+    for (int q = 0; q < QB; ++q) je[q] = q < nqb ? jexp[k][q] : 0;
+    long long h[QB][4], x[QB][4];
+#pragma unroll
+    for (int q = 0; q < QB; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) h[q][i] = x[q][i] = 0;
+    double total = 0.0;  // of the output this lane holds: 4 q + (re cos, im cos, re sin, im sin)
+    int n = 0;
+    auto flush = [&]() {
+        int p0 = 0, p1 = 0, p2 = 0;
+#pragma unroll
+        for (int o = 0; o < 4 * QB; ++o) {
+            const long long v = h[o / 4][o % 4] + ((x[o / 4][o % 4] + (1 << 28)) >> 29);
+            const int s0 = __reduce_add_sync(0xffffffffu, (int)v & 0x3ffffff);
+            const int s1 = __reduce_add_sync(0xffffffffu, (int)(v >> 26) & 0x3ffffff);
+            const int s2 = __reduce_add_sync(0xffffffffu, (int)(v >> 52));
+            if (lane == o) {
+                p0 = s0;
+                p1 = s1;
+                p2 = s2;
+            }
+            h[o / 4][o % 4] = x[o / 4][o % 4] = 0;
+        }
+        total += fma((double)p2, 4503599627370496.0, fma((double)p1, 67108864.0, (double)p0));
+        n = 0;
+    };
+    int4 tv = make_int4(0, 0, 0, 0);
+    double jv[QB];
+    auto load = [&](int j) {
+        if (j < jend) {
+            tv = *t;
+#pragma unroll
+            for (int q = 0; q < QB; ++q) jv[q] = q < nqb ? jn[q * qstep] : 0.0;
+        }
+        t += aw * 32;
+        jn += aw * 32;
+    };
+    if (live) load(g * 32);
+    for (int j0 = 0; j0 < jend; j0 += kSumTile) {
+        __syncthreads();  // the previous tile has been read
+#pragma unroll
+        for (int q = 0; q < QB; ++q) {
+            const int j = j0 + threadIdx.x;
+            int4 w = make_int4(0, 0, 0, 0);
+            if (q < nqb && j < jend) {
+                const double* p = rows + q * qstep + (size_t)(a.N + 1) * a.na_pad + j;
+                const int2 re = mp_split(mp_fixed(p[0], xexp[q])), im = mp_split(mp_fixed(p[a.na_pad], xexp[q]));
+                w = make_int4(re.x, re.y, im.x, im.y);
+            }
+            Xs[q][threadIdx.x] = w;
+        }
+        __syncthreads();
+        if (!live) continue;
+        for (int c = g * 32; c < kSumTile && j0 + c < jend; c += aw * 32) {
+            const int4 v = tv;
+            int2 jw[QB];
+#pragma unroll
+            for (int q = 0; q < QB; ++q) jw[q] = mp_split(mp_fixed(jv[q], je[q]));
+            load(j0 + c + aw * 32);
+#pragma unroll
+            for (int q = 0; q < QB; ++q) {
+                const int4 w = Xs[q][c + lane];
+                const int2 re = mp_split(mp_mul(jw[q], make_int2(w.x, w.y)));
+                const int2 im = mp_split(mp_mul(jw[q], make_int2(w.z, w.w)));
+                h[q][0] += mp_wide(re.x, v.x, 0);
+                x[q][0] += mp_wide(re.x, v.y, mp_wide(re.y, v.x, 0));
+                h[q][1] += mp_wide(im.x, v.x, 0);
+                x[q][1] += mp_wide(im.x, v.y, mp_wide(im.y, v.x, 0));
+                h[q][2] += mp_wide(re.x, v.z, 0);
+                x[q][2] += mp_wide(re.x, v.w, mp_wide(re.y, v.z, 0));
+                h[q][3] += mp_wide(im.x, v.z, 0);
+                x[q][3] += mp_wide(im.x, v.w, mp_wide(im.y, v.z, 0));
+            }
+            ++n;
+        }
+        if (n > 48) {
+            flush();
+        } else if (n & 8 || n > 16) {  // the cross products' sums (2^57 each) into the high ones
+#pragma unroll
+            for (int o = 0; o < 4 * QB; ++o) {
+                h[o / 4][o % 4] += x[o / 4][o % 4] >> 29;
+                x[o / 4][o % 4] &= (1 << 29) - 1;
+            }
+        }
+    }
+    if (live) {
+        flush();
+        if (lane < 4 * QB) part[warp][lane] = total;
+    }
+    __syncthreads();
+    const double norm = sqrt(2 * 3.14159265358979323846), h2 = 0.70710678118654752440;
+    for (int i = threadIdx.x; i < cnt * nqb; i += kSumWarps * 32) {
+        const int kk = i / nqb, q = i - kk * nqb, nn = a.ns[k0 + kk];
+        double sum[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int w = kk; w < aw * cnt; w += cnt)
+            for (int o = 0; o < 4; ++o) sum[o] += part[w][4 * q + o];
+        const int e = jexp[kk][q] + xexp[q] - 56;
+        const double f = jexp[kk][q] == 4096 || xexp[q] == 4096 ? nan("") : norm;
+        const double2 C = make_double2(f * scalbn(sum[0], e), f * scalbn(sum[1], e));
+        const double2 S = make_double2(f * scalbn(sum[2], e), f * scalbn(sum[3], e));
+        double snq, cnq;
+        sincos(nn * a.qcyl[3 * (q0 + q) + 1], &snq, &cnq);
+        for (int u = a.nmom0[k0 + kk]; u < a.nmom0[k0 + kk + 1]; ++u) {
+            const int mk = a.nout[u], l = a.mom[2 * mk], m = a.mom[2 * mk + 1];
+            double2 v;
+            if (l == 0 && m == 0) {
+                v = C;
+            } else {
+                double2 w;  // sum_j X_j J_n cos / sin (n (phi_j - phi_q))
+                if (m == 0 || m == 2) w = make_double2(cnq * C.x + snq * S.x, cnq * C.y + snq * S.y);
+                else w = make_double2(cnq * S.x - snq * C.x, cnq * S.y - snq * C.y);
+                if (m < 2) {
+                    const double c = h2 * 2.0 * ((l & 1) ? -1.0 : 1.0);
+                    v = make_double2(c * w.x, c * w.y);
+                } else {  // times i sqrt(1/2) 2 (-1)^(l-1)
+                    const double c = h2 * 2.0 * (((l - 1) & 1) ? -1.0 : 1.0);
+                    v = make_double2(-c * w.y, c * w.x);
+                }
+            }
+            a.A[((size_t)(q0 + q) * a.nmom + mk) * a.nf + a.f0 + fl] = v;
+        }
+    }
+}
+constexpr int kCylQ = 5;  // q-vectors of a CTA, at most
+
+template <int QB>
+cudaError_t launch_cylinder_sum(int qb, const MpCylinder& a, dim3 grid, cudaStream_t st) {
+    if (qb < QB) {
+        if constexpr (QB > 1) return launch_cylinder_sum<QB - 1>(qb, a, grid, st);
+    }
+    mp_cylinder_sum_kernel<QB><<<grid, kSumWarps * 32, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -868,6 +1003,20 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
         std::reverse(groups.begin(), groups.end());  // whole groups first
     }
     const size_t npair = pm.size();
+    // cylinder: the orders n of the moments, ascending, each with its moments
+    std::vector<int> ns, nmom0, nout;
+    if (cyl) {
+        std::vector<std::vector<int>> at(2 * (size_t)L + 1);
+        for (size_t k = 0; k < nmom; ++k)
+            at[moments[2 * k + 1] < 2 ? 2 * moments[2 * k] : 2 * moments[2 * k] - 1].push_back((int)k);
+        for (int n = 0; n <= 2 * L; ++n) {
+            if (at[n].empty()) continue;
+            ns.push_back(n);
+            nmom0.push_back((int)nout.size());
+            nout.insert(nout.end(), at[n].begin(), at[n].end());
+        }
+        nmom0.push_back((int)nout.size());
+    }
     // one packed upload of every small input (16-byte aligned pieces)
     std::vector<unsigned char> blob;
     auto put = [&](const void* h, size_t bytes) {
@@ -884,6 +1033,9 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
     const size_t o_pmom = put(pmom.data(), pmom.size() * sizeof(int));
     const size_t o_pout = put(pout.data(), pout.size() * sizeof(int));
     const size_t o_pm = put(pm.data(), pm.size() * sizeof(int));
+    const size_t o_ns = put(ns.data(), ns.size() * sizeof(int));
+    const size_t o_nmom0 = put(nmom0.data(), nmom0.size() * sizeof(int));
+    const size_t o_nout = put(nout.data(), nout.size() * sizeof(int));
     MCK(p->mp_in.ensure(blob.size()));
     MCK(p->mp_amp.ensure(nq * nmom * nf * sizeof(double2)));
     MCK(p->mp_out.ensure(nq * (nf + 2) * sizeof(double2)));
@@ -934,12 +1086,12 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
         if (cyl) memcpy(s.mp_axis, axis, sizeof(s.mp_axis));
     }
     const double* d_cf = reinterpret_cast<const double*>(dptr(o_cf));
+    // frame batches: basis of up to a quarter of the free memory (at most 16 GB), so that
+    // one contraction launch has thousands of CTAs
+    size_t free_b = 0, total_b = 0;
+    MCK(cudaMemGetInfo(&free_b, &total_b));
+    const size_t budget = std::max<size_t>((size_t)1 << 28, std::min<size_t>((size_t)16 << 30, free_b / 4));
     if (!cyl) {
-        // frame batches: basis of up to a quarter of the free memory (at most 16 GB), so that
-        // one contraction launch has thousands of CTAs
-        size_t free_b = 0, total_b = 0;
-        MCK(cudaMemGetInfo(&free_b, &total_b));
-        const size_t budget = std::max<size_t>((size_t)1 << 28, std::min<size_t>((size_t)16 << 30, free_b / 4));
         const size_t per_frame = na_pad * (nq * (L + 1) * sizeof(double) + npair * sizeof(int4));
         const size_t nfb = std::max<size_t>(1, std::min<size_t>({nf, budget / per_frame, (size_t)65535}));  // grid y
         const size_t ysm = legendre_bytes(L);
@@ -999,28 +1151,45 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             launches += 2;
         }
     } else {
+        const int N = 2 * L;
+        const size_t nn = ns.size();
+        const size_t per_frame = na_pad * (nq * (N + 3) * sizeof(double) + nn * sizeof(int4));
+        const size_t nfb = std::max<size_t>(1, std::min<size_t>({nf, budget / per_frame, (size_t)65535}));  // grid y
+        MCK(p->mp_Jb.ensure(nfb * nq * (N + 3) * na_pad * sizeof(double)));
+        MCK(p->mp_Yc.ensure(nfb * nn * na_pad * sizeof(int4)));
+        MCK(p->mp_ycf.ensure(nfb * nq * (N + 3) * sizeof(unsigned)));
+        const size_t nqc = (nq + kCylQ - 1) / kCylQ, qb = (nq + nqc - 1) / nqc;  // as even as they go
         MpCylinder ca{};
         ca.cyl = s.mp_xyz.as<float4>();
-        ca.cls = s.cls.as<int>();
         ca.cf = d_cf;
         ca.qcyl = reinterpret_cast<const double*>(dptr(o_qin));
+        ca.Jb = p->mp_Jb.as<double>();
+        ca.jmax = p->mp_ycf.as<unsigned>();
+        ca.Tc = p->mp_Yc.as<int4>();
+        ca.ns = reinterpret_cast<const int*>(dptr(o_ns));
+        ca.nmom0 = reinterpret_cast<const int*>(dptr(o_nmom0));
+        ca.nout = reinterpret_cast<const int*>(dptr(o_nout));
         ca.mom = reinterpret_cast<const int*>(dptr(o_mom));
         ca.A = p->mp_amp.as<double2>();
         ca.na_pad = (int)na_pad;
         ca.na = (int)s.na;
         ca.nclass = (int)nclass;
         ca.nq = (int)nq;
-        ca.N = 2 * L;
+        ca.N = N;
+        ca.nn = (int)nn;
         ca.nmom = (int)nmom;
         ca.nf = (int)nf;
-        const size_t sm = cylinder_smem(2 * L);
-        if (sm > 48 * 1024) MCK(cudaFuncSetAttribute(mp_cylinder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        for (size_t f0 = 0; f0 < nf; f0 += 65535) {  // frames in grid y, at most 65,535 per launch
+        for (size_t f0 = 0; f0 < nf; f0 += nfb) {
             ca.f0 = (int)f0;
-            const unsigned nfl = (unsigned)std::min<size_t>(65535, nf - f0);
-            mp_cylinder_kernel<<<dim3((unsigned)((nq + kCylQB - 1) / kCylQB), nfl), kCylThreads, sm, st>>>(ca);
+            ca.nfb = (int)std::min(nfb, nf - f0);
+            const size_t na2 = (size_t)ca.nfb * na_pad;
+            mp_angle_kernel<<<grid_blocks(na2, 128, 64), 128, 0, st>>>(ca);
             MCK(cudaGetLastError());
-            ++launches;
+            mp_jn_kernel<<<grid_blocks(na2 * nq, 128, 16), 128, 0, st>>>(ca);
+            MCK(cudaGetLastError());
+            MCK(launch_cylinder_sum<kCylQ>(
+                (int)qb, ca, dim3((unsigned)((nn + kSumWarps - 1) / kSumWarps), (unsigned)ca.nfb, (unsigned)nqc), st));
+            launches += 3;
         }
     }
     const size_t phase_launches = launches;
