@@ -13,9 +13,8 @@
 //   * translations and the fit's apply step: one thread per (frame, atom), again with
 //     explicitly rounded operations in the reference's order;
 //   * the fit's 3x3 correlation matrices (center_of_mass.cpp:79-98) are summed per frame on
-//     the device; their SVDs (3x3, per frame) run on the host with a one-sided Jacobi
-//     method, and the rotations go back to the device.
-// Everything stays resident; the host sees nf x 9 doubles per fit step.
+//     the device, and so are their SVDs (3x3, one thread per frame, a one-sided Jacobi method).
+// Everything stays resident; no step waits for the host.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -288,60 +287,77 @@ unsigned grid_for(size_t n, int threads) {
 }
 
 // ---------------------------------------------------------------------------------------
-// 3x3 fit rotation (host)
+// 3x3 fit rotation
 // ---------------------------------------------------------------------------------------
-double det3(const double* a) {
+__device__ double det3(const double* a) {
     return a[0] * (a[4] * a[8] - a[5] * a[7]) - a[1] * (a[3] * a[8] - a[5] * a[6]) + a[2] * (a[3] * a[7] - a[4] * a[6]);
+}
+
+// One rotation of Hestenes' iteration on columns P and Q; whether there was something to rotate:
+// products below 2.3e-16 of the columns' lengths are rounding (a bar of 1e-17 was mostly never
+// met: 45 sweeps instead of 3, which turned rounding errors over and over; mean error of the
+// rotation 4.7e-16 instead of 5.4e-16).
+template <int P, int Q>
+__device__ bool svd3_rotate(double (&A)[9], double (&V)[9]) {
+    double alpha = 0, beta = 0, gamma = 0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        alpha += A[3 * r + P] * A[3 * r + P];
+        beta += A[3 * r + Q] * A[3 * r + Q];
+        gamma += A[3 * r + P] * A[3 * r + Q];
+    }
+    if (gamma == 0.0 || fabs(gamma) <= 2.3e-16 * sqrt(alpha * beta)) return false;
+    const double zeta = (beta - alpha) / (2.0 * gamma);
+    const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+    const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const double ap = A[3 * r + P], aq = A[3 * r + Q];
+        A[3 * r + P] = c * ap - s * aq;
+        A[3 * r + Q] = s * ap + c * aq;
+        const double vp = V[3 * r + P], vq = V[3 * r + Q];
+        V[3 * r + P] = c * vp - s * vq;
+        V[3 * r + Q] = s * vp + c * vq;
+    }
+    return true;
 }
 
 // K = U diag(S) V^T by one-sided Jacobi rotations of K's columns (Hestenes), singular
 // values in descending order as LAPACK's gesvd returns them. Row-major 3x3.
-void svd3(const double* K, double* U, double* S, double* V) {
-    double A[9];
-    memcpy(A, K, sizeof(A));
-    for (int i = 0; i < 9; ++i) V[i] = (i % 4 == 0) ? 1.0 : 0.0;
-    const int pairs[3][2] = {{0, 1}, {0, 2}, {1, 2}};
+__device__ void svd3(const double* K, double (&U)[9], double (&S)[3], double (&V)[9]) {
+    double A[9], W[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        A[i] = K[i];
+        W[i] = (i % 4 == 0) ? 1.0 : 0.0;
+    }
     for (int sweep = 0; sweep < 64; ++sweep) {
-        bool rotated = false;
-        for (const auto& pq : pairs) {
-            const int p = pq[0], q = pq[1];
-            double alpha = 0, beta = 0, gamma = 0;
-            for (int r = 0; r < 3; ++r) {
-                alpha += A[3 * r + p] * A[3 * r + p];
-                beta += A[3 * r + q] * A[3 * r + q];
-                gamma += A[3 * r + p] * A[3 * r + q];
-            }
-            if (gamma == 0.0 || std::fabs(gamma) <= 1e-17 * std::sqrt(alpha * beta)) continue;
-            rotated = true;
-            const double zeta = (beta - alpha) / (2.0 * gamma);
-            const double t = std::copysign(1.0, zeta) / (std::fabs(zeta) + std::sqrt(1.0 + zeta * zeta));
-            const double c = 1.0 / std::sqrt(1.0 + t * t), s = c * t;
-            for (int r = 0; r < 3; ++r) {
-                const double ap = A[3 * r + p], aq = A[3 * r + q];
-                A[3 * r + p] = c * ap - s * aq;
-                A[3 * r + q] = s * ap + c * aq;
-                const double vp = V[3 * r + p], vq = V[3 * r + q];
-                V[3 * r + p] = c * vp - s * vq;
-                V[3 * r + q] = s * vp + c * vq;
-            }
-        }
+        bool rotated = svd3_rotate<0, 1>(A, W);
+        rotated = svd3_rotate<0, 2>(A, W) || rotated;
+        rotated = svd3_rotate<1, 2>(A, W) || rotated;
         if (!rotated) break;
     }
-    int order[3] = {0, 1, 2};
     double nrm[3];
-    for (int j = 0; j < 3; ++j)
-        nrm[j] = std::sqrt(A[j] * A[j] + A[3 + j] * A[3 + j] + A[6 + j] * A[6 + j]);
-    std::sort(order, order + 3, [&](int a, int b) { return nrm[a] > nrm[b]; });
-    double Vs[9];
+    for (int j = 0; j < 3; ++j) nrm[j] = sqrt(A[j] * A[j] + A[3 + j] * A[3 + j] + A[6 + j] * A[6 + j]);
+    int order[3] = {0, 1, 2};
+    auto sort2 = [&](int a, int b) {
+        if (nrm[order[b]] > nrm[order[a]]) {
+            const int o = order[a];
+            order[a] = order[b];
+            order[b] = o;
+        }
+    };
+    sort2(0, 1);
+    sort2(1, 2);
+    sort2(0, 1);
     for (int j = 0; j < 3; ++j) {
         const int o = order[j];
         S[j] = nrm[o];
         for (int r = 0; r < 3; ++r) {
             U[3 * r + j] = nrm[o] > 0 ? A[3 * r + o] / nrm[o] : 0.0;
-            Vs[3 * r + j] = V[3 * r + o];
+            V[3 * r + j] = W[3 * r + o];
         }
     }
-    memcpy(V, Vs, sizeof(Vs));
     // complete U where singular values vanish: unit vectors orthogonal to the others
     const double tiny = 1e-300;
     if (S[0] <= tiny) {
@@ -350,13 +366,11 @@ void svd3(const double* K, double* U, double* S, double* V) {
     }
     if (S[1] <= tiny) {  // a unit vector orthogonal to u0
         const double u0[3] = {U[0], U[3], U[6]};
-        const int m = std::fabs(u0[0]) <= std::fabs(u0[1]) && std::fabs(u0[0]) <= std::fabs(u0[2]) ? 0
-                      : std::fabs(u0[1]) <= std::fabs(u0[2])                                      ? 1
-                                                                                                  : 2;
+        const int m = fabs(u0[0]) <= fabs(u0[1]) && fabs(u0[0]) <= fabs(u0[2]) ? 0 : fabs(u0[1]) <= fabs(u0[2]) ? 1 : 2;
         double e[3] = {0, 0, 0};
         e[m] = 1.0;
         double w[3] = {e[0] - u0[m] * u0[0], e[1] - u0[m] * u0[1], e[2] - u0[m] * u0[2]};
-        const double n = std::sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+        const double n = sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
         for (int r = 0; r < 3; ++r) U[3 * r + 1] = w[r] / n;
     }
     if (S[2] <= tiny) {  // u2 = u0 x u1
@@ -368,16 +382,19 @@ void svd3(const double* K, double* U, double* S, double* V) {
 }
 
 // Rotation of Fit (center_of_mass.cpp:100-112): K = U S V^T, d = det(U V^T),
-// R = U diag(1, 1, d) V^T.
-void fit_rotation(const double* K, double* R) {
-    double U[9], S[3], V[9];
-    svd3(K, U, S, V);
-    double UVt[9];
+// R = U diag(1, 1, d) V^T. One thread per frame: a chain of some 3,000 dependent FP64 operations,
+// latency alone (37 us for 256 frames; on the host, 64 sweeps and the copies both ways, 0.75 ms).
+__global__ void __launch_bounds__(32) pp_rotation_kernel(const double* __restrict__ K, int nf, double* __restrict__ R) {
+    const int f = blockIdx.x * 32 + threadIdx.x;
+    if (f >= nf) return;
+    double U[9], S[3], V[9], UVt[9];
+    svd3(K + 9 * (size_t)f, U, S, V);
     for (int r = 0; r < 3; ++r)
         for (int c = 0; c < 3; ++c) UVt[3 * r + c] = U[3 * r] * V[3 * c] + U[3 * r + 1] * V[3 * c + 1] + U[3 * r + 2] * V[3 * c + 2];
     const double d = det3(UVt);
     for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 3; ++c) R[3 * r + c] = U[3 * r] * V[3 * c] + U[3 * r + 1] * V[3 * c + 1] + d * U[3 * r + 2] * V[3 * c + 2];
+        for (int c = 0; c < 3; ++c)
+            R[9 * (size_t)f + 3 * r + c] = U[3 * r] * V[3 * c] + U[3 * r + 1] * V[3 * c + 1] + d * U[3 * r + 2] * V[3 * c + 2];
 }
 
 int fail(std::string& m, int code, const std::string& what) {
@@ -492,7 +509,6 @@ extern "C" int sass_stage_frames_prepass(sass_plan* p, const float* frames, size
     const unsigned gf = (unsigned)((nf + kPerFrameThreads - 1) / kPerFrameThreads);
     auto L = [&](size_t off) { return reinterpret_cast<const size_t*>(dl + off); };
     auto D = [&](size_t off) { return reinterpret_cast<const double*>(dl + off); };
-    std::vector<double> hK(nf * 9), hR(nf * 9);
 
     for (size_t i = 0; i < nsteps; ++i) {
         const sass_prepass_step& q = steps[i];
@@ -531,10 +547,7 @@ extern "C" int sass_stage_frames_prepass(sass_plan* p, const float* frames, size
                                ref_one ? com_ref : ComJob{C, nref * 3, nullptr, D(o.rmass), nref, nfi, va}, st);
                     launch_kmat(C, ref_one ? D(o.refxyz) : nullptr, D(o.rmass), nref, nfi, vb, va, ref_one, vK, st);
                     PCK(cudaGetLastError());
-                    PCK(cudaMemcpyAsync(hK.data(), vK, nf * 9 * sizeof(double), cudaMemcpyDeviceToHost, st));
-                    PCK(cudaStreamSynchronize(st));
-                    for (size_t f = 0; f < nf; ++f) fit_rotation(&hK[9 * f], &hR[9 * f]);
-                    PCK(cudaMemcpyAsync(vR, hR.data(), nf * 9 * sizeof(double), cudaMemcpyHostToDevice, st));
+                    pp_rotation_kernel<<<(unsigned)((nf + 31) / 32), 32, 0, st>>>(vK, nfi, vR);
                     pp_fit_apply_kernel<<<grid_for(nf * nref, 256), 256, 0, st>>>(C, nref, nfi, vR, vb, va, ref_one);
                     if (q.nfit)
                         pp_scatter_kernel<<<grid_for(nf * q.nfit, 256), 256, 0, st>>>(W, nsys, L(o.ftg), L(o.fsrc), q.nfit,
