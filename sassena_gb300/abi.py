@@ -179,6 +179,17 @@ def load(path=LIB_PATH):
     return L
 
 
+def _results(nq, nf):
+    """Buffers of (fqt, fq, fq2) as (re, im) pairs, which a successful call fills: left unset, so that
+    a large one is not written twice."""
+    return np.empty((nq, nf, 2)), np.empty((nq, 2)), np.empty((nq, 2))
+
+
+def _complex(a):
+    """The pairs [..., 2] as complex numbers, in place."""
+    return a.view(np.complex128)[..., 0]
+
+
 def _ptr(a):
     return a.ctypes.data_as(_vp) if isinstance(a, np.ndarray) else _vp(a)
 
@@ -279,7 +290,7 @@ class Plan:
             e.fit_target, e.nfit = lst("fit_target")
             e.fit_source, _ = lst("fit_source")
             e.translations, _ = lst("translations", np.float64, (-1, 3))
-        out = np.zeros((self.nf, self.na, 3), dtype=np.float32) if return_staged else None
+        out = np.empty((self.nf, self.na, 3), dtype=np.float32) if return_staged else None
         self._check(self.lib.sass_stage_frames_prepass(self._h, _ptr(fr), nsys, _ptr(ms), arr, len(steps),
                                                        _ptr(tg), _ptr(out) if return_staged else None))
         return out
@@ -300,15 +311,12 @@ class Plan:
         cf = np.ascontiguousarray(class_factors, dtype=np.float64).reshape(nq, self.nclass)
         mom = np.ascontiguousarray(moments, dtype=np.int32).reshape(-1, 2)
         ax = np.ascontiguousarray(axis, dtype=np.float64)
-        fqt = np.zeros((nq, self.nf, 2))
-        fq = np.zeros((nq, 2))
-        fq2 = np.zeros((nq, 2))
+        fqt, fq, fq2 = _results(nq, self.nf)
         t = {"sphere": 0, "cylinder": 1}[kind]
         self._check(self.lib.sass_multipole_compute(self._h, t, nq, _ptr(q), _ptr(cf), len(mom),
                                                     _ptr(mom), _ptr(ax), _ptr(fqt), _ptr(fq),
                                                     _ptr(fq2)))
-        return (fqt[..., 0] + 1j * fqt[..., 1], fq[:, 0] + 1j * fq[:, 1],
-                fq2[:, 0] + 1j * fq2[:, 1])
+        return _complex(fqt), _complex(fq), _complex(fq2)
 
     def set_poly(self, poly_pairs):
         """Pairs of each lane's q-vectors whose sin/cos use the FP32 pipe (direct kernel)."""
@@ -329,13 +337,10 @@ class Plan:
         nq = len(offs) - 1
         sv = np.ascontiguousarray(subvectors, dtype=np.float64).reshape(-1, 3)
         cf = np.ascontiguousarray(class_factors, dtype=np.float64).reshape(nq, self.nclass)
-        fqt = np.zeros((nq, self.nf, 2))
-        fq = np.zeros((nq, 2))
-        fq2 = np.zeros((nq, 2))
+        fqt, fq, fq2 = _results(nq, self.nf)
         self._check(self.lib.sass_compute(self._h, nq, _ptr(offs), _ptr(sv), _ptr(cf), _ptr(fqt),
                                           _ptr(fq), _ptr(fq2), 0))
-        return (fqt[..., 0] + 1j * fqt[..., 1], fq[:, 0] + 1j * fq[:, 1],
-                fq2[:, 0] + 1j * fq2[:, 1])
+        return _complex(fqt), _complex(fq), _complex(fq2)
 
     def compute_device(self, sub_offsets, d_subvectors, d_class_factors, d_fqt, d_fq, d_fq2):
         """All array arguments except sub_offsets are device pointers (ints)."""
@@ -348,10 +353,10 @@ class Plan:
         sv = np.ascontiguousarray(subvectors, dtype=np.float64).reshape(-1, 3)
         sh = np.ascontiguousarray(sub_shell, dtype=np.int32)
         cf = np.ascontiguousarray(class_factors, dtype=np.float64).reshape(-1, self.nclass)
-        out = np.zeros((len(sv), self.nf, 2))
+        out = np.empty((len(sv), self.nf, 2))
         self._check(self.lib.sass_amplitudes(self._h, len(sv), _ptr(sv), _ptr(sh), len(cf),
                                              _ptr(cf), _ptr(out)))
-        return out[..., 0] + 1j * out[..., 1]
+        return _complex(out)
 
     def timing(self):
         t = Timing()
@@ -461,11 +466,9 @@ class Batch:
 
     def results(self, i):
         nq, nf = self.shapes[i]
-        fqt = np.zeros((nq, nf, 2))
-        fq = np.zeros((nq, 2))
-        fq2 = np.zeros((nq, 2))
+        fqt, fq, fq2 = _results(nq, nf)
         self._check(self.lib.sass_batch_results(self._h, i, _ptr(fqt), _ptr(fq), _ptr(fq2)))
-        return (fqt[..., 0] + 1j * fqt[..., 1], fq[:, 0] + 1j * fq[:, 1], fq2[:, 0] + 1j * fq2[:, 1])
+        return _complex(fqt), _complex(fq), _complex(fq2)
 
     def timing(self):
         t = Timing()
@@ -563,13 +566,12 @@ def compute_cv(plan, net, qlen, dirs, class_factors, nquad=32768):
     d = np.ascontiguousarray(dirs, np.float64).reshape(-1, 3)
     cf = np.ascontiguousarray(class_factors, np.float64).reshape(len(q), plan.nclass)
     nq, nf = len(q), plan.nf
-    a, b = np.zeros((nq, nf, 2)), np.zeros((nq, nf, 2))
-    c, e = np.zeros((nq, 2)), np.zeros((nq, 2))
+    a, c, e = _results(nq, nf)
+    b = np.empty_like(a)
     diag = np.zeros((nq, 3))
     plan._check(plan.lib.sass_compute_cv(plan._h, net._h, nq, _ptr(q), len(d), _ptr(d), _ptr(cf),
                                          nquad, _ptr(a), _ptr(b), _ptr(c), _ptr(e), _ptr(diag)))
-    z = lambda v: v[..., 0] + 1j * v[..., 1]  # noqa: E731
-    return z(a), z(b), z(c), z(e), diag
+    return _complex(a), _complex(b), _complex(c), _complex(e), diag
 
 
 def probe_pipes(device=0):
