@@ -111,4 +111,14 @@ __device__ __forceinline__ double2 csub(double2 a, double2 b) {
     return make_double2(a.x - b.x, a.y - b.y);
 }
 
+// Atom j of a row of the class-sorted copy. Atoms lie in pairs, (x0 x1 y0 y1) (z0 z1 w0 w1), so that
+// two of them are the halves of paired FP32 operands.
+__device__ __forceinline__ void store_paired(float4* row, int j, float4 v) {
+    float* p = reinterpret_cast<float*>(row + (j & ~1)) + (j & 1);
+    p[0] = v.x;
+    p[2] = v.y;
+    p[4] = v.z;
+    p[6] = v.w;
+}
+
 }  // namespace sassgpu

@@ -713,7 +713,7 @@ __global__ void stage_kernel(const float* __restrict__ raw, int nf, int na, int 
                 r.y = p[1];
                 r.z = p[2];
             }
-            if (xyz_rec) xyz_rec[f * na_rec + rec_inv[j]] = make_float4(r.x, r.y, r.z, 1.f);
+            if (xyz_rec) store_paired(xyz_rec + f * na_rec, rec_inv[j], make_float4(r.x, r.y, r.z, 1.f));
             far = max(far, __float_as_uint(r.x * r.x + r.y * r.y + r.z * r.z) & 0x7fffffffu);
         }
         xyz[idx] = r;

@@ -1102,7 +1102,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     std::vector<GridTileDesc> gtiles;
     std::vector<double> gshells;
     std::vector<size_t> gitem;
-    size_t gws = 256;  // the weights' coefficients first
+    size_t gws = 0;
     grid_table_ = 0;
     for (size_t i = 0; i < items.size(); ++i) {
         if (!grid_on[i]) continue;
@@ -1448,13 +1448,13 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
         ++phase_launches;
     }
     if (coherent && ngrid_tiles_) {
-        ECK(launch_grid_tables(d_gsys_, ngrid_systems_, grid_table_, d_gshells_, grid_set_, grid_ws_.as<float2>(), st));
+        ECK(launch_grid_tables(d_gsys_, ngrid_systems_, grid_table_, d_gshells_, st));
         GridLaunch gl{};
         gl.systems = d_gsys_;
         gl.tiles = d_gtiles_;
         gl.ntiles = ngrid_tiles_;
         gl.counter = counter_.as<unsigned>() + 3;
-        gl.coef = grid_ws_.as<float2>();
+        gl.set = grid_set_;
         ECK(launch_phase_grid(gl, grid_points_, grid_frames_, st));
         launches += 2;
         ++phase_launches;

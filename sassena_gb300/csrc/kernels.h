@@ -155,7 +155,7 @@ struct RecGroup {
 };
 
 struct RecSystem {
-    const float4* xyzw;       // class-sorted coordinates [nf][na_rec]; padding atoms at the origin
+    const float4* xyzw;       // class-sorted coordinates [nf][na_rec] in pairs; padding atoms at the origin
     const int* block_class;   // [na_rec / 32] class (low 16 bits) | padding atoms << 16 of every 32-atom block
     const double* cf;         // [nq][nclass] class factors
     const double* dirs;       // [nd][3] base vectors (FP64)
@@ -200,7 +200,7 @@ cudaError_t launch_permute_stage(const float4* src, int na_pad_src, const int* m
 // Gridded phase sum (FP32 form): all shells of a direction from one grid of its projections.
 // ---------------------------------------------------------------------------------------
 struct GridSystem {
-    const float4* xyzw;       // class-sorted coordinates [nf][na_rec], w = 0 for padding atoms
+    const float4* xyzw;       // class-sorted coordinates [nf][na_rec] in pairs, w = 0 for padding atoms
     const int* block_class;   // [na_rec / 32] class | padding atoms << 16
     const double* cf;         // [nq][nclass] class factors
     const double* dirs;       // [nd][3] base vectors
@@ -231,7 +231,7 @@ struct GridLaunch {
     const GridTileDesc* tiles;
     int ntiles;
     unsigned int* counter;    // work-queue counter, zero before the launch
-    const float2* coef;       // [9] weight coefficients (launch_grid_tables)
+    int set;                  // weights
     int grid_bytes, ring_bytes;  // set by launch_phase_grid
 };
 
@@ -242,8 +242,8 @@ constexpr double kGridSigma[2] = {3.0, 4.0};  // grid points per half period at 
 double grid_deconvolution(int set, double l);
 int grid_ctas(int grid_points, int ring_frames);
 // shells: per system [nq] lam_k h / 2 pi, then [nq] 1 / D(lam_k h)
-cudaError_t launch_grid_tables(const GridSystem* systems, int nsys, int max_points, const double* shells, int set,
-                               float2* coef, cudaStream_t st);
+cudaError_t launch_grid_tables(const GridSystem* systems, int nsys, int max_points, const double* shells,
+                               cudaStream_t st);
 cudaError_t launch_phase_grid(GridLaunch a, int grid_points, int ring_frames, cudaStream_t st);
 
 // ---------------------------------------------------------------------------------------
@@ -411,7 +411,7 @@ cudaError_t launch_store_kernel(const double2* tw64, int lg_tw, double2* k64, fl
                                 int lg, cudaStream_t st);
 
 // Staging: raw frame-major float [nf][na][3] -> float4 [nf][na_pad] (minus centre); with
-// xyz_rec, also the class-sorted copy xyz_rec[f][rec_inv[j]] = (x, y, z, 1). `raw` may be
+// xyz_rec, also the class-sorted copy with atom j at rec_inv[j] (x, y, z, 1). `raw` may be
 // host memory the device reads in place.
 // With `rmax2` (zeroed by the caller) also the largest |r|^2 of the staged frames, as float bits.
 cudaError_t launch_stage(const float* raw, int nf, int na, int na_pad, double cx, double cy,

@@ -30,12 +30,13 @@
 // so the adds have no bank conflicts. The 32 lanes of a tile are 32 directions of one frame, or
 // 16 x 2 or 8 x 4 for the directions left over. The four warps of a CTA share the grid: each
 // takes every fourth block of 32 atoms, and then its share of the shells' transforms. Issue
-// bounds it: about 44 instructions per 32 (atom, direction, frame).
+// and the shared-memory adds bound it: about 31 instructions, six of them adds, per 32 (atom,
+// direction, frame), and the transforms of the grid.
 //
 // Measured on a GB300 (phase kernel; before: shell recurrence, direct kernel for the batch):
-//   100,000 atoms x 16 frames x 100 shells x 250 directions     6.3 -> 0.86 ms
+//   100,000 atoms x 16 frames x 100 shells x 250 directions     6.3 -> 0.80 ms
 //   8 uneven systems, 5 to 30 unevenly spaced shells            11.6 -> 2.8 ms
-//   10,000 atoms x 1,024 frames x 20 shells x 500 directions   15.3 -> 8.5 ms
+//   10,000 atoms x 1,024 frames x 20 shells x 500 directions   15.3 -> 7.8 ms
 #include <algorithm>
 #include <cmath>
 
@@ -145,54 +146,69 @@ __device__ __noinline__ void grid_flush(const int* __restrict__ col, float4* __r
     }
 }
 
+// Both halves' coefficients [set][weight][power of z], operands from constant memory: in registers
+// they took 36, and the loop could not be unrolled as far (8.45 -> 8.25 ms paired alone, 7.83 with these
+// and sixteen pairs a turn).
 struct GridCoef {
-    float2 c[3][3];  // pairs of mirrored weights: (even, odd) coefficients of z^0, z^2, z^4
+    float2 c[2][3][6];
+    constexpr GridCoef() : c{} {
+        for (int s = 0; s < 2; ++s)
+            for (int n = 0; n < 3; ++n)
+                for (int k = 0; k < 6; ++k) c[s][n][k].x = c[s][n][k].y = grid_coef(s, n, k);
+    }
 };
+__constant__ GridCoef kGridCoef;
 
-// Adds one atom: its six weights in grid units, rounded by adding 1.5 2^23, whose bits are then
-// taken off as an integer.
-__device__ __forceinline__ void grid_add(const GridCoef& w, const float4 r, float ux, float uy, float uz, float bw,
-                                         unsigned colbase) {
+// Adds two atoms, one in each half of the paired FP32 instructions (33 of them; 26 single and 12
+// paired ones an atom at a time): their six weights in grid units, rounded by adding 1.5 2^23,
+// whose bits are then taken off as an integer.
+template <int SET>
+__device__ __forceinline__ void grid_add2(const float4 xy, const float4 zw, float2 ux, float2 uy, float2 uz,
+                                          float2 bw, unsigned colbase) {
+    const float2 magic = make_float2(12582912.f, 12582912.f);
     // the middle of the six points lies between two of them: the half unit puts it on an integer
-    const float x = fmaf(r.z, uz, fmaf(r.y, uy, fmaf(r.x, ux, -0.5f)));
-    const float t = __fadd_rn(x, 12582912.f);  // rounds to the nearest integer
-    const float z = __fsub_rn(x, __fsub_rn(t, 12582912.f));
-    const unsigned p = colbase + (__float_as_uint(t) << 7);
-    const float wt = __fmul_rn(r.w, bw), z2 = __fmul_rn(z, z);
-    const float2 zz = make_float2(z2, z2);
-    float c[6];
+    const float2 x = __ffma2_rn(make_float2(zw.x, zw.y), uz,
+                                __ffma2_rn(make_float2(xy.z, xy.w), uy,
+                                           __ffma2_rn(make_float2(xy.x, xy.y), ux, make_float2(-0.5f, -0.5f))));
+    const float2 t = __fadd2_rn(x, magic);  // rounds to the nearest integer
+    const float2 r = __fadd2_rn(t, make_float2(-12582912.f, -12582912.f));
+    const float2 z = __ffma2_rn(r, make_float2(-1.f, -1.f), x), nz = __ffma2_rn(x, make_float2(-1.f, -1.f), r);
+    const float2 wt = __fmul2_rn(make_float2(zw.z, zw.w), bw), z2 = __fmul2_rn(z, z);
+    const unsigned p0 = colbase + (__float_as_uint(t.x) << 7), p1 = colbase + (__float_as_uint(t.y) << 7);
+    const auto& w = kGridCoef.c[SET];
+    float2 v[6];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const float2 eo = __ffma2_rn(__ffma2_rn(w.c[i][2], zz, w.c[i][1]), zz, w.c[i][0]);
-        c[i] = fmaf(z, eo.y, eo.x);
-        c[5 - i] = fmaf(-z, eo.y, eo.x);
+        const float2 e = __ffma2_rn(__ffma2_rn(w[i][4], z2, w[i][2]), z2, w[i][0]);
+        const float2 o = __ffma2_rn(__ffma2_rn(w[i][5], z2, w[i][3]), z2, w[i][1]);
+        v[i] = __ffma2_rn(wt, __ffma2_rn(z, o, e), magic);
+        v[5 - i] = __ffma2_rn(wt, __ffma2_rn(nz, o, e), magic);
     }
-#define GRID_ADD(i)                                                                       \
-    asm volatile("red.shared.add.u32 [%0 + %1], %2;" ::"r"(p), "n"((i) * 128),            \
-                 "r"(__float_as_uint(fmaf(wt, c[i], 12582912.f)) - 0x4B400000u)            \
+#define GRID_ADD(P, i, V)                                                                                     \
+    asm volatile("red.shared.add.u32 [%0 + %1], %2;" ::"r"(P), "n"((i) * 128), "r"(__float_as_uint(V) - 0x4B400000u) \
                  : "memory")
-    GRID_ADD(0);
-    GRID_ADD(1);
-    GRID_ADD(2);
-    GRID_ADD(3);
-    GRID_ADD(4);
-    GRID_ADD(5);
+    GRID_ADD(p0, 0, v[0].x);
+    GRID_ADD(p0, 1, v[1].x);
+    GRID_ADD(p0, 2, v[2].x);
+    GRID_ADD(p0, 3, v[3].x);
+    GRID_ADD(p0, 4, v[4].x);
+    GRID_ADD(p0, 5, v[5].x);
+    GRID_ADD(p1, 0, v[0].y);
+    GRID_ADD(p1, 1, v[1].y);
+    GRID_ADD(p1, 2, v[2].y);
+    GRID_ADD(p1, 3, v[3].y);
+    GRID_ADD(p1, 4, v[4].y);
+    GRID_ADD(p1, 5, v[5].y);
 #undef GRID_ADD
 }
 
+template <int SET>
 __global__ void __launch_bounds__(kGridWarps * 32, 4) phase_grid_kernel(const GridLaunch a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ unsigned s_unit;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int* col = reinterpret_cast<int*>(smem) + lane;
     float4* ring = reinterpret_cast<float4*>(smem + a.grid_bytes + warp * a.ring_bytes);
-    // loaded, not compile-time constants: these stay in registers
-    GridCoef wc;
-#pragma unroll
-    for (int i = 0; i < 9; ++i)
-        asm volatile("ld.global.v2.f32 {%0, %1}, [%2];"
-                     : "=f"(wc.c[i / 3][i % 3].x), "=f"(wc.c[i / 3][i % 3].y)
-                     : "l"(a.coef + i));
     auto clear = [&](int points) {
         for (int i = threadIdx.x; i < points * 8; i += kGridWarps * 32)
             reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -245,8 +261,10 @@ __global__ void __launch_bounds__(kGridWarps * 32, 4) phase_grid_kernel(const Gr
                 }
                 __syncwarp();
                 const float4* at = ring + (slot * F + fl) * 32;
-#pragma unroll 16
-                for (int j = 0; j < 32; ++j) grid_add(wc, at[j], ux, uy, uz, bw, colbase);
+#pragma unroll
+                for (int j = 0; j < 32; j += 2)
+                    grid_add2<SET>(at[j], at[j + 1], make_float2(ux, ux), make_float2(uy, uy), make_float2(uz, uz),
+                                   make_float2(bw, bw), colbase);
                 __syncwarp();  // this slot is refilled two blocks on
             }
             __syncthreads();
@@ -265,12 +283,7 @@ __global__ void __launch_bounds__(kGridWarps * 32, 4) phase_grid_kernel(const Gr
 // atoms (then a slice is summed once): the same at all shells, finite, and within 16 of each other
 // so that no atom is lost in the grid's units; the atoms' weights per class in those units, the
 // unit itself (gw[nclass]) and the factors per class and shell.
-__global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const double* __restrict__ shells, int set,
-                                   float2* __restrict__ coef) {
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 9) {
-        const int n = threadIdx.x / 3, k = 2 * (threadIdx.x % 3);  // [weight][power of z^2]
-        coef[threadIdx.x] = make_float2(grid_coef(set, n, k), grid_coef(set, n, k + 1));
-    }
+__global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const double* __restrict__ shells) {
     const GridSystem s = systems[blockIdx.y];
     const int nk = (s.nq + kGridChunk - 1) / kGridChunk * kGridChunk;
     const double* lam = shells + s.shell_off;  // [nq] lam_k h in revolutions, then [nq] 1 / D
@@ -370,11 +383,11 @@ int grid_ctas(int grid_points, int ring_frames) {
     return std::min(4, kGridSmem / (grid_points * 128 + kGridWarps * grid_ring_bytes(ring_frames) + 2048));
 }
 
-cudaError_t launch_grid_tables(const GridSystem* systems, int nsys, int max_points, const double* shells, int set,
-                               float2* coef, cudaStream_t st) {
+cudaError_t launch_grid_tables(const GridSystem* systems, int nsys, int max_points, const double* shells,
+                               cudaStream_t st) {
     if (nsys <= 0) return cudaSuccess;
     const int blocks = std::max(1, std::min(64, (max_points + 255) / 256));
-    grid_tables_kernel<<<dim3((unsigned)blocks, (unsigned)nsys), 256, 0, st>>>(systems, shells, set, coef);
+    grid_tables_kernel<<<dim3((unsigned)blocks, (unsigned)nsys), 256, 0, st>>>(systems, shells);
     return cudaGetLastError();
 }
 
@@ -385,11 +398,12 @@ cudaError_t launch_phase_grid(GridLaunch a, int grid_points, int ring_frames, cu
     a.grid_bytes = grid_points * 128;
     a.ring_bytes = grid_ring_bytes(ring_frames);
     const int bytes = a.grid_bytes + kGridWarps * a.ring_bytes;
-    cudaError_t e = cudaFuncSetAttribute(phase_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const auto kernel = a.set ? phase_grid_kernel<1> : phase_grid_kernel<0>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     const long long units = (long long)a.ntiles * 8;
     const unsigned grid = (unsigned)std::min<long long>((long long)current_sms() * ctas, units);
-    phase_grid_kernel<<<grid, kGridWarps * 32, bytes, st>>>(a);
+    kernel<<<grid, kGridWarps * 32, bytes, st>>>(a);
     return cudaGetLastError();
 }
 

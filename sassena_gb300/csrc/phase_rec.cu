@@ -157,8 +157,9 @@ __global__ void __launch_bounds__(kRecWarps * 32, K <= 20 ? 2 : 1) phase_rec_ker
                 for (int b = 0; b < NB; ++b) {
 #pragma unroll 4
                     for (int jj = 0; jj < kRecBlock; ++jj) {
-                        const float4 r = cx[b * kRecBlock + jj];
-                        const float du = fmaf(r.z, uz, fmaf(r.y, uy, __fmul_rn(r.x, ux)));
+                        const float4 xy = cx[b * kRecBlock + (jj & ~1)], zw = cx[b * kRecBlock + (jj | 1)];
+                        const float rx = jj & 1 ? xy.y : xy.x, ry = jj & 1 ? xy.w : xy.z, rz = jj & 1 ? zw.y : zw.x;
+                        const float du = fmaf(rz, uz, fmaf(ry, uy, __fmul_rn(rx, ux)));
                         const float2 dd = make_float2(du, du);
                         // (lam0, dlam) x u.r in revolutions, reduced to [-1/2, 1/2]: n is the
                         // nearest integer of the rounded product, then f = lam u.r - n by FMA
@@ -318,7 +319,7 @@ cudaError_t launch_phase_rec(const RecLaunch& a, cudaStream_t st) {
     return cudaErrorInvalidValue;
 }
 
-// Class-sorted copy of the staged coordinates: dst[f][j] = src[f][map[j]] (w = 1), or
+// Class-sorted copy of the staged coordinates, in pairs: atom j of dst is src[f][map[j]] (w = 1), or
 // the origin (w = 0) where map[j] < 0; a padding atom at the origin contributes exactly
 // 1 to the real part of every shell, which the kernel subtracts by count.
 __global__ void permute_stage_kernel(const float4* __restrict__ src, int na_pad_src, const int* __restrict__ map,
@@ -333,7 +334,7 @@ __global__ void permute_stage_kernel(const float4* __restrict__ src, int na_pad_
             r = src[f * na_pad_src + s];
             r.w = 1.f;
         }
-        dst[i] = r;
+        store_paired(dst + f * na_dst, j, r);
     }
 }
 
