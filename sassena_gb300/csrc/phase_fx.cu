@@ -19,9 +19,11 @@
 //     rounding leaves (below 2^-35) in FP32.
 // Per term the errors add to 1.6e-16 rms (FP32 rounding of the cubic term of sin x and of the low
 // phase words). Amplitudes against 80-bit arithmetic, rms: 300 atoms at q r <= 20 2.8e-14 (FP64
-// kernel 7.6e-14), 2,000 atoms at q r <= 250 7.7e-14 (2.1e-12: FP64 rounds q.r). Measured on a GB300, 3,000 atoms x 250 frames x 12 shells x
-// 60 directions: FP64 kernel 39.9 ms, this one 1.75 ms (3.1e11 terms/s, 32 clocks of an SM per
-// 32 terms), S(q,t) off by 1.9e-15 of its norm (2.6e-15 before).
+// kernel 7.6e-14), 2,000 atoms at q r <= 250 7.7e-14 (2.1e-12: FP64 rounds q.r). Measured on a
+// GB300, 3,000 atoms x 250 frames x 12 shells x 60 directions: FP64 kernel 39.9 ms, this one
+// 1.57 ms (3.4e11 terms/s, 29 clocks of an SM per 32 terms: the FMA pipe, which also takes the
+// integer products, and the issue slots are both near three quarters busy), S(q,t) off by 1.9e-15
+// of its norm (2.6e-15 before).
 //
 // A warp owns 32 q-vectors (any shells: the factor is read per lane) and one frame, and
 // streams the atoms in class order in blocks of 32: the lanes convert one atom each to the
@@ -122,11 +124,11 @@ struct FxSums {
     long long c, s;       // table values, 2^-55
     long long lc, ls;     // upper half of C (S) times the upper bits of d, 2^-65 revolutions
     unsigned gc, gs;      // the rest on the 2^-39 grid (bit patterns of magic sums)
-    float fc, fs;         // what the grid leaves, units of 2^-23
+    float2 f;             // what the grid leaves, units of 2^-23
     __device__ __forceinline__ void clear() {
         c = s = lc = ls = 0;
         gc = gs = 0u;
-        fc = fs = 0.f;
+        f = make_float2(0.f, 0.f);
     }
 };
 
@@ -159,20 +161,19 @@ __device__ __forceinline__ void fx_term(unsigned hi, unsigned lo, float dt, cons
     a.s += (long long)(((unsigned long long)e.w << 32) | e.z);
     a.lc += (long long)chi * sh;
     a.ls += (long long)shi * sh;
-    {   // to subtract from cos: C u + S ys + Sl x
-        const float g1 = fmaf(ch, uh, kFxMagic), r1 = fmaf(ch, uh, __fsub_rn(kFxMagic, g1));
-        const float g2 = fmaf(sn, ys, g1), r2 = fmaf(sn, ys, __fsub_rn(g1, g2));
-        const float g3 = fmaf(sl, xhs, g2), r3 = fmaf(sl, xhs, __fsub_rn(g2, g3));
-        a.gc += __float_as_uint(g3);
-        a.fc = __fadd_rn(a.fc, __fadd_rn(__fadd_rn(fmaf(cl, uhs, fmaf(ch, ul, r1)), r2), r3));
-    }
-    {   // to subtract from sin: S u - C ys - Cl x
-        const float g1 = fmaf(sn, uh, kFxMagic), r1 = fmaf(sn, uh, __fsub_rn(kFxMagic, g1));
-        const float g2 = fmaf(-ch, ys, g1), r2 = fmaf(-ch, ys, __fsub_rn(g1, g2));
-        const float g3 = fmaf(-cl, xhs, g2), r3 = fmaf(-cl, xhs, __fsub_rn(g2, g3));
-        a.gs += __float_as_uint(g3);
-        a.fs = __fadd_rn(a.fs, __fadd_rn(__fadd_rn(fmaf(sl, uhs, fmaf(sn, ul, r1)), r2), r3));
-    }
+    // to subtract from cos: C u + S ys + Sl x; from sin: S u - C ys - Cl x: the halves of paired
+    // instructions (14 for 28; 1.75 -> 1.57 ms with sixteen terms a turn)
+    const float2 A = make_float2(ch, sn), B = make_float2(sn, -ch), D = make_float2(sl, -cl), m1 = make_float2(-1.f, -1.f);
+    const float2 u2 = make_float2(uh, uh), y2 = make_float2(ys, ys), x2 = make_float2(xhs, xhs);
+    const float2 g1 = __ffma2_rn(A, u2, make_float2(kFxMagic, kFxMagic));
+    const float2 r1 = __ffma2_rn(A, u2, __ffma2_rn(g1, m1, make_float2(kFxMagic, kFxMagic)));
+    const float2 g2 = __ffma2_rn(B, y2, g1), r2 = __ffma2_rn(B, y2, __ffma2_rn(g2, m1, g1));
+    const float2 g3 = __ffma2_rn(D, x2, g2), r3 = __ffma2_rn(D, x2, __ffma2_rn(g3, m1, g2));
+    a.gc += __float_as_uint(g3.x);
+    a.gs += __float_as_uint(g3.y);
+    const float2 t = __fadd2_rn(__fadd2_rn(__ffma2_rn(make_float2(cl, sl), make_float2(uhs, uhs),
+                                                      __ffma2_rn(A, make_float2(ul, ul), r1)), r2), r3);
+    a.f = __fadd2_rn(a.f, t);
 }
 
 // The sums of n atoms (npad of them padding: phase 0) in units of 2^-55.
@@ -180,8 +181,8 @@ __device__ __forceinline__ void fx_total(const FxSums& a, int n, int npad, long 
     const long long k2pi = 0x1921fb54442d184ll;  // 2 pi 2^54: 2^-65 revolutions to 2^-55
     const unsigned off = (unsigned)n * __float_as_uint(kFxMagic);
     tc = a.c - ((long long)npad << 55) - __mul64hi(a.ls, k2pi) - ((long long)(int)(a.gc - off) << 16) -
-         __float2ll_rn(a.fc * 4294967296.f);
-    ts = a.s + __mul64hi(a.lc, k2pi) - ((long long)(int)(a.gs - off) << 16) - __float2ll_rn(a.fs * 4294967296.f);
+         __float2ll_rn(a.f.x * 4294967296.f);
+    ts = a.s + __mul64hi(a.lc, k2pi) - ((long long)(int)(a.gs - off) << 16) - __float2ll_rn(a.f.y * 4294967296.f);
 }
 
 __global__ void __launch_bounds__(kFxWarps * 32, 1) phase_fx_kernel(const FxLaunch a) {
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kFxWarps * 32, 1) phase_fx_kernel(const FxLaun
             } else {
                 n += 32;
                 npad += cur >> 16;
-#pragma unroll 2
+#pragma unroll 16
                 for (int jj = 0; jj < 32; ++jj) {
                     const uint4 R = ri[jj];
                     const float4 F = rf[jj];
