@@ -258,8 +258,7 @@ __device__ __forceinline__ long long mp_wide(int a, int b, long long c) {
 }
 // a b / 2^57
 __device__ __forceinline__ long long mp_mul(int2 a, int2 b) {
-    const long long x = (long long)a.x * b.y + (long long)a.y * b.x + (1ll << 27);
-    return 2 * (long long)a.x * b.x + (x >> 28);
+    return 2 * mp_wide(a.x, b.x, 0) + (mp_wide(a.x, b.y, mp_wide(a.y, b.x, 1ll << 27)) >> 28);
 }
 // |v| <= 1 (or rounded above it) in units of 2^-57
 __device__ __forceinline__ int2 mp_unit(double v) {
