@@ -385,7 +385,8 @@ def profile_traffic(kernel, workload):
 def phase_roofline(w, sch, phase_ms, corr_ms, sfu, fma):
     """Roofline of the step's dominant kernel against its live-measured ceiling.
 
-    Coherent: the shell-recurrence kernel (>= 2 FMA + 2 FADD per term on the FP32 pipe) or the
+    Coherent: the gridded kernel (six shared-memory additions per atom, direction and frame, for
+    all shells), the shell-recurrence kernel (>= 2 FMA + 2 FADD per term on the FP32 pipe) or the
     direct kernel (sin + cos per term on the SFU). Incoherent: the fused series + FFT kernel,
     bound by its FP32 FFT work (5 L log2 L flops per series of NF frames) or the SFU."""
     terms = w.terms()
@@ -405,9 +406,19 @@ def phase_roofline(w, sch, phase_ms, corr_ms, sfu, fma):
                 "schedule": sch}
     achieved = terms / (phase_ms * 1e-3)
     rec_only = sch["rec_tiles"] > 0 and sch["direct_tiles"] == 0
-    kernel = "phase_rec_kernel" if rec_only else "phase_sum_kernel"
+    grid = rec_only and sch["rec_shells_per_lane"] == 0  # the schedule counts gridded tiles as such
+    kernel = "phase_grid_kernel" if grid else "phase_rec_kernel" if rec_only else "phase_sum_kernel"
     traffic = profile_traffic(kernel, w.name)
-    if rec_only:
+    if grid:
+        # an SM's shared memory takes one access of 32 lanes a clock, while its FP32 pipe gives
+        # 128 results: 32 atoms x directions x frames per 6 accesses, each good for every shell
+        peak = fma / 128.0 * 32.0 / 6.0 * sch["rec_shells"]
+        roof = {"bound": "shared-memory additions", "peak_source": "measured live: sass_probe_pipes FP32 %.4g "
+                "lane-ops/s / 128 accesses/s, 6 per 32 (atom, direction, frame) of %d shells"
+                % (fma, sch["rec_shells"]),
+                "sfu_results_per_s": sfu,
+                "direct_evaluation_ceiling": sfu / 2.0}
+    elif rec_only:
         # per term at least one FMA per component (recurrence) and one FADD per component
         # (accumulation) on the FP32 pipe: 4 lane operations
         peak = fma / 4.0
@@ -439,24 +450,24 @@ def _cplx(a):
 
 
 def fp64_roofline(w, t64, terms, dev):
-    """The plain FP64 form's phase-sum kernel against the FP64 pipe rate measured live
-    (sass_probe_fp64). Its FP64 pipe instructions per term (products, sums and the
-    software sin/cos) come from the ncu capture in profiles/phase_sum_kernel_fp64_<workload>.json."""
+    """The plain FP64 form's phase-sum kernel (fixed point) against the half of the FP32 pipe that
+    takes integer products and paired instructions, at the rate measured live (sass_probe_pipes).
+    Its instructions there per term come from the ncu capture in profiles/phase_fx_kernel.json."""
     from sassena_gb300 import abi
-    fma = abi.probe_fp64(dev)
-    prof = os.path.join(ROOT, "profiles", "phase_sum_kernel_fp64_%s.json" % w.name)
+    _, fma = abi.probe_pipes(dev)
+    prof = os.path.join(ROOT, "profiles", "phase_fx_kernel.json")
     per_term = None
     if os.path.exists(prof):
         with open(prof) as f:
-            per_term = json.load(f).get("fp64_pipe_inst_per_term")
+            per_term = json.load(f).get("fmaheavy_inst_per_term")
     achieved = terms / (t64["phase_ms"] * 1e-3)
-    roof = {"bound": "fp64", "kernel": "phase_sum_kernel<double>", "kernel_ms": t64["phase_ms"],
-            "fp64_fma_per_s": fma, "achieved": achieved, "unit": "terms/s"}
+    roof = {"bound": "integer products", "kernel": "phase_fx_kernel", "kernel_ms": t64["phase_ms"],
+            "fp32_fma_per_s": fma, "fp64_fma_per_s": abi.probe_fp64(dev), "achieved": achieved, "unit": "terms/s"}
     if per_term:
-        roof.update({"fp64_pipe_inst_per_term": per_term, "peak": fma / per_term,
-                     "frac": achieved * per_term / fma,
-                     "peak_source": "measured live: sass_probe_fp64 %.4g FP64 FMA/s / %.1f FP64-pipe "
-                                    "instructions per term (ncu)" % (fma, per_term)})
+        roof.update({"fmaheavy_inst_per_term": per_term, "peak": fma / 2.0 / per_term,
+                     "frac": achieved * per_term * 2.0 / fma,
+                     "peak_source": "measured live: sass_probe_pipes FP32 %.4g lane-ops/s / 2 / %.1f "
+                                    "instructions per term on that half (ncu)" % (fma, per_term)})
     return roof
 
 
@@ -881,9 +892,11 @@ def run_batched(args, dist):
     t0 = time.perf_counter()
     with abi.Batch(ws[::8], precision="fp32", device=dev, stream=stream.cuda_stream) as sub:
         tuned = sub.autotune(repeats=1)
+        gridded = sub.schedule()["rec_tiles"] > 0 and not tuned["rec_shells_per_lane"]
     tune_s = time.perf_counter() - t0
     t0 = time.perf_counter()
-    rec = tuned["rec_shells_per_lane"] or -1  # the subset's choice: a width, or off
+    # the subset's choice: a recurrence width, the automatic path (gridded), or off
+    rec = tuned["rec_shells_per_lane"] or (0 if gridded else -1)
     b = abi.Batch(ws, precision="fp32", device=dev, stream=stream.cuda_stream)
     b.set_tile(tuned["q_per_lane"], tuned["warps"], tuned["atoms"], tuned["split_atoms"])
     b.set_recurrence(rec)
