@@ -797,8 +797,14 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         int ns = 1;
         if (fx_on_[i]) {
             // a warp tile runs on its own: split until there are about four for each of the
-            // 24 warps of an SM, with at least 4 blocks of 32 atoms in a slice
-            max_split = std::max(1, (int)(items[i].sys->na_rec / 128));
+            // 24 warps of an SM, with at least 4 blocks of 32 atoms in a slice; fewer where even
+            // those leave warps idle, since a warp alone takes about 300 clocks a term (200 atoms,
+            // 50 frames, 48 q-vectors: phase kernel and reduction 61 us with 4 blocks, 41 with 2,
+            // 33 with 1)
+            const size_t nb = items[i].sys->na_rec / 32;
+            size_t least = 4;
+            while (least > 1 && fx_units * (nb / least) < (size_t)sms * 24) least /= 2;
+            max_split = (int)std::max<size_t>(1, nb / least);
             if (cfg.split_atoms > 0) ns = (int)((items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms);
             else ns = (int)std::min<size_t>(64, ((size_t)sms * 96 + fx_units - 1) / std::max<size_t>(fx_units, 1));
         } else if (grid_on[i]) {
