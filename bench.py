@@ -450,18 +450,22 @@ def _cplx(a):
 
 
 def fp64_roofline(w, t64, terms, dev):
-    """The plain FP64 form's phase-sum kernel (fixed point) against the half of the FP32 pipe that
-    takes integer products and paired instructions, at the rate measured live (sass_probe_pipes).
-    Its instructions there per term come from the ncu capture in profiles/phase_fx_kernel.json."""
+    """The plain FP64 form's dominant kernel (fixed point: the phase sum, or the incoherent transforms
+    of padded lengths 64 to 256) against the half of the FP32 pipe that takes integer products and
+    paired instructions, at the rate measured live (sass_probe_pipes). Its instructions there per
+    term come from the ncu capture in profiles/<kernel>.json (for the transforms: of length 256)."""
     from sassena_gb300 import abi
     _, fma = abi.probe_pipes(dev)
-    prof = os.path.join(ROOT, "profiles", "phase_fx_kernel.json")
+    kernel, key = ("self_fx_kernel", "corr_ms") if w.scattering == "self" else ("phase_fx_kernel", "phase_ms")
+    prof = os.path.join(ROOT, "profiles", kernel + ".json")
+    if w.scattering == "self" and not 64 < w.nf <= 128:
+        prof = ""
     per_term = None
     if os.path.exists(prof):
         with open(prof) as f:
             per_term = json.load(f).get("fmaheavy_inst_per_term")
-    achieved = terms / (t64["phase_ms"] * 1e-3)
-    roof = {"bound": "integer products", "kernel": "phase_fx_kernel", "kernel_ms": t64["phase_ms"],
+    achieved = terms / (t64[key] * 1e-3)
+    roof = {"bound": "integer products", "kernel": kernel, "kernel_ms": t64[key],
             "fp32_fma_per_s": fma, "fp64_fma_per_s": abi.probe_fp64(dev), "achieved": achieved, "unit": "terms/s"}
     if per_term:
         roof.update({"fmaheavy_inst_per_term": per_term, "peak": fma / 2.0 / per_term,
@@ -638,7 +642,8 @@ def run_ours(args, dist):
     sch = plan.schedule()
     sfu, fma = abi.probe_pipes(dev)
     if args.precision == "fp64":
-        roof = fp64_roofline(w, {"phase_ms": statistics.median(phase_ms)}, terms, dev)
+        roof = fp64_roofline(w, {"phase_ms": statistics.median(phase_ms), "corr_ms": statistics.median(corr_ms)},
+                             terms, dev)
         roof["schedule"] = sch
     else:
         roof = phase_roofline(w, sch, statistics.median(phase_ms), statistics.median(corr_ms), sfu, fma)
@@ -760,18 +765,19 @@ def run_multipole(args, dist):
 
     fp64 = abi.probe_fp64(dev)
     ph = statistics.median(phase_ms)
-    # algorithmic FP64 work of the moment sums: sphere 2 FMA per term (real j_l b times a
-    # complex Y); cylinder 6 operations per atom, q, frame and order (J cos, J sin, 4 FMA)
+    # the sums over atoms run in integers; what stays in FP64 are the basis functions, at the
+    # least the two operations a step of their recurrences
+    L = args.resolution
     if kind == "sphere":
-        ops = 2.0 * terms
-        per = "2 FMA per term (sum_j b j_l(qr) conj(Y_lm))"
+        ops = 2.0 * w.na * w.nf * ((L + 1) * (L + 2) / 2 + w.nq * (L + 1))
+        per = "2 FP64 operations per atom, frame and (l, m >= 0), and per atom, frame, q and l"
     else:
-        ops = 6.0 * w.na * w.nq * w.nf * (2 * args.resolution + 1)
-        per = "6 FP64 operations per atom, q, frame and order n <= 2L"
+        ops = w.na * w.nf * (2 * L + 1) * (4.0 + 2.0 * w.nq)
+        per = "4 FP64 operations per atom, frame and order n <= 2L, and 2 more per q"
     achieved = ops / (ph * 1e-3)
     roof = {"bound": "fp64", "achieved": achieved, "peak": fp64, "unit": "FP64 op/s",
             "frac": achieved / fp64, "traffic": None,
-            "kernel": "mp_sphere_basis+contract" if kind == "sphere" else "mp_cylinder_kernel",
+            "kernel": "mp_ylm+jl+sphere_sum" if kind == "sphere" else "mp_angle+jn+cylinder_sum",
             "kernel_ms": ph, "peak_source": "measured live: sass_probe_fp64 %.4g FMA/s; "
                                             "algorithmic work %s" % (fp64, per)}
     out = {"metric": MP_METRIC, "value": value, "unit": "terms/s", "n_gpus": dist.world,

@@ -59,8 +59,9 @@ extern "C" {
 #define SASS_METHOD_FFTW 0
 #define SASS_METHOD_DIRECT 1
 
-/* Arithmetic of the phase sum. FP64 reproduces the reference's FP64 sums;
- * FP32 is the fast form (FP32 phase, Kahan, FP64 cross-block reductions). */
+/* Arithmetic of the phase sum. FP64 gives the reference's FP64 sums within 1e-12 (64-bit
+ * fixed point; with a tile shape set by hand the reference's own FP64 operations);
+ * FP32 is the fast form (FP32 phase, exact or compensated sums). */
 #define SASS_PRECISION_FP64 0
 #define SASS_PRECISION_FP32 1
 
@@ -228,17 +229,19 @@ int sass_frame_center(const sass_plan* plan, double* center3);
  * abstract_vectors_scatter_device.cpp:112-130) and consecutive |q| lie on a line (linear
  * scans), runs of at least 3 such shells are evaluated by a kernel that carries
  * exp(i q_k u.r) from shell to shell with a three-term recurrence: two reduced sin/cos
- * pairs per atom for up to `shells_per_lane` shells. 0 = automatic (default), -1 = off,
- * else one of 4, 8, 12, 16, 20, 24, 32. FP64 plans ignore it. */
+ * pairs per atom for up to `shells_per_lane` shells. 0 = automatic (default): the gridded
+ * kernel where the shells share a direction set, at any spacing, and it costs less, else the
+ * recurrence; -1 = off (neither); else one of 4, 8, 12, 16, 20, 24, 32 (the recurrence alone).
+ * FP64 plans ignore it. */
 int sass_set_shell_recurrence(sass_plan* plan, int shells_per_lane);
 
 /* How the last sass_compute (or batch run) scheduled the phase sum. */
 typedef struct sass_schedule {
     double terms;                  /* atom x sub-vector x frame terms */
     uint64_t direct_tiles;         /* tiles of the direct phase-sum kernel */
-    uint64_t rec_tiles;            /* tiles of the shell-recurrence kernel */
-    uint64_t rec_shells;           /* q-vectors evaluated by the recurrence */
-    int rec_shells_per_lane;       /* 0: recurrence not used */
+    uint64_t rec_tiles;            /* tiles of the shell-recurrence or gridded kernel */
+    uint64_t rec_shells;           /* q-vectors evaluated by them */
+    int rec_shells_per_lane;       /* the recurrence's width; 0: not used (rec_tiles > 0: gridded) */
     int q_per_lane, warps, atoms;  /* direct kernel tile shape */
     int atom_splits;               /* largest atom-split count */
     int poly_pairs;                /* direct kernel: q-vector pairs per lane on the FP32 pipe */
@@ -351,7 +354,7 @@ void sass_host_free(void* p);
  * throughput of `device` with pipe microbenchmarks; the phase sum's roofline. */
 int sass_probe_pipes(int device, double* sfu_ops_per_s, double* fp32_fma_per_s);
 /* FP64 FMA rate of the device (independent fma chains over every SM), FMA/s: the
- * ceiling of the FP64 forms and of the multipole devices. */
+ * ceiling of what runs in FP64 (the multipole devices' basis functions, long transforms). */
 int sass_probe_fp64(int device, double* fp64_fma_per_s);
 
 /* Allocation-free coherent autocorrelation + orientational average (FP64), for
