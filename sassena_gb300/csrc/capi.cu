@@ -526,7 +526,9 @@ int sass_compute(sass_plan* p, size_t nq, const size_t* offs, const double* subv
     }
     // batches of whole q-vectors bounded by the amplitude budget (coherent path)
     const size_t budget = p->d.amplitude_budget_bytes ? p->d.amplitude_budget_bytes : ((size_t)4 << 30);
-    const size_t per_sub = nf * sizeof(double2);
+    // (a batch's shells share the gridded sum's pass over the atoms: 4,096 directions x 100 shells x
+    // 2,048 frames took four passes at 16 bytes a value, which FP32 amplitudes do not have)
+    const size_t per_sub = nf * (p->d.precision == SASS_PRECISION_FP32 ? sizeof(float2) : sizeof(double2));
     EngineConfig cfg = engine_config(p->d);
     cfg.shape = p->shape;
     cfg.split_atoms = p->split_atoms;
