@@ -809,14 +809,15 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
             else ns = (int)std::min<size_t>(64, ((size_t)sms * 96 + fx_units - 1) / std::max<size_t>(fx_units, 1));
         } else if (grid_on[i]) {
             // as above, four for each of the CTAs of an SM, with slices of at least 1,024 atoms, since
-            // each pays for its own transform, and at most kGridMaxSlice
+            // each pays for its own transform, and at most kGridMaxSlice; where the partial sums'
+            // memory allows fewer slices than that, they are longer, and above kGridMaxSum a tile
+            // sums several grids one after the other
             const size_t nr = items[i].sys->na_rec;
             max_split = std::max(1, (int)(nr / 128));
             const size_t want = ((size_t)sms * grid_ctas(grid_points_, grid_frames_) * 4 + grid_units - 1) /
                                 std::max<size_t>(grid_units, 1);
-            size_t n = std::min(want, nr / 1024);
-            if (cfg.split_atoms > 0) n = (items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms;
-            ns = (int)std::max(n, (nr + kGridMaxSlice - 1) / kGridMaxSlice);
+            ns = (int)std::max(std::min(want, nr / 1024), (nr + kGridMaxSlice - 1) / kGridMaxSlice);
+            if (cfg.split_atoms > 0) ns = (int)((items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms);
         } else if (cfg.split_atoms > 0) {
             ns = (int)((items[i].sys->na_pad + cfg.split_atoms - 1) / cfg.split_atoms);
         } else if (base_tiles < target) {
@@ -1147,7 +1148,8 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         g.gw = reinterpret_cast<float*>(take((size_t)(g.nclass + 1) * sizeof(float)));
         g.konst = reinterpret_cast<int*>(take(sizeof(int)));
         const long long nb = (long long)(s.na_rec / 32), ns = nsplit_[i];
-        g.slice_atoms = (int)((nb + ns - 1) / ns) * 32;
+        const long long bt = (nb + ns - 1) / ns, grids = (bt * 32 + (long long)kGridMaxSum - 1) / (long long)kGridMaxSum;
+        g.slice_atoms = (int)((bt + grids - 1) / grids) * 32;
         gsys.push_back(g);
         for (const GridLanes& gl : grid_lanes(g.nd))
             for (int f0 = 0; f0 < g.nf; f0 += 256 >> gl.lgd)

@@ -215,7 +215,7 @@ struct GridSystem {
     int na_rec, nf, nd, nclass, nq;
     int G, off;               // grid points; the point of projection 0
     int shell_off;            // of the system's [2][nq] shell constants
-    int slice_atoms;          // most atoms of a tile
+    int slice_atoms;          // most atoms summed in one grid (a multiple of 32)
 };
 
 struct GridTileDesc {
@@ -236,7 +236,11 @@ struct GridLaunch {
 };
 
 constexpr int kGridShellChunk = 8;
-constexpr size_t kGridMaxSlice = 4096;        // atoms per tile: the unit of the integer grid grows with them
+// Atoms of one grid: the unit of its integers grows with them (rounding a weight to 9e-7 of the
+// largest factor at 4,096, to 3.5e-6 at 16,384). Slices are made no longer than the first; the
+// second is the limit (100,000 atoms, 64 frames, 200 x 2,000: 20 slices of 5,000 atoms 31.5 ms,
+// each as two grids 44).
+constexpr size_t kGridMaxSlice = 4096, kGridMaxSum = 16384;
 constexpr double kGridSigma[2] = {3.0, 4.0};  // grid points per half period at the largest shell, per weight set
 // D(l) of the weights `set`; CTAs per SM for that many grid points and staged frames (0: too many)
 double grid_deconvolution(int set, double l);

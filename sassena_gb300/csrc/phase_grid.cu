@@ -23,7 +23,7 @@
 // lanes (FP32 adds are a read and a write, whose latency a warp also waits for between atoms), in
 // any order with the same result, and without the bias that small weights take when they are
 // added to a large FP32 sum. The unit is the largest sum a slice can reach over 2^31, so no cell
-// overflows; a slice of at most 4,096 atoms then rounds each weight to 9e-7 of the largest
+// overflows; a grid of 4,096 atoms rounds each weight to 9e-7 of the largest
 // factor (6e-7 rms in A per atom).
 //
 // Layout. A lane owns one (direction, frame) and a column of the grid in shared memory, [g][lane],
@@ -78,7 +78,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // and, up to the sign, sin: one paired FMA per shell and pair of points on (G_g + G_-g,
 // G_g - G_-g). The transform table streams through `ring` (2 KB) by asynchronous copies of 16
 // points x 8 shells: read straight from L2, its latency took as long as the atoms.
-// `add`: later classes of the same slice add to what the first wrote.
+// `add`: later parts of the same tile add to what the first wrote.
 __device__ __noinline__ void grid_flush(const int* __restrict__ col, float4* __restrict__ ring, int lane, int warp,
                                         const GridSystem& sys, const float* __restrict__ fac, float unit,
                                         float2* __restrict__ dst, bool store, bool add) {
@@ -244,11 +244,11 @@ __global__ void __launch_bounds__(kGridWarps * 32, 4) phase_grid_kernel(const Gr
         };
         for (int b0 = td.b_begin; live && b0 < td.b_end;) {
             // the blocks up to b1 are summed in one grid: one class, or all where the factors
-            // weight the atoms
-            const int cls = __ldg(sys.block_class + b0) & 0xffff;
-            int b1 = td.b_end;
+            // weight the atoms, and at most slice_atoms
+            const int cls = __ldg(sys.block_class + b0) & 0xffff, end = min(td.b_end, b0 + sys.slice_atoms / 32);
+            int b1 = end;
             if (!konst)
-                for (b1 = b0 + 1; b1 < td.b_end && (__ldg(sys.block_class + b1) & 0xffff) == cls;) ++b1;
+                for (b1 = b0 + 1; b1 < end && (__ldg(sys.block_class + b1) & 0xffff) == cls;) ++b1;
             int b = b0 + warp;
             if (b < b1) load(b, 0);
             for (int slot = 0; b < b1; b += kGridWarps, slot ^= 1) {

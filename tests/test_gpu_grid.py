@@ -96,3 +96,18 @@ def test_non_finite_coordinates_take_the_other_kernels(native_lib):
     assert np.isnan(got[:, 3]).all()
     keep = [0, 1, 2, 4, 5]
     assert (np.abs(got[:, keep] - ref[:, keep]) <= 2 * BAR * np.abs(ref).max()).all()
+
+
+@pytest.mark.parametrize("na", [9001, 20000])
+@pytest.mark.parametrize("factors", ["constant", "varying", "wide"])
+def test_long_slices(native_lib, na, factors):
+    # one slice asked for: one grid up to 16,384 atoms, then several, one after the other
+    w = case(na, 3, 18, 20, 77, factors=factors)
+    with abi.Plan(w.na, w.nf, len(w.class_names), "all", "square", precision="fp32") as p:
+        p.stage(w.coords)
+        p.set_classes(w.atom_class)
+        p.set_tile(0, 0, 0, 1)
+        got = p.compute(w.sub_offsets(), w.subvectors(), w.class_factors)
+        assert p.schedule()["rec_tiles"] > 0 and p.schedule()["atom_splits"] == 1
+    ref = oracle.all_vectors(w.coords, w.sub_offsets(), w.subvectors(), w.factors(), 1, 0, nthreads=8)
+    assert rel_err_sqt(got[0], ref[0]).max() <= BAR
