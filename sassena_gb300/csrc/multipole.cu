@@ -1152,16 +1152,16 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
     } else {
         const int N = 2 * L;
         const size_t nn = ns.size();
-        const size_t per_frame = na_pad * (nq * (N + 3) * sizeof(double) + nn * sizeof(int4));
-        const size_t nfb = std::max<size_t>(1, std::min<size_t>({nf, budget / per_frame, (size_t)65535}));  // grid y
-        MCK(p->mp_Jb.ensure(nfb * nq * (N + 3) * na_pad * sizeof(double)));
-        MCK(p->mp_Yc.ensure(nfb * nn * na_pad * sizeof(int4)));
-        MCK(p->mp_ycf.ensure(nfb * nq * (N + 3) * sizeof(unsigned)));
-        const size_t nqc = (nq + kCylQ - 1) / kCylQ, qb = (nq + nqc - 1) / nqc;  // as even as they go
+        // as many q-vectors at a time as the basis of one frame has room for (all, but for very
+        // large systems)
+        const size_t per_q = na_pad * (N + 3) * sizeof(double), angles = na_pad * nn * sizeof(int4);
+        const size_t nqm = std::max<size_t>(1, std::min<size_t>(nq, budget > angles ? (budget - angles) / per_q : 1));
+        const size_t nfb = std::max<size_t>(1, std::min<size_t>({nf, budget / (nqm * per_q + angles), (size_t)65535}));  // grid y
+        MCK(p->mp_Jb.ensure(nfb * nqm * per_q));
+        MCK(p->mp_Yc.ensure(nfb * angles));
+        MCK(p->mp_ycf.ensure(nfb * nqm * (N + 3) * sizeof(unsigned)));
         MpCylinder ca{};
         ca.cyl = s.mp_xyz.as<float4>();
-        ca.cf = d_cf;
-        ca.qcyl = reinterpret_cast<const double*>(dptr(o_qin));
         ca.Jb = p->mp_Jb.as<double>();
         ca.jmax = p->mp_ycf.as<unsigned>();
         ca.Tc = p->mp_Yc.as<int4>();
@@ -1169,22 +1169,28 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
         ca.nmom0 = reinterpret_cast<const int*>(dptr(o_nmom0));
         ca.nout = reinterpret_cast<const int*>(dptr(o_nout));
         ca.mom = reinterpret_cast<const int*>(dptr(o_mom));
-        ca.A = p->mp_amp.as<double2>();
         ca.na_pad = (int)na_pad;
         ca.na = (int)s.na;
         ca.nclass = (int)nclass;
-        ca.nq = (int)nq;
         ca.N = N;
         ca.nn = (int)nn;
         ca.nmom = (int)nmom;
         ca.nf = (int)nf;
-        for (size_t f0 = 0; f0 < nf; f0 += nfb) {
+        const size_t qparts = (nq + nqm - 1) / nqm, fparts = (nf + nfb - 1) / nfb;
+        for (size_t part = 0; part < fparts * qparts; ++part) {
+            const size_t f0 = part / qparts * nfb, q0 = part % qparts * nqm;
+            const size_t nqn = std::min(nqm, nq - q0), nqc = (nqn + kCylQ - 1) / kCylQ;
+            const size_t qb = (nqn + nqc - 1) / nqc;  // as even as they go
             ca.f0 = (int)f0;
             ca.nfb = (int)std::min(nfb, nf - f0);
+            ca.nq = (int)nqn;
+            ca.cf = d_cf + q0 * nclass;
+            ca.qcyl = reinterpret_cast<const double*>(dptr(o_qin)) + 3 * q0;
+            ca.A = p->mp_amp.as<double2>() + q0 * nmom * nf;
             const size_t na2 = (size_t)ca.nfb * na_pad;
             mp_angle_kernel<<<grid_blocks(na2, 128, 64), 128, 0, st>>>(ca);
             MCK(cudaGetLastError());
-            mp_jn_kernel<<<grid_blocks(na2 * nq, 128, 16), 128, 0, st>>>(ca);
+            mp_jn_kernel<<<grid_blocks(na2 * nqn, 128, 16), 128, 0, st>>>(ca);
             MCK(cudaGetLastError());
             MCK(launch_cylinder_sum<kCylQ>(
                 (int)qb, ca, dim3((unsigned)((nn + kSumWarps - 1) / kSumWarps), (unsigned)ca.nfb, (unsigned)nqc), st));
