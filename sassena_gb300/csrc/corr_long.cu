@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kLongNT) long_row_kernel(LongArgs a) {
             buf[i + kLongC / 2] = cmul(csub(u, w), twc[i]);
         }
         __syncthreads();
-        dif_tail<T2, kLongNT>(buf, twc, kLongRowLg, 0);
+        dif_tail4<T2, kLongNT>(buf, twc, kLongRowLg, 0);
         if (MODE == 1) {
             T2* out = reinterpret_cast<T2*>(a.xout) + (size_t)k1 * kLongC;
             for (int i = threadIdx.x; i < kLongC; i += kLongNT) out[i] = cconj(buf[i]);
