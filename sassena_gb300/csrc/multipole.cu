@@ -410,7 +410,6 @@ __device__ void cyl_bessel_row(int N, double x, double* out, size_t stride, cons
 // ---------------------------------------------------------------------------------------
 struct MpSphereBasis {
     const float4* sph;  // [nf][na_pad] (r, phi, theta, class), atoms in order of frame-0 radius
-    const int* cls;     // [na_pad] (-1 padding)
     const double* cf;   // [nq][nclass]
     const double* qlen; // [nq]
     const int* idx;     // [L+1][L+1]: pair (l, m >= 0) or -1
@@ -1107,7 +1106,6 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             const int nb = (int)std::min(nfb, nf - f0);
             MpSphereBasis ba{};
             ba.sph = s.mp_xyz.as<float4>();
-            ba.cls = s.cls.as<int>();
             ba.cf = d_cf;
             ba.qlen = reinterpret_cast<const double*>(dptr(o_qin));
             ba.idx = reinterpret_cast<const int*>(dptr(o_idx));

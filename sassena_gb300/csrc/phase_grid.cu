@@ -22,7 +22,7 @@
 // The grid holds 32-bit integers: shared memory adds integers in place at one access per 32
 // lanes (FP32 adds are a read and a write, whose latency a warp also waits for between atoms), in
 // any order with the same result, and without the bias that small weights take when they are
-// added to a large FP32 sum. The unit is the largest sum a slice can reach over 2^31, so no cell
+// added to a large FP32 sum. The unit is the largest sum a grid can reach over 2^31, so no cell
 // overflows; a grid of 4,096 atoms rounds each weight to 9e-7 of the largest
 // factor (6e-7 rms in A per atom).
 //
