@@ -18,6 +18,8 @@
 //     b_j(q) j_l(|q| r_j) [q x atom] with conj(Y_l^m(j)) [atom x m]. Basis kernels write both
 //     factors for a batch of frames to HBM (every Y_l^m with m >= 0 once, not once per q, in
 //     fixed point); a contraction kernel sums every (q, m) output of one (frame, l) in integers.
+//     Where the amplitudes of a (frame, q) are so small beside the bounds of both factors that the
+//     integers' digits do not reach them, the same sums are taken again in FP64 (MpRedo below).
 //   cylinder: basis kernels write J_n(q_r r) for every order n <= 2L, X = b exp(i s z q_z), and
 //     cos(n phi), sin(n phi) of a batch of frames; a contraction kernel sums X_j J_n cos(n phi_j)
 //     and ... sin(n phi_j) over atoms in integers; each moment is formed from them with
@@ -192,7 +194,7 @@ __device__ void sph_bessel_row(int L, double x, double b, double* out, size_t st
 
 // The normalised associated Legendre functions as P_l^m = g_lm y_lm with
 //   y_lm = al_lm x y_{l-1,m} - y_{l-2,m}, y_mm = P_mm, y_{m+1,m} = x P_mm
-// (two FP64 instructions a step instead of three; the factors g_lm, 0.1 to 2, are applied to the
+// (two FP64 instructions a step instead of three; the factors g_lm, 0.5 to 9, are applied to the
 // sums over atoms): from P_l = a_l (x P_{l-1} - b_l P_{l-2}), a = sqrt((4l^2 - 1)/(l^2 - m^2)),
 // b = sqrt(((l-1)^2 - m^2)/(4 (l-1)^2 - 1)), g_l = a_l b_l g_{l-2} and al_l = a_l g_{l-1} / g_l.
 // Per (l, m) with m <= l, i = (l (l + 1)) / 2 + m: al[i], g[i], and ex[i] with |y_lm| < 2^ex from
@@ -235,15 +237,21 @@ __global__ void ylm_coeff_kernel(int L, MpLegendre t) {
     }
 }
 
-// Fixed-point numbers of the sphere's contraction: v = (h 2^29 + l) 2^(E - 57), |v| < 2^E, l in
-// [-2^28, 2^28).
+// v in units of 2^(E - 58), |v| < 2^E
 __device__ __forceinline__ long long mp_fixed(double v, int E) {
     const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
     const unsigned long long m =
-        ((((unsigned long long)((hi & 0xfffff) | (e ? 0x100000 : 0))) << 32) | (unsigned)__double2loint(v)) << 4;
+        ((((unsigned long long)((hi & 0xfffff) | (e ? 0x100000 : 0))) << 32) | (unsigned)__double2loint(v)) << 5;
     const long long t = (long long)(m >> min(max(E + 1022 - e, 0), 63));
     const long long sg = (long long)(hi >> 31);
     return (t ^ sg) - sg;
+}
+// Fixed-point numbers of the contractions: v = (h 2^29 + l) 2^(E - 57), l in [-2^28, 2^28). Rounded to
+// nearest: cut off, a column of terms of one sign would lose half a unit each.
+__device__ __forceinline__ int2 mp_words(double v, int E) {
+    const long long t = mp_fixed(v, E);
+    const int h = (int)((t + (1ll << 29) + 1) >> 30);
+    return make_int2(h, (int)((unsigned)t + 1u - ((unsigned)h << 30)) >> 1);
 }
 __device__ __forceinline__ int2 mp_split(long long t) {
     const int h = (int)((t + (1ll << 28)) >> 29);
@@ -262,13 +270,15 @@ __device__ __forceinline__ long long mp_mul(int2 a, int2 b) {
 }
 // |v| <= 1 (or rounded above it) in units of 2^-57
 __device__ __forceinline__ int2 mp_unit(double v) {
-    return mp_split(min(max(mp_fixed(v, 1) << 1, -(1ll << 57)), 1ll << 57));
+    return mp_split(min(max(mp_fixed(v, 1), -(1ll << 57)), 1ll << 57));
 }
 
 // conj(Y_l^m(theta, phi)) / g_lm, m >= 0, for the requested pairs (idx[l (L+1) + m] -> pair, or -1)
-// written to out[k * stride] as fixed-point words (re, im); m outer, l inner, so the Legendre
-// recurrence carries two values. e^{i m phi} by rotation (m multiplications of e^{i phi}); its
-// products with the Legendre functions are integers (the FP64 pipe is the bound here).
+// written to out[k * stride] as fixed-point words (re, im) or, with FIXED false, as a double2; m
+// outer, l inner, so the Legendre recurrence carries two values. e^{i m phi} by rotation (m
+// multiplications of e^{i phi}); its products with the Legendre functions are integers (the FP64 pipe
+// is the bound here).
+template <bool FIXED>
 __device__ void conj_ylm_row(int L, double theta, double phi, const int* __restrict__ idx,
                              const MpLegendre& t, int4* out, size_t stride) {
     const double x = cos(theta), s = sqrt((1 - x) * (1 + x));
@@ -287,7 +297,11 @@ __device__ void conj_ylm_row(int L, double theta, double phi, const int* __restr
         auto emit = [&](int l, double P) {
             const int k = idx[l * (L + 1) + m];
             if (k < 0) return;
-            const int2 pi = mp_split(mp_fixed(P, t.ex[l * (l + 1) / 2 + m]));
+            if constexpr (!FIXED) {
+                reinterpret_cast<double2*>(out)[k * stride] = make_double2(P * cm, -P * sm);
+                return;
+            }
+            const int2 pi = mp_words(P, t.ex[l * (l + 1) / 2 + m]);
             const int2 re = mp_split(mp_mul(pi, ci)), im = mp_split(-mp_mul(pi, si));
             out[k * stride] = make_int4(re.x, re.y, im.x, im.y);
         };
@@ -406,6 +420,53 @@ __device__ void cyl_bessel_row(int N, double x, double* out, size_t stride, cons
 }
 
 // ---------------------------------------------------------------------------------------
+// Sums again in FP64
+// ---------------------------------------------------------------------------------------
+// The contractions hold a factor in units of 2^-57 of a bound that is common to all atoms of a frame,
+// so a product is off by about 2^-57 of the product of the two bounds, whatever its own size. That is
+// far below FP64's rounding where the bounds are reached by the same atoms, but not where every product
+// is small beside them: harmonics of high m of atoms near the polar axis (theta^m; a column on the axis,
+// 500 atoms, the moment (12, 12) alone: 5e-6 of S(q, 0)), a class of factor 0 that holds the large
+// Bessel functions, the sine moments of atoms in one half plane. So the amplitudes of each (frame, q),
+// over all the moments asked for, are compared with the error expected of them, and where it is more
+// than 2^-47 of their norm the frame's angular functions are written as FP64 numbers and the sums taken
+// of those. Ordinary calls have none: the test of 64 frames x 10 q x 441 moments takes 12 us and the two
+// empty launches 4 us each. Of a column of 5,000 atoms, the 182 moments of |m| >= 8 (64 frames, 10 q) are
+// all summed again: 1.7 ms without, 3.5 ms so, 5.9 ms with the FP64 sums alone.
+struct MpRedo {
+    unsigned* word;  // [nfb][nq + 1] whether (frame, q) is summed again; last: any q of the frame
+    int nq;
+    __device__ unsigned* at(int fl, int q) const { return word + (size_t)fl * (nq + 1) + q; }
+    __device__ unsigned any(int fl) const { return *at(fl, nq); }
+};
+
+// One warp: the norm of the moments A[k * stride] against their expected error, 2^(e - 57) for each atom of
+// each moment, 2^e the largest product of two rows' bounds (a lane's share of the rows in `e`).
+// Amplitudes that are not finite stay so.
+__device__ __forceinline__ void mp_judge(const MpRedo& r, int fl, int q, int e, const double2* A, size_t stride,
+                                         int nmom, int na) {
+    const int lane = threadIdx.x & 31;
+    double sum2 = 0.0;
+#pragma unroll 8
+    for (int k = lane; k < nmom; k += 32) {
+        const double2 v = A[k * stride];
+        sum2 = fma(v.x, v.x, fma(v.y, v.y, sum2));
+    }
+    for (int o = 16; o; o >>= 1) sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane) return;
+    const double u = scalbn(1.0, e - 57 + 47);
+    const unsigned redo = u * u * nmom * na > sum2;
+    *r.at(fl, q) = redo;
+    if (redo) atomicOr(r.at(fl, r.nq), 1u);
+}
+
+// Exponent of a row whose largest magnitude has the upper half `m`; 4096: not finite.
+__device__ __forceinline__ int mp_exponent(unsigned m) {
+    return m >= 0x7ff00000u ? 4096 : max((int)(m >> 20), 1) - 1022;
+}
+
+// ---------------------------------------------------------------------------------------
 // sphere: basis and contraction
 // ---------------------------------------------------------------------------------------
 struct MpSphereBasis {
@@ -417,13 +478,21 @@ struct MpSphereBasis {
     double* Jb;         // [nfb][nq][L+1][na_pad]  b_j(q) j_l(|q| r_j)
     unsigned* jmax;     // [nfb][nq][L+1] largest |Jb| of the row, its upper half's bits
     int4* Yc;           // [nfb][npair][na_pad]    conj(Y_l^m(j)) / g_lm, m >= 0, in fixed point
+    MpRedo redo;
     int na_pad, nclass, nq, L, npair, f0, nfb;
 };
 
 // conj(Y_l^m) / g_lm of every (frame, atom) of the batch; the tables live in shared memory. Also
-// clears jmax for the kernel that follows.
+// clears jmax and the frames' redo words for the kernels that follow. With FIXED false: FP64 numbers
+// in the same place, of the frames that are summed again.
+template <bool FIXED>
 __global__ void __launch_bounds__(128) mp_ylm_kernel(MpSphereBasis a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    if constexpr (!FIXED) {
+        bool some = false;
+        for (int f = threadIdx.x; f < a.nfb; f += blockDim.x) some = some || a.redo.any(f);
+        if (!__syncthreads_or(some)) return;
+    }
     const MpLegendre from = legendre_at(a.legendre, a.L), t = legendre_at(smem, a.L);
     const int ncf = (a.L + 1) * (a.L + 2) / 2;
     for (int i = threadIdx.x; i < ncf; i += blockDim.x) {
@@ -433,11 +502,17 @@ __global__ void __launch_bounds__(128) mp_ylm_kernel(MpSphereBasis a) {
     for (int i = threadIdx.x; i <= a.L; i += blockDim.x) t.sd[i] = from.sd[i];
     __syncthreads();
     const size_t n = (size_t)a.nfb * a.na_pad, n0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.L + 1); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+    if constexpr (FIXED) {
+        for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.L + 1); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+        for (size_t i = n0; i < (size_t)a.nfb; i += (size_t)gridDim.x * blockDim.x) *a.redo.at((int)i, a.nq) = 0u;
+    }
     for (size_t i = n0; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int fl = (int)(i / a.na_pad), j = (int)(i - (size_t)fl * a.na_pad);
+        if constexpr (!FIXED) {
+            if (!a.redo.any(fl)) continue;
+        }
         const float4 c = a.sph[(size_t)(a.f0 + fl) * a.na_pad + j];
-        conj_ylm_row(a.L, (double)c.z, (double)c.y, a.idx, t, a.Yc + (size_t)fl * a.npair * a.na_pad + j, a.na_pad);
+        conj_ylm_row<FIXED>(a.L, (double)c.z, (double)c.y, a.idx, t, a.Yc + (size_t)fl * a.npair * a.na_pad + j, a.na_pad);
     }
 }
 
@@ -477,9 +552,30 @@ struct MpSphereContract {
     const int* pmom;     // [npair + 1] first entry of each pair in pout
     const int* pout;     // moments of the pairs, 2 moment + (m < 0)
     const int* pm;       // [npair] m of the pair
+    const int* pl;       // [npair] l
     double2* A;          // [nq][nmom][nf]
+    MpRedo redo;
     int na_pad, na, nq, L, nmom, npair, nf, f0;
 };
+
+// The amplitudes of a pair's moments from v = sum_j b_j j_l conj(Y_l^m): times i^l, and for -m
+// (-1)^m times the conjugate (b_j j_l is real).
+__device__ __forceinline__ void mp_sphere_store(const MpSphereContract& a, int pair, int l, int q, int fl, double2 v) {
+    for (int i = a.pmom[pair]; i < a.pmom[pair + 1]; ++i) {
+        const int out = a.pout[i];
+        double2 u = v;
+        if (out & 1) u = (a.pm[pair] & 1) ? make_double2(-v.x, v.y) : make_double2(v.x, -v.y);
+        double2 w;
+        switch (l & 3) {
+            case 0: w = make_double2(u.x, u.y); break;
+            case 1: w = make_double2(-u.y, u.x); break;
+            case 2: w = make_double2(-u.x, -u.y); break;
+            default: w = make_double2(u.y, -u.x); break;
+        }
+        a.A[((size_t)q * a.nmom + (out >> 1)) * a.nf + a.f0 + fl] = w;
+    }
+}
+constexpr double kMp4Pi = 4 * 3.14159265358979323846;
 
 constexpr int kSumWarps = 8, kSumTile = 256;  // atoms of a tile
 static_assert(kSumTile == kSumWarps * 32, "a thread converts one atom of a tile");
@@ -493,8 +589,7 @@ __device__ __forceinline__ void mp_cp_async16(void* dst, const void* src) {
 // integers: the FP64 pipe takes 19 clocks of an SM per warp FMA, a product of 58-bit numbers as
 // three 32 x 32 -> 64-bit multiplications about 1.7 each. J gets the exponent of its row's largest
 // value, Y that of its bound, so that both keep 57 bits below it; the low halves' product, below
-// 2^-58 of the largest, is left out. Only m >= 0 is summed: b_j j_l is real, so the sum for -m is
-// (-1)^m times the conjugate. A lane is an atom, a warp a pair (or, of fewer pairs than warps, a
+// 2^-58 of the largest, is left out; where that is not enough see MpRedo. Only m >= 0 is summed. A lane is an atom, a warp a pair (or, of fewer pairs than warps, a
 // pair and a part of the atoms): Y is read once, straight from memory; the tile's J words are
 // shared. QB x 2 sums of two words each stay in registers; before they could overflow (62-bit
 // products, 56 atoms a lane) they are added over the lanes by 26-bit pieces and go to FP64.
@@ -512,8 +607,7 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_sphere_sum_kernel(MpSphe
     const size_t qstep = (size_t)(a.L + 1) * a.na_pad;
     const int jend = (a.na + 31) & ~31;  // <= na_pad; b_j = 0 past na
     if (threadIdx.x < nqb) {
-        const unsigned mx = a.jmax[((size_t)fl * a.nq + q0 + threadIdx.x) * (a.L + 1) + l];
-        rowe[threadIdx.x] = mx >= 0x7ff00000u ? 4096 : max((int)(mx >> 20), 1) - 1022;  // 4096: not finite
+        rowe[threadIdx.x] = mp_exponent(a.jmax[((size_t)fl * a.nq + q0 + threadIdx.x) * (a.L + 1) + l]);
     }
     auto fetch = [&](int j0) {  // two atoms a thread and row
         for (int i = threadIdx.x; i < nqb * (kSumTile / 2); i += kSumWarps * 32) {
@@ -562,7 +656,7 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_sphere_sum_kernel(MpSphe
 #pragma unroll
         for (int q = 0; q < QB; ++q) {
             int2 w = make_int2(0, 0);
-            if (q < nqb && j0 + (int)threadIdx.x < jend) w = mp_split(mp_fixed(raw[q][threadIdx.x], rowe[q]));
+            if (q < nqb && j0 + (int)threadIdx.x < jend) w = mp_words(raw[q][threadIdx.x], rowe[q]);
             Js[q][threadIdx.x] = w;
         }
         __syncthreads();
@@ -599,8 +693,6 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_sphere_sum_kernel(MpSphe
         if (lane < 2 * QB) part[warp][lane] = total;
     }
     __syncthreads();
-    // times 4 pi i^l
-    const double f4 = 4 * 3.14159265358979323846;
     for (int o = threadIdx.x; o < cnt * nqb; o += kSumWarps * 32) {
         const int q = o / cnt, kk = o - q * cnt, pair = grp.y + kk;
         double2 v = make_double2(0.0, 0.0);
@@ -608,22 +700,53 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_sphere_sum_kernel(MpSphe
             v.x += part[w][2 * q];
             v.y += part[w][2 * q + 1];
         }
-        const double f = rowe[q] == 4096 ? nan("") : f4;
+        const double f = rowe[q] == 4096 ? nan("") : kMp4Pi;
         const MpLegendre lt = legendre_at(a.legendre, a.L);
         const int i0 = l * (l + 1) / 2 + a.pm[pair], e = rowe[q] + lt.ex[i0] - 56;
         v = make_double2(f * lt.g[i0] * scalbn(v.x, e), f * lt.g[i0] * scalbn(v.y, e));
-        for (int i = a.pmom[pair]; i < a.pmom[pair + 1]; ++i) {
-            const int out = a.pout[i];
-            double2 u = v;
-            if (out & 1) u = (a.pm[pair] & 1) ? make_double2(-v.x, v.y) : make_double2(v.x, -v.y);
-            double2 w;
-            switch (l & 3) {
-                case 0: w = make_double2(u.x, u.y); break;
-                case 1: w = make_double2(-u.y, u.x); break;
-                case 2: w = make_double2(-u.x, -u.y); break;
-                default: w = make_double2(u.y, -u.x); break;
+        mp_sphere_store(a, pair, l, q0 + q, fl, v);
+    }
+}
+
+// One warp per (frame, q). 4 pi g_lm times the bound 2^ex is below 2 sqrt(4 pi (2l + 1)).
+__global__ void __launch_bounds__(kSumWarps * 32) mp_sphere_judge_kernel(MpSphereContract a) {
+    const int fl = blockIdx.x;
+    for (int q = blockIdx.y * kSumWarps + (threadIdx.x >> 5); q < a.nq; q += gridDim.y * kSumWarps) {
+        const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q) * (a.L + 1);
+        int e = -4096;
+        for (int k = threadIdx.x & 31; k < a.npair; k += 32) {
+            const int l = a.pl[k];
+            e = max(e, mp_exponent(mx[l]) + 3 + (33 - __clz(2 * l + 1)) / 2);
+        }
+        mp_judge(a.redo, fl, q, e, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
+    }
+}
+
+// The sums of a (frame, q) in FP64, a warp per pair: 2 FMAs an atom, which the FP64 pipe bounds.
+__global__ void __launch_bounds__(kSumWarps * 32) mp_sphere_redo_kernel(MpSphereContract a) {
+    const int fl = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jend = (a.na + 31) & ~31;
+    if (!a.redo.any(fl)) return;
+    const double* g = legendre_at(a.legendre, a.L).g;
+    for (int q = blockIdx.z; q < a.nq; q += gridDim.z) {
+        if (!*a.redo.at(fl, q)) continue;
+        for (int k = blockIdx.x * kSumWarps + warp; k < a.npair; k += gridDim.x * kSumWarps) {
+            const int l = a.pl[k];
+            const double* J = a.Jb + (((size_t)fl * a.nq + q) * (a.L + 1) + l) * a.na_pad;
+            const double2* Y = reinterpret_cast<const double2*>(a.Yc) + ((size_t)fl * a.npair + k) * a.na_pad;
+            double2 v = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int j = lane; j < jend; j += 32) {
+                const double b = J[j];
+                const double2 y = Y[j];
+                v.x = fma(b, y.x, v.x);
+                v.y = fma(b, y.y, v.y);
             }
-            a.A[((size_t)(q0 + q) * a.nmom + (out >> 1)) * a.nf + a.f0 + fl] = w;
+            for (int o = 16; o; o >>= 1) {
+                v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+                v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+            }
+            const double f = kMp4Pi * g[l * (l + 1) / 2 + a.pm[k]];
+            if (lane == 0) mp_sphere_store(a, k, l, q, fl, make_double2(f * v.x, f * v.y));
         }
     }
 }
@@ -653,16 +776,25 @@ struct MpCylinder {
     const int* nout;     // [nmom] the moments of the orders
     const int* mom;      // [nmom][2]
     double2* A;          // [nq][nmom][nf]
+    MpRedo redo;
     int na_pad, na, nclass, nq, N, nn, nmom, nf, f0, nfb;
 };
 
 // cos(n phi), sin(n phi) of every (frame, atom) of the batch by rotation, n ascending. Also clears
-// jmax for the kernel that follows.
+// jmax and the frames' redo words for the kernels that follow. With FIXED false: FP64 numbers in the
+// same place, of the frames that are summed again.
+template <bool FIXED>
 __global__ void __launch_bounds__(128) mp_angle_kernel(MpCylinder a) {
     const size_t n = (size_t)a.nfb * a.na_pad, n0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.N + 3); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+    if constexpr (FIXED) {
+        for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.N + 3); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+        for (size_t i = n0; i < (size_t)a.nfb; i += (size_t)gridDim.x * blockDim.x) *a.redo.at((int)i, a.nq) = 0u;
+    }
     for (size_t i = n0; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int fl = (int)(i / a.na_pad), j = (int)(i - (size_t)fl * a.na_pad);
+        if constexpr (!FIXED) {
+            if (!a.redo.any(fl)) continue;
+        }
         double s1, c1, cp = 1, sp = 0;
         sincos((double)a.cyl[(size_t)(a.f0 + fl) * a.na_pad + j].y, &s1, &c1);
         int4* out = a.Tc + (size_t)fl * a.nn * a.na_pad + j;
@@ -672,8 +804,12 @@ __global__ void __launch_bounds__(128) mp_angle_kernel(MpCylinder a) {
                 sp = sp * c1 + cp * s1;
                 cp = cq;
             }
-            const int2 c = mp_unit(cp), s = mp_unit(sp);
-            out[(size_t)k * a.na_pad] = make_int4(c.x, c.y, s.x, s.y);
+            if constexpr (FIXED) {
+                const int2 c = mp_unit(cp), s = mp_unit(sp);
+                out[(size_t)k * a.na_pad] = make_int4(c.x, c.y, s.x, s.y);
+            } else {
+                reinterpret_cast<double2*>(out)[(size_t)k * a.na_pad] = make_double2(cp, sp);
+            }
         }
     }
 }
@@ -710,6 +846,33 @@ __global__ void __launch_bounds__(128) mp_jn_kernel(MpCylinder a) {
     }
 }
 
+// The amplitudes of an order's moments from C, S = sqrt(2 pi) sum_j X_j J_n(j) (cos, sin)(n phi_j).
+__device__ __forceinline__ void mp_cylinder_store(const MpCylinder& a, int k, int q, int fl, double2 C, double2 S) {
+    const double h2 = 0.70710678118654752440;
+    double snq, cnq;
+    sincos(a.ns[k] * a.qcyl[3 * q + 1], &snq, &cnq);
+    for (int u = a.nmom0[k]; u < a.nmom0[k + 1]; ++u) {
+        const int mk = a.nout[u], l = a.mom[2 * mk], m = a.mom[2 * mk + 1];
+        double2 v;
+        if (l == 0 && m == 0) {
+            v = C;
+        } else {
+            double2 w;  // sum_j X_j J_n cos / sin (n (phi_j - phi_q))
+            if (m == 0 || m == 2) w = make_double2(cnq * C.x + snq * S.x, cnq * C.y + snq * S.y);
+            else w = make_double2(cnq * S.x - snq * C.x, cnq * S.y - snq * C.y);
+            if (m < 2) {
+                const double c = h2 * 2.0 * ((l & 1) ? -1.0 : 1.0);
+                v = make_double2(c * w.x, c * w.y);
+            } else {  // times i sqrt(1/2) 2 (-1)^(l-1)
+                const double c = h2 * 2.0 * (((l - 1) & 1) ? -1.0 : 1.0);
+                v = make_double2(-c * w.y, c * w.x);
+            }
+        }
+        a.A[((size_t)q * a.nmom + mk) * a.nf + a.f0 + fl] = v;
+    }
+}
+constexpr double kMpSqrt2Pi = 2.50662827463100050242;
+
 // sum_j X_j J_n(j) (cos, sin)(n phi_j) of one frame for up to 8 orders n and QB q-vectors, in integers
 // as mp_sphere_sum_kernel sums: a lane is an atom, a warp an order (or a part of one's atoms). The
 // tile's X words are shared; J and the angles are read once, straight from memory. X J is one
@@ -728,11 +891,10 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_cylinder_sum_kernel(MpCy
     const double* rows = a.Jb + ((size_t)fl * a.nq + q0) * qstep;
     const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q0) * (a.N + 3);
     const int jend = (a.na + 31) & ~31;  // <= na_pad; b_j = 0 past na
-    auto exponent = [](unsigned m) { return m >= 0x7ff00000u ? 4096 : max((int)(m >> 20), 1) - 1022; };
     for (int i = threadIdx.x; i < cnt * nqb; i += kSumWarps * 32)
-        jexp[i / nqb][i % nqb] = exponent(mx[(size_t)(i % nqb) * (a.N + 3) + a.ns[k0 + i / nqb]]);
+        jexp[i / nqb][i % nqb] = mp_exponent(mx[(size_t)(i % nqb) * (a.N + 3) + a.ns[k0 + i / nqb]]);
     if (threadIdx.x < nqb)
-        xexp[threadIdx.x] = exponent(max(mx[(size_t)threadIdx.x * (a.N + 3) + a.N + 1],
+        xexp[threadIdx.x] = mp_exponent(max(mx[(size_t)threadIdx.x * (a.N + 3) + a.N + 1],
                                          mx[(size_t)threadIdx.x * (a.N + 3) + a.N + 2]));
     __syncthreads();
     const int aw = cnt > 4 ? 1 : cnt > 2 ? 2 : cnt > 1 ? 4 : 8;
@@ -788,7 +950,7 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_cylinder_sum_kernel(MpCy
             int4 w = make_int4(0, 0, 0, 0);
             if (q < nqb && j < jend) {
                 const double* p = rows + q * qstep + (size_t)(a.N + 1) * a.na_pad + j;
-                const int2 re = mp_split(mp_fixed(p[0], xexp[q])), im = mp_split(mp_fixed(p[a.na_pad], xexp[q]));
+                const int2 re = mp_words(p[0], xexp[q]), im = mp_words(p[a.na_pad], xexp[q]);
                 w = make_int4(re.x, re.y, im.x, im.y);
             }
             Xs[q][threadIdx.x] = w;
@@ -799,7 +961,7 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_cylinder_sum_kernel(MpCy
             const int4 v = tv;
             int2 jw[QB];
 #pragma unroll
-            for (int q = 0; q < QB; ++q) jw[q] = mp_split(mp_fixed(jv[q], je[q]));
+            for (int q = 0; q < QB; ++q) jw[q] = mp_words(jv[q], je[q]);
             load(j0 + c + aw * 32);
 #pragma unroll
             for (int q = 0; q < QB; ++q) {
@@ -832,36 +994,57 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_cylinder_sum_kernel(MpCy
         if (lane < 4 * QB) part[warp][lane] = total;
     }
     __syncthreads();
-    const double norm = sqrt(2 * 3.14159265358979323846), h2 = 0.70710678118654752440;
     for (int i = threadIdx.x; i < cnt * nqb; i += kSumWarps * 32) {
-        const int kk = i / nqb, q = i - kk * nqb, nn = a.ns[k0 + kk];
+        const int kk = i / nqb, q = i - kk * nqb;
         double sum[4] = {0.0, 0.0, 0.0, 0.0};
         for (int w = kk; w < aw * cnt; w += cnt)
             for (int o = 0; o < 4; ++o) sum[o] += part[w][4 * q + o];
         const int e = jexp[kk][q] + xexp[q] - 56;
-        const double f = jexp[kk][q] == 4096 || xexp[q] == 4096 ? nan("") : norm;
-        const double2 C = make_double2(f * scalbn(sum[0], e), f * scalbn(sum[1], e));
-        const double2 S = make_double2(f * scalbn(sum[2], e), f * scalbn(sum[3], e));
-        double snq, cnq;
-        sincos(nn * a.qcyl[3 * (q0 + q) + 1], &snq, &cnq);
-        for (int u = a.nmom0[k0 + kk]; u < a.nmom0[k0 + kk + 1]; ++u) {
-            const int mk = a.nout[u], l = a.mom[2 * mk], m = a.mom[2 * mk + 1];
-            double2 v;
-            if (l == 0 && m == 0) {
-                v = C;
-            } else {
-                double2 w;  // sum_j X_j J_n cos / sin (n (phi_j - phi_q))
-                if (m == 0 || m == 2) w = make_double2(cnq * C.x + snq * S.x, cnq * C.y + snq * S.y);
-                else w = make_double2(cnq * S.x - snq * C.x, cnq * S.y - snq * C.y);
-                if (m < 2) {
-                    const double c = h2 * 2.0 * ((l & 1) ? -1.0 : 1.0);
-                    v = make_double2(c * w.x, c * w.y);
-                } else {  // times i sqrt(1/2) 2 (-1)^(l-1)
-                    const double c = h2 * 2.0 * (((l - 1) & 1) ? -1.0 : 1.0);
-                    v = make_double2(-c * w.y, c * w.x);
-                }
+        const double f = jexp[kk][q] == 4096 || xexp[q] == 4096 ? nan("") : kMpSqrt2Pi;
+        mp_cylinder_store(a, k0 + kk, q0 + q, fl, make_double2(f * scalbn(sum[0], e), f * scalbn(sum[1], e)),
+                          make_double2(f * scalbn(sum[2], e), f * scalbn(sum[3], e)));
+    }
+}
+
+// As mp_sphere_judge_kernel. A moment is 2 sqrt(pi) (cos C' + sin S'): below 2^2 of the sums C', S'.
+__global__ void __launch_bounds__(kSumWarps * 32) mp_cylinder_judge_kernel(MpCylinder a) {
+    const int fl = blockIdx.x;
+    for (int q = blockIdx.y * kSumWarps + (threadIdx.x >> 5); q < a.nq; q += gridDim.y * kSumWarps) {
+        const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q) * (a.N + 3);
+        const int xe = mp_exponent(max(mx[a.N + 1], mx[a.N + 2]));
+        int e = -4096;
+        for (int k = threadIdx.x & 31; k < a.nn; k += 32) e = max(e, mp_exponent(mx[a.ns[k]]) + xe + 2);
+        mp_judge(a.redo, fl, q, e, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
+    }
+}
+
+// As mp_sphere_redo_kernel, a warp per order.
+__global__ void __launch_bounds__(kSumWarps * 32) mp_cylinder_redo_kernel(MpCylinder a) {
+    const int fl = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jend = (a.na + 31) & ~31;
+    if (!a.redo.any(fl)) return;
+    for (int q = blockIdx.z; q < a.nq; q += gridDim.z) {
+        if (!*a.redo.at(fl, q)) continue;
+        const double* rows = a.Jb + ((size_t)fl * a.nq + q) * (a.N + 3) * a.na_pad;
+        const double *xr = rows + (size_t)(a.N + 1) * a.na_pad, *xi = xr + a.na_pad;
+        for (int k = blockIdx.x * kSumWarps + warp; k < a.nn; k += gridDim.x * kSumWarps) {
+            const double* J = rows + (size_t)a.ns[k] * a.na_pad;
+            const double2* T = reinterpret_cast<const double2*>(a.Tc) + ((size_t)fl * a.nn + k) * a.na_pad;
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+            for (int j = lane; j < jend; j += 32) {
+                const double2 t = T[j];
+                const double c = J[j] * t.x, s = J[j] * t.y;
+                v[0] = fma(xr[j], c, v[0]);
+                v[1] = fma(xi[j], c, v[1]);
+                v[2] = fma(xr[j], s, v[2]);
+                v[3] = fma(xi[j], s, v[3]);
             }
-            a.A[((size_t)(q0 + q) * a.nmom + mk) * a.nf + a.f0 + fl] = v;
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+            if (lane == 0)
+                mp_cylinder_store(a, k, q, fl, make_double2(kMpSqrt2Pi * v[0], kMpSqrt2Pi * v[1]),
+                                  make_double2(kMpSqrt2Pi * v[2], kMpSqrt2Pi * v[3]));
         }
     }
 }
@@ -908,6 +1091,14 @@ bool axis_base(const double* axis, MpBase& b) {
 int fail(std::string& m, int code, const std::string& what) {
     m = what;
     return code;
+}
+
+dim3 judge_grid(int nfb, size_t nq) {
+    return dim3((unsigned)nfb, (unsigned)std::min<size_t>((nq + kSumWarps - 1) / kSumWarps, 64));
+}
+dim3 redo_grid(size_t rows, int nfb, size_t nq) {  // few CTAs, since most calls have nothing to do
+    return dim3((unsigned)std::min<size_t>((rows + kSumWarps - 1) / kSumWarps, 4), (unsigned)nfb,
+                (unsigned)std::min<size_t>(nq, 64));
 }
 
 }  // namespace
@@ -976,7 +1167,7 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
     }
     // sphere: the pairs (l, |m|) of the moments, in order of l, each with its moments (2 moment +
     // (m < 0)), and groups of at most 8 pairs of one l
-    std::vector<int> idx((size_t)(L + 1) * (L + 1), -1), pmom, pout, pm;
+    std::vector<int> idx((size_t)(L + 1) * (L + 1), -1), pmom, pout, pm, pl;
     std::vector<int4> groups;
     if (!cyl) {
         std::vector<std::vector<int>> at((size_t)(L + 1) * (L + 1));
@@ -991,6 +1182,7 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
                 if (v.empty()) continue;
                 idx[l * (L + 1) + m] = (int)pm.size();
                 pm.push_back(m);
+                pl.push_back(l);
                 pmom.push_back((int)pout.size());
                 pout.insert(pout.end(), v.begin(), v.end());
             }
@@ -1031,6 +1223,7 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
     const size_t o_pmom = put(pmom.data(), pmom.size() * sizeof(int));
     const size_t o_pout = put(pout.data(), pout.size() * sizeof(int));
     const size_t o_pm = put(pm.data(), pm.size() * sizeof(int));
+    const size_t o_pl = put(pl.data(), pl.size() * sizeof(int));
     const size_t o_ns = put(ns.data(), ns.size() * sizeof(int));
     const size_t o_nmom0 = put(nmom0.data(), nmom0.size() * sizeof(int));
     const size_t o_nout = put(nout.data(), nout.size() * sizeof(int));
@@ -1094,7 +1287,7 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
         const size_t nfb = std::max<size_t>(1, std::min<size_t>({nf, budget / per_frame, (size_t)65535}));  // grid y
         const size_t ysm = legendre_bytes(L);
         const size_t jmax_bytes = nfb * nq * (L + 1) * sizeof(unsigned);
-        MCK(p->mp_ycf.ensure((ysm + 15) / 16 * 16 + jmax_bytes));
+        MCK(p->mp_ycf.ensure((ysm + 15) / 16 * 16 + jmax_bytes + nfb * (nq + 1) * sizeof(unsigned)));
         ylm_coeff_kernel<<<1, 64, 0, st>>>(L, legendre_at(p->mp_ycf.p, L));
         MCK(cudaGetLastError());
         ++launches;
@@ -1111,6 +1304,7 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ba.idx = reinterpret_cast<const int*>(dptr(o_idx));
             ba.legendre = p->mp_ycf.p;
             ba.jmax = reinterpret_cast<unsigned*>(p->mp_ycf.as<unsigned char>() + (ysm + 15) / 16 * 16);
+            ba.redo = MpRedo{ba.jmax + nfb * nq * (L + 1), (int)nq};
             ba.Jb = p->mp_Jb.as<double>();
             ba.Yc = p->mp_Yc.as<int4>();
             ba.na_pad = (int)na_pad;
@@ -1121,7 +1315,7 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ba.f0 = (int)f0;
             ba.nfb = nb;
             const size_t ny = (size_t)nb * na_pad, nj = ny * nq;
-            mp_ylm_kernel<<<grid_blocks(ny, 128, 64), 128, ysm, st>>>(ba);
+            mp_ylm_kernel<true><<<grid_blocks(ny, 128, 64), 128, ysm, st>>>(ba);
             MCK(cudaGetLastError());
             mp_jl_kernel<<<grid_blocks(nj, 128, 16), 128, 0, st>>>(ba);
             MCK(cudaGetLastError());
@@ -1135,6 +1329,8 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ca.pmom = reinterpret_cast<const int*>(dptr(o_pmom));
             ca.pout = reinterpret_cast<const int*>(dptr(o_pout));
             ca.pm = reinterpret_cast<const int*>(dptr(o_pm));
+            ca.pl = reinterpret_cast<const int*>(dptr(o_pl));
+            ca.redo = ba.redo;
             ca.A = p->mp_amp.as<double2>();
             ca.na_pad = (int)na_pad;
             ca.na = (int)s.na;
@@ -1145,7 +1341,14 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ca.nf = (int)nf;
             ca.f0 = (int)f0;
             MCK(launch_sphere_sum<kSumQ>((int)qb, ca, dim3((unsigned)groups.size(), (unsigned)nb, (unsigned)nqc), st));
-            launches += 2;
+            // where the integers' digits do not reach: again in FP64
+            mp_sphere_judge_kernel<<<judge_grid(nb, nq), kSumWarps * 32, 0, st>>>(ca);
+            MCK(cudaGetLastError());
+            mp_ylm_kernel<false><<<grid_blocks(ny, 128, 16), 128, ysm, st>>>(ba);
+            MCK(cudaGetLastError());
+            mp_sphere_redo_kernel<<<redo_grid(npair, nb, nq), kSumWarps * 32, 0, st>>>(ca);
+            MCK(cudaGetLastError());
+            launches += 5;
         }
     } else {
         const int N = 2 * L;
@@ -1157,7 +1360,7 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
         const size_t nfb = std::max<size_t>(1, std::min<size_t>({nf, budget / (nqm * per_q + angles), (size_t)65535}));  // grid y
         MCK(p->mp_Jb.ensure(nfb * nqm * per_q));
         MCK(p->mp_Yc.ensure(nfb * angles));
-        MCK(p->mp_ycf.ensure(nfb * nqm * (N + 3) * sizeof(unsigned)));
+        MCK(p->mp_ycf.ensure(nfb * (nqm * (N + 4) + 1) * sizeof(unsigned)));  // jmax and the redo words
         MpCylinder ca{};
         ca.cyl = s.mp_xyz.as<float4>();
         ca.Jb = p->mp_Jb.as<double>();
@@ -1182,17 +1385,24 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ca.f0 = (int)f0;
             ca.nfb = (int)std::min(nfb, nf - f0);
             ca.nq = (int)nqn;
+            ca.redo = MpRedo{ca.jmax + nfb * nqm * (N + 3), (int)nqn};
             ca.cf = d_cf + q0 * nclass;
             ca.qcyl = reinterpret_cast<const double*>(dptr(o_qin)) + 3 * q0;
             ca.A = p->mp_amp.as<double2>() + q0 * nmom * nf;
             const size_t na2 = (size_t)ca.nfb * na_pad;
-            mp_angle_kernel<<<grid_blocks(na2, 128, 64), 128, 0, st>>>(ca);
+            mp_angle_kernel<true><<<grid_blocks(na2, 128, 64), 128, 0, st>>>(ca);
             MCK(cudaGetLastError());
             mp_jn_kernel<<<grid_blocks(na2 * nqn, 128, 16), 128, 0, st>>>(ca);
             MCK(cudaGetLastError());
             MCK(launch_cylinder_sum<kCylQ>(
                 (int)qb, ca, dim3((unsigned)((nn + kSumWarps - 1) / kSumWarps), (unsigned)ca.nfb, (unsigned)nqc), st));
-            launches += 3;
+            mp_cylinder_judge_kernel<<<judge_grid(ca.nfb, nqn), kSumWarps * 32, 0, st>>>(ca);
+            MCK(cudaGetLastError());
+            mp_angle_kernel<false><<<grid_blocks(na2, 128, 16), 128, 0, st>>>(ca);
+            MCK(cudaGetLastError());
+            mp_cylinder_redo_kernel<<<redo_grid(nn, ca.nfb, nqn), kSumWarps * 32, 0, st>>>(ca);
+            MCK(cudaGetLastError());
+            launches += 6;
         }
     }
     const size_t phase_launches = launches;
