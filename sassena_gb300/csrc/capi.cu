@@ -99,6 +99,7 @@ struct sass_batch {
     std::vector<std::vector<double>> lam;  // product structure per system (empty: none)
     std::vector<int> lam_base;
     std::vector<double> umax;
+    std::vector<char> uniform;
     std::string msg;
     sass_timing timing{};
     cudaEvent_t ev[kEvents] = {};
@@ -296,6 +297,20 @@ int product_of(std::string& m, const double* qv, bool on_device, const std::vect
         h = copy.data();
     }
     detect_product(h, offs, lam, base, umax);
+    return SASS_OK;
+}
+
+// uniform_factors of nq rows of class factors; from the device only where there are classes to tell apart.
+int uniform_of(std::string& m, const SystemState& s, const double* cf, bool on_device, size_t nq, bool& uniform) {
+    std::vector<double> copy;
+    if (on_device) {
+        uniform = false;
+        if (!cf || s.nclass < 2) return SASS_OK;
+        copy.resize(nq * s.nclass);
+        CK(m, cudaMemcpy(copy.data(), cf, copy.size() * sizeof(double), cudaMemcpyDeviceToHost));
+        cf = copy.data();
+    }
+    uniform = uniform_factors(s, cf, nq);
     return SASS_OK;
 }
 
@@ -552,6 +567,9 @@ int sass_compute(sass_plan* p, size_t nq, const size_t* offs, const double* subv
             rc = product_of(p->msg, io_on_device ? d_qv + 3 * offs[i] : subvectors + 3 * offs[i], io_on_device != 0,
                             it.offs, it.lam, it.lam_base, it.umax);
             if (rc) return rc;
+            rc = uniform_of(p->msg, p->sys, io_on_device ? it.lam.empty() ? nullptr : d_cf + nclass * i : class_factors + nclass * i,
+                            io_on_device != 0, j - i, it.uniform);
+            if (rc) return rc;
         }
         it.d_cf = d_cf + nclass * i;
         it.d_fqt = d_fqt + i * nf;
@@ -638,6 +656,7 @@ int sass_autotune(sass_plan* p, size_t nq, const size_t* offs, const double* sub
         rc = product_of(p->msg, subvectors, false, items[0].offs, items[0].lam, items[0].lam_base,
                         items[0].umax);
         if (rc) return rc;
+        items[0].uniform = uniform_factors(p->sys, class_factors, nq);
     }
     TuneChoice best;
     double ms = 0;
@@ -823,6 +842,7 @@ int sass_batch_create(const sass_plan_desc* desc, size_t nsystems, const sass_sy
         if (rc) return rc;
         rc = set_system_classes(*st, s.atom_class, false, b->st, b->msg);
         if (rc) return rc;
+        b->uniform.push_back(!b->lam.back().empty() && uniform_factors(*st, s.class_factors, s.nq));
     }
     CK(b->msg, b->qv.ensure(qv_n * sizeof(double)));
     CK(b->msg, b->cf.ensure(cf_n * sizeof(double)));
@@ -848,6 +868,7 @@ static std::vector<WorkItem> batch_items(sass_batch* b) {
         it.lam = b->lam[i];
         it.lam_base = b->lam_base[i];
         it.umax = b->umax[i];
+        it.uniform = b->uniform[i] != 0;
         it.d_cf = b->cf.as<double>() + b->cf_off[i];
         it.d_fqt = reinterpret_cast<double2*>(b->out.as<double>() + b->fqt_off[i]);
         it.d_fq = reinterpret_cast<double2*>(b->out.as<double>() + b->fq_off[i]);

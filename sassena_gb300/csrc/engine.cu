@@ -330,6 +330,8 @@ int set_system_classes(SystemState& s, const int32_t* cls, bool on_device, cudaS
     ECK(cudaMemcpyAsync(s.cls.p, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     ECK(cudaStreamSynchronize(st));
     s.h_cls.assign(h.begin(), h.begin() + s.na);
+    s.class_atoms.assign(s.nclass, 0);
+    for (int32_t c : s.h_cls) ++s.class_atoms[c];
     s.classes_set = true;
     ++s.class_gen;
     s.rec_map_ok = s.rec_ready = s.rec_valid = false;
@@ -383,6 +385,20 @@ bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vect
     }
     umax = std::sqrt(best);
     return true;
+}
+
+bool uniform_factors(const SystemState& s, const double* cf, size_t nq) {
+    float lo = INFINITY, hi = 0.f;
+    for (size_t c = 0; c < s.nclass; ++c) {
+        const float b0 = (float)cf[c];
+        for (size_t k = 0; k < nq; ++k)
+            if (!((float)cf[k * s.nclass + c] == b0) || std::isinf(b0)) return false;
+        if (s.class_atoms[c] && b0 != 0.f) {
+            lo = std::min(lo, std::fabs(b0));
+            hi = std::max(hi, std::fabs(b0));
+        }
+    }
+    return hi <= 16.f * lo;
 }
 
 std::vector<std::pair<int, int>> arithmetic_runs(const std::vector<double>& lam, int min_len) {
@@ -460,13 +476,31 @@ std::vector<GridLanes> grid_lanes(int nd) {
     return v;
 }
 
+// Slots of the class-sorted copy, as build_rec_map lays it out, and the classes that have atoms.
+size_t class_slots(const SystemState& s, size_t& classes) {
+    size_t n = 0;
+    classes = 0;
+    for (size_t a : s.class_atoms) {
+        n += (a + 31) / 32 * 32;
+        classes += a > 0;
+    }
+    return std::max<size_t>((n + 127) / 128 * 128, 128);
+}
+
 // Items the gridded kernel takes, the weight set, the largest grid and the frames per warp. In
 // clocks of an SM per 32 (atom, direction, frame): the grid costs 12 and its transforms nq G / 1.5
 // per slice, the recurrence 1.18 (K + 5.5) per group of K equally spaced shells, the direct kernel
 // 4.5 per shell (measured on a GB300 at 10,000 atoms). Below 512 atoms the transforms and the
-// grid's clearing outweigh the atoms. Two CTAs per SM still fill three quarters of the issue
+// grid's clearing outweigh the atoms. Two CTAs per SM still fill two thirds of the issue
 // slots; grids that leave one are not taken. The finer weight set (more points) is used where it
 // leaves all four CTAs.
+// Classes: each is padded to 32 atoms, in time (the recurrence's too) and in the copy, which may hold
+// twice the staged slots and the padding of the recurrence's 32 classes, no more. Factors that cannot
+// weight the atoms have a grid, its transforms and its share of the amplitudes for every class: a
+// further 2,000 + nq (G / 1.5 + 130). Of 270 systems (600 to 20,000 atoms, 1 to 40 classes, factors
+// constant or varying with q, 5 to 100 shells, equally spaced or not) the choice so is within 15 % of
+// the faster kernel for 266 and 1.32 times as long at most; without the classes' terms 31 were slower
+// by 12 % to 190 % (600 atoms, 20 classes, 100 shells: gridded 1.45 ms, recurrence 0.50).
 void choose_grid(const std::vector<WorkItem>& items, std::vector<char>& on, int& set, int& points, int& frames) {
     bool any = false;
     set = 1;
@@ -478,18 +512,24 @@ void choose_grid(const std::vector<WorkItem>& items, std::vector<char>& on, int&
             continue;
         const int G = grid_shape(it, 0).G;
         if (G > 4096 || grid_ctas(G, 4) < 2) continue;
+        size_t classes = 0;
+        const size_t slots = class_slots(s, classes);
+        if (slots > 2 * s.na_pad + 32 * kRecMaxClass) continue;
         const int nd = (int)it.offs[1], nq = (int)it.lam.size();
         double lanes = 0;
         for (const GridLanes& g : grid_lanes(nd)) lanes += 1 << g.lgd;
         const double slice = (double)std::min(s.na, kGridMaxSlice);
-        const double grid = ((grid_ctas(G, 4) < 4 ? 15.0 : 12.0) + (double)nq * G / (1.5 * slice)) * lanes / nd;
+        const double pad = (double)slots / (double)s.na, transform = nq * G / 1.5;
+        const double further = it.uniform ? 0.0 : (double)(classes - 1) * (2000.0 + 130.0 * nq + transform);
+        const double base = grid_ctas(G, 4) < 3 ? 18.0 : grid_ctas(G, 4) < 4 ? 15.0 : 12.0;
+        const double grid = (base * pad + transform / slice + further / (double)s.na) * lanes / nd;
         const auto runs = arithmetic_runs(it.lam, 3);
         double other = 4.5 * nq;
         if (s.nclass <= (size_t)kRecMaxClass && !runs.empty()) {
             const int K = choose_rec_k({runs});
             for (const auto& ae : runs) {
                 const int n = ae.second - ae.first, ng = (n + K - 1) / K;
-                other += ng * 1.18 * rec_group_cost(K) * std::ceil(ng * nd / 32.0) * 32.0 / (ng * nd) - 4.5 * n;
+                other += ng * 1.18 * rec_group_cost(K) * pad * std::ceil(ng * nd / 32.0) * 32.0 / (ng * nd) - 4.5 * n;
             }
         }
         if (grid > 0.9 * other) continue;
@@ -620,6 +660,7 @@ static std::vector<uint64_t> prepare_key(const EngineConfig& c, const std::vecto
         for (double l : it.lam) d(l);
         u((uint64_t)(int64_t)it.lam_base);
         d(it.umax);
+        u(it.uniform);
         for (const void* q : {(const void*)it.d_qv, (const void*)it.d_cf, (const void*)it.d_fqt,
                               (const void*)it.d_fq, (const void*)it.d_fq2, (const void*)it.d_wsqrt,
                               (const void*)it.d_fqt_w, (const void*)it.d_fq_w, (const void*)it.d_fq2_w,
@@ -694,10 +735,20 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
     grid_frames_ = 1;
     grid_set_ = 0;
     if (f32 && coherent && cfg.rec_k == 0) choose_grid(items, grid_on, grid_set_, grid_points_, grid_frames_);
+    // an automatic choice whose class-sorted copy finds no memory falls back to the kernel that needs none
+    auto sorted_copy = [&](size_t i, bool& use) {
+        const int rc = ensure_rec_layout(*items[i].sys, err);
+        use = rc == kOk;
+        if (rc != kErrOom || cfg.rec_k > 0) return rc;
+        err.clear();
+        return kOk;
+    };
     for (size_t i = 0; i < items.size(); ++i)
         if (grid_on[i]) {
-            const int rc = ensure_rec_layout(*items[i].sys, err);
+            bool use = false;
+            const int rc = sorted_copy(i, use);
             if (rc) return rc;
+            grid_on[i] = use;
         }
 
     // ---- shell-recurrence groups (FP32 form; shells along one direction set) ---------------------
@@ -726,8 +777,10 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         for (size_t i = 0; rec_k_ && i < items.size(); ++i) {
             if (runs[i].empty()) continue;
             const WorkItem& it = items[i];
-            int rc = ensure_rec_layout(*it.sys, err);
+            bool use = false;
+            const int rc = sorted_copy(i, use);
             if (rc) return rc;
+            if (!use) continue;
             rec_on[i].assign(it.offs.size() - 1, 0);
             item_g0[i] = (int)rgroups.size();
             item_nd[i] = (int)(it.offs[1] - it.offs[0]);

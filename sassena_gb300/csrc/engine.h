@@ -61,6 +61,7 @@ struct SystemState {
     void* prefetch_locked = nullptr;
     // class-sorted copy for the shell-recurrence kernel (built on first use)
     std::vector<int32_t> h_cls;   // [na] classes (host copy)
+    std::vector<size_t> class_atoms;  // [nclass] atoms of each class
     DevBuf xyz_rec, block_class;  // [nf][na_rec] float4 with w; [na_rec / 32] int
     DevBuf rec_map, rec_inv;      // [na_rec] atom of each slot (-1: padding); [na] slot of each atom
     size_t na_rec = 0;
@@ -92,6 +93,7 @@ struct WorkItem {
     std::vector<double> lam;
     int lam_base = -1;
     double umax = 0;  // length of the longest base vector
+    bool uniform = false;          // uniform_factors of d_cf (false also where it is not known)
     const double* d_cf = nullptr;  // [nq][nclass]
     double2* d_fqt = nullptr;      // [nq][nf]
     double2* d_fq = nullptr;       // [nq]
@@ -141,6 +143,9 @@ void drop_prefetch(SystemState& s);
 // `umax` is the length of the longest base vector.
 bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vector<double>& lam, int& base,
                     double& umax);
+// Whether the gridded sum can weight the atoms of `s` by class factors cf [nq][nclass] (host) and so take
+// all classes in one grid: the rule that grid_tables_kernel applies to them on the device.
+bool uniform_factors(const SystemState& s, const double* cf, size_t nq);
 // Maximal runs [a, e) of at least min_len shells whose lam lies on a line within
 // 2.5e-7 of the run's largest |lam| (float-rounded linear scans qualify).
 std::vector<std::pair<int, int>> arithmetic_runs(const std::vector<double>& lam, int min_len);
