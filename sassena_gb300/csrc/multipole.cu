@@ -430,15 +430,21 @@ __device__ void cyl_bessel_row(int N, double x, double* out, size_t stride, cons
 // Bessel functions, the sine moments of atoms in one half plane. So the amplitudes of each (frame, q),
 // over all the moments asked for, are compared with the error expected of them, and where it is more
 // than 2^-47 of their norm the frame's angular functions are written as FP64 numbers and the sums taken
-// of those. Ordinary calls have none: the test of 64 frames x 10 q x 441 moments takes 12 us and the two
-// empty launches 4 us each. Of a column of 5,000 atoms, the 182 moments of |m| >= 8 (64 frames, 10 q) are
-// all summed again: 1.7 ms without, 3.5 ms so, 5.9 ms with the FP64 sums alone.
+// of those. One cluster of kRedoCtas CTAs a frame tests it and, where needed, does both. Ordinary calls have
+// none: 64 frames, 10 q, 441 moments 2.500 ms without the test, 2.504 so (2.53 with the three steps
+// as kernels of their own). Of a column of 5,000 atoms, the 182 moments of |m| >= 8 are all summed again:
+// 1.7 ms without, 4.4 so, 5.9 with FP64 sums alone.
+constexpr int kRedoCtas = 8;
 struct MpRedo {
     unsigned* word;  // [nfb][nq + 1] whether (frame, q) is summed again; last: any q of the frame
     int nq;
     __device__ unsigned* at(int fl, int q) const { return word + (size_t)fl * (nq + 1) + q; }
-    __device__ unsigned any(int fl) const { return *at(fl, nq); }
 };
+
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // One warp: the norm of the moments A[k * stride] against their expected error, 2^(e - 57) for each atom of
 // each moment, 2^e the largest product of two rows' bounds (a lane's share of the rows in `e`).
@@ -482,37 +488,31 @@ struct MpSphereBasis {
     int na_pad, nclass, nq, L, npair, f0, nfb;
 };
 
-// conj(Y_l^m) / g_lm of every (frame, atom) of the batch; the tables live in shared memory. Also
-// clears jmax and the frames' redo words for the kernels that follow. With FIXED false: FP64 numbers
-// in the same place, of the frames that are summed again.
-template <bool FIXED>
-__global__ void __launch_bounds__(128) mp_ylm_kernel(MpSphereBasis a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    if constexpr (!FIXED) {
-        bool some = false;
-        for (int f = threadIdx.x; f < a.nfb; f += blockDim.x) some = some || a.redo.any(f);
-        if (!__syncthreads_or(some)) return;
-    }
-    const MpLegendre from = legendre_at(a.legendre, a.L), t = legendre_at(smem, a.L);
-    const int ncf = (a.L + 1) * (a.L + 2) / 2;
+// The tables of the Legendre functions, in shared memory at `smem`.
+__device__ __forceinline__ MpLegendre mp_tables(void* legendre, int L, void* smem) {
+    const MpLegendre from = legendre_at(legendre, L), t = legendre_at(smem, L);
+    const int ncf = (L + 1) * (L + 2) / 2;
     for (int i = threadIdx.x; i < ncf; i += blockDim.x) {
         t.al[i] = from.al[i];
         t.ex[i] = from.ex[i];
     }
-    for (int i = threadIdx.x; i <= a.L; i += blockDim.x) t.sd[i] = from.sd[i];
+    for (int i = threadIdx.x; i <= L; i += blockDim.x) t.sd[i] = from.sd[i];
     __syncthreads();
+    return t;
+}
+
+// conj(Y_l^m) / g_lm of every (frame, atom) of the batch. Also clears jmax and the frames' redo words for
+// the kernels that follow.
+__global__ void __launch_bounds__(128) mp_ylm_kernel(MpSphereBasis a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const MpLegendre t = mp_tables(a.legendre, a.L, smem);
     const size_t n = (size_t)a.nfb * a.na_pad, n0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if constexpr (FIXED) {
-        for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.L + 1); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
-        for (size_t i = n0; i < (size_t)a.nfb; i += (size_t)gridDim.x * blockDim.x) *a.redo.at((int)i, a.nq) = 0u;
-    }
+    for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.L + 1); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+    for (size_t i = n0; i < (size_t)a.nfb; i += (size_t)gridDim.x * blockDim.x) *a.redo.at((int)i, a.nq) = 0u;
     for (size_t i = n0; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int fl = (int)(i / a.na_pad), j = (int)(i - (size_t)fl * a.na_pad);
-        if constexpr (!FIXED) {
-            if (!a.redo.any(fl)) continue;
-        }
         const float4 c = a.sph[(size_t)(a.f0 + fl) * a.na_pad + j];
-        conj_ylm_row<FIXED>(a.L, (double)c.z, (double)c.y, a.idx, t, a.Yc + (size_t)fl * a.npair * a.na_pad + j, a.na_pad);
+        conj_ylm_row<true>(a.L, (double)c.z, (double)c.y, a.idx, t, a.Yc + (size_t)fl * a.npair * a.na_pad + j, a.na_pad);
     }
 }
 
@@ -544,9 +544,11 @@ __global__ void __launch_bounds__(128) mp_jl_kernel(MpSphereBasis a) {
 }
 
 struct MpSphereContract {
+    const float4* sph;
+    const int* idx;
     const double* Jb;
     const unsigned* jmax;
-    const int4* Yc;
+    int4* Yc;
     void* legendre;
     const int4* groups;  // [ngroups] (l, first pair, pairs (at most 8), 0): pairs of one l, consecutive
     const int* pmom;     // [npair + 1] first entry of each pair in pout
@@ -708,31 +710,40 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_sphere_sum_kernel(MpSphe
     }
 }
 
-// One warp per (frame, q). 4 pi g_lm times the bound 2^ex is below 2 sqrt(4 pi (2l + 1)).
-__global__ void __launch_bounds__(kSumWarps * 32) mp_sphere_judge_kernel(MpSphereContract a) {
-    const int fl = blockIdx.x;
-    for (int q = blockIdx.y * kSumWarps + (threadIdx.x >> 5); q < a.nq; q += gridDim.y * kSumWarps) {
+// A frame's amplitudes against their expected error (4 pi g_lm times the bound 2^ex is below
+// 2 sqrt(4 pi (2l + 1))) and, where they need it, their sums in FP64: the harmonics as FP64 numbers in
+// place of the words, then a warp a pair, 2 FMAs an atom, which the FP64 pipe bounds.
+__global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(kSumWarps * 32) mp_sphere_redo_kernel(MpSphereContract a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int fl = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jend = (a.na + 31) & ~31;
+    const int w0 = blockIdx.x * kSumWarps + warp, wn = kRedoCtas * kSumWarps;
+    for (int q = w0; q < a.nq; q += wn) {
         const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q) * (a.L + 1);
         int e = -4096;
-        for (int k = threadIdx.x & 31; k < a.npair; k += 32) {
+        for (int k = lane; k < a.npair; k += 32) {
             const int l = a.pl[k];
             e = max(e, mp_exponent(mx[l]) + 3 + (33 - __clz(2 * l + 1)) / 2);
         }
         mp_judge(a.redo, fl, q, e, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
     }
-}
-
-// The sums of a (frame, q) in FP64, a warp per pair: 2 FMAs an atom, which the FP64 pipe bounds.
-__global__ void __launch_bounds__(kSumWarps * 32) mp_sphere_redo_kernel(MpSphereContract a) {
-    const int fl = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jend = (a.na + 31) & ~31;
-    if (!a.redo.any(fl)) return;
+    cluster_barrier();
+    if (*reinterpret_cast<volatile unsigned*>(a.redo.at(fl, a.nq)) == 0u) return;  // the same for the whole cluster
+    int4* Yf = a.Yc + (size_t)fl * a.npair * a.na_pad;
+    {
+        const MpLegendre t = mp_tables(a.legendre, a.L, smem);
+        for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < jend; j += kRedoCtas * blockDim.x) {
+            const float4 c = a.sph[(size_t)(a.f0 + fl) * a.na_pad + j];
+            conj_ylm_row<false>(a.L, (double)c.z, (double)c.y, a.idx, t, Yf + j, a.na_pad);
+        }
+    }
+    cluster_barrier();
     const double* g = legendre_at(a.legendre, a.L).g;
-    for (int q = blockIdx.z; q < a.nq; q += gridDim.z) {
+    for (int q = 0; q < a.nq; ++q) {
         if (!*a.redo.at(fl, q)) continue;
-        for (int k = blockIdx.x * kSumWarps + warp; k < a.npair; k += gridDim.x * kSumWarps) {
+        for (int k = w0; k < a.npair; k += wn) {
             const int l = a.pl[k];
             const double* J = a.Jb + (((size_t)fl * a.nq + q) * (a.L + 1) + l) * a.na_pad;
-            const double2* Y = reinterpret_cast<const double2*>(a.Yc) + ((size_t)fl * a.npair + k) * a.na_pad;
+            const double2* Y = reinterpret_cast<const double2*>(Yf) + (size_t)k * a.na_pad;
             double2 v = make_double2(0.0, 0.0);
 #pragma unroll 4
             for (int j = lane; j < jend; j += 32) {
@@ -780,37 +791,36 @@ struct MpCylinder {
     int na_pad, na, nclass, nq, N, nn, nmom, nf, f0, nfb;
 };
 
-// cos(n phi), sin(n phi) of every (frame, atom) of the batch by rotation, n ascending. Also clears
-// jmax and the frames' redo words for the kernels that follow. With FIXED false: FP64 numbers in the
-// same place, of the frames that are summed again.
+// cos(n phi), sin(n phi) of one atom by rotation, n ascending, to out[k * na_pad]: fixed-point words or,
+// with FIXED false, a double2.
 template <bool FIXED>
+__device__ void mp_angle_row(const MpCylinder& a, double phi, int4* out) {
+    double s1, c1, cp = 1, sp = 0;
+    sincos(phi, &s1, &c1);
+    for (int k = 0, at = 0; k < a.nn; ++k) {
+        for (const int order = a.ns[k]; at < order; ++at) {
+            const double cq = cp * c1 - sp * s1;
+            sp = sp * c1 + cp * s1;
+            cp = cq;
+        }
+        if constexpr (FIXED) {
+            const int2 c = mp_unit(cp), s = mp_unit(sp);
+            out[(size_t)k * a.na_pad] = make_int4(c.x, c.y, s.x, s.y);
+        } else {
+            reinterpret_cast<double2*>(out)[(size_t)k * a.na_pad] = make_double2(cp, sp);
+        }
+    }
+}
+
+// The angles of every (frame, atom) of the batch. Also clears jmax and the frames' redo words for the
+// kernels that follow.
 __global__ void __launch_bounds__(128) mp_angle_kernel(MpCylinder a) {
     const size_t n = (size_t)a.nfb * a.na_pad, n0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if constexpr (FIXED) {
-        for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.N + 3); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
-        for (size_t i = n0; i < (size_t)a.nfb; i += (size_t)gridDim.x * blockDim.x) *a.redo.at((int)i, a.nq) = 0u;
-    }
+    for (size_t i = n0; i < (size_t)a.nfb * a.nq * (a.N + 3); i += (size_t)gridDim.x * blockDim.x) a.jmax[i] = 0u;
+    for (size_t i = n0; i < (size_t)a.nfb; i += (size_t)gridDim.x * blockDim.x) *a.redo.at((int)i, a.nq) = 0u;
     for (size_t i = n0; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int fl = (int)(i / a.na_pad), j = (int)(i - (size_t)fl * a.na_pad);
-        if constexpr (!FIXED) {
-            if (!a.redo.any(fl)) continue;
-        }
-        double s1, c1, cp = 1, sp = 0;
-        sincos((double)a.cyl[(size_t)(a.f0 + fl) * a.na_pad + j].y, &s1, &c1);
-        int4* out = a.Tc + (size_t)fl * a.nn * a.na_pad + j;
-        for (int k = 0, at = 0; k < a.nn; ++k) {
-            for (const int order = a.ns[k]; at < order; ++at) {
-                const double cq = cp * c1 - sp * s1;
-                sp = sp * c1 + cp * s1;
-                cp = cq;
-            }
-            if constexpr (FIXED) {
-                const int2 c = mp_unit(cp), s = mp_unit(sp);
-                out[(size_t)k * a.na_pad] = make_int4(c.x, c.y, s.x, s.y);
-            } else {
-                reinterpret_cast<double2*>(out)[(size_t)k * a.na_pad] = make_double2(cp, sp);
-            }
-        }
+        mp_angle_row<true>(a, (double)a.cyl[(size_t)(a.f0 + fl) * a.na_pad + j].y, a.Tc + (size_t)fl * a.nn * a.na_pad + j);
     }
 }
 
@@ -1006,29 +1016,31 @@ __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_cylinder_sum_kernel(MpCy
     }
 }
 
-// As mp_sphere_judge_kernel. A moment is 2 sqrt(pi) (cos C' + sin S'): below 2^2 of the sums C', S'.
-__global__ void __launch_bounds__(kSumWarps * 32) mp_cylinder_judge_kernel(MpCylinder a) {
-    const int fl = blockIdx.x;
-    for (int q = blockIdx.y * kSumWarps + (threadIdx.x >> 5); q < a.nq; q += gridDim.y * kSumWarps) {
+// As mp_sphere_redo_kernel, a warp an order. A moment is 2 sqrt(pi) (cos C' + sin S'): below 2^2 of the
+// sums C', S'.
+__global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(kSumWarps * 32) mp_cylinder_redo_kernel(MpCylinder a) {
+    const int fl = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jend = (a.na + 31) & ~31;
+    const int w0 = blockIdx.x * kSumWarps + warp, wn = kRedoCtas * kSumWarps;
+    for (int q = w0; q < a.nq; q += wn) {
         const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q) * (a.N + 3);
         const int xe = mp_exponent(max(mx[a.N + 1], mx[a.N + 2]));
         int e = -4096;
-        for (int k = threadIdx.x & 31; k < a.nn; k += 32) e = max(e, mp_exponent(mx[a.ns[k]]) + xe + 2);
+        for (int k = lane; k < a.nn; k += 32) e = max(e, mp_exponent(mx[a.ns[k]]) + xe + 2);
         mp_judge(a.redo, fl, q, e, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
     }
-}
-
-// As mp_sphere_redo_kernel, a warp per order.
-__global__ void __launch_bounds__(kSumWarps * 32) mp_cylinder_redo_kernel(MpCylinder a) {
-    const int fl = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jend = (a.na + 31) & ~31;
-    if (!a.redo.any(fl)) return;
-    for (int q = blockIdx.z; q < a.nq; q += gridDim.z) {
+    cluster_barrier();
+    if (*reinterpret_cast<volatile unsigned*>(a.redo.at(fl, a.nq)) == 0u) return;  // the same for the whole cluster
+    int4* Tf = a.Tc + (size_t)fl * a.nn * a.na_pad;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < jend; j += kRedoCtas * blockDim.x)
+        mp_angle_row<false>(a, (double)a.cyl[(size_t)(a.f0 + fl) * a.na_pad + j].y, Tf + j);
+    cluster_barrier();
+    for (int q = 0; q < a.nq; ++q) {
         if (!*a.redo.at(fl, q)) continue;
         const double* rows = a.Jb + ((size_t)fl * a.nq + q) * (a.N + 3) * a.na_pad;
         const double *xr = rows + (size_t)(a.N + 1) * a.na_pad, *xi = xr + a.na_pad;
-        for (int k = blockIdx.x * kSumWarps + warp; k < a.nn; k += gridDim.x * kSumWarps) {
+        for (int k = w0; k < a.nn; k += wn) {
             const double* J = rows + (size_t)a.ns[k] * a.na_pad;
-            const double2* T = reinterpret_cast<const double2*>(a.Tc) + ((size_t)fl * a.nn + k) * a.na_pad;
+            const double2* T = reinterpret_cast<const double2*>(Tf) + (size_t)k * a.na_pad;
             double v[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 4
             for (int j = lane; j < jend; j += 32) {
@@ -1091,14 +1103,6 @@ bool axis_base(const double* axis, MpBase& b) {
 int fail(std::string& m, int code, const std::string& what) {
     m = what;
     return code;
-}
-
-dim3 judge_grid(int nfb, size_t nq) {
-    return dim3((unsigned)nfb, (unsigned)std::min<size_t>((nq + kSumWarps - 1) / kSumWarps, 64));
-}
-dim3 redo_grid(size_t rows, int nfb, size_t nq) {  // few CTAs, since most calls have nothing to do
-    return dim3((unsigned)std::min<size_t>((rows + kSumWarps - 1) / kSumWarps, 4), (unsigned)nfb,
-                (unsigned)std::min<size_t>(nq, 64));
 }
 
 }  // namespace
@@ -1315,12 +1319,14 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ba.f0 = (int)f0;
             ba.nfb = nb;
             const size_t ny = (size_t)nb * na_pad, nj = ny * nq;
-            mp_ylm_kernel<true><<<grid_blocks(ny, 128, 64), 128, ysm, st>>>(ba);
+            mp_ylm_kernel<<<grid_blocks(ny, 128, 64), 128, ysm, st>>>(ba);
             MCK(cudaGetLastError());
             mp_jl_kernel<<<grid_blocks(nj, 128, 16), 128, 0, st>>>(ba);
             MCK(cudaGetLastError());
             ++launches;
             MpSphereContract ca{};
+            ca.sph = ba.sph;
+            ca.idx = ba.idx;
             ca.Jb = p->mp_Jb.as<double>();
             ca.jmax = ba.jmax;
             ca.Yc = p->mp_Yc.as<int4>();
@@ -1342,13 +1348,9 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ca.f0 = (int)f0;
             MCK(launch_sphere_sum<kSumQ>((int)qb, ca, dim3((unsigned)groups.size(), (unsigned)nb, (unsigned)nqc), st));
             // where the integers' digits do not reach: again in FP64
-            mp_sphere_judge_kernel<<<judge_grid(nb, nq), kSumWarps * 32, 0, st>>>(ca);
+            mp_sphere_redo_kernel<<<dim3(kRedoCtas, (unsigned)nb), kSumWarps * 32, ysm, st>>>(ca);
             MCK(cudaGetLastError());
-            mp_ylm_kernel<false><<<grid_blocks(ny, 128, 16), 128, ysm, st>>>(ba);
-            MCK(cudaGetLastError());
-            mp_sphere_redo_kernel<<<redo_grid(npair, nb, nq), kSumWarps * 32, 0, st>>>(ca);
-            MCK(cudaGetLastError());
-            launches += 5;
+            launches += 3;
         }
     } else {
         const int N = 2 * L;
@@ -1390,19 +1392,15 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
             ca.qcyl = reinterpret_cast<const double*>(dptr(o_qin)) + 3 * q0;
             ca.A = p->mp_amp.as<double2>() + q0 * nmom * nf;
             const size_t na2 = (size_t)ca.nfb * na_pad;
-            mp_angle_kernel<true><<<grid_blocks(na2, 128, 64), 128, 0, st>>>(ca);
+            mp_angle_kernel<<<grid_blocks(na2, 128, 64), 128, 0, st>>>(ca);
             MCK(cudaGetLastError());
             mp_jn_kernel<<<grid_blocks(na2 * nqn, 128, 16), 128, 0, st>>>(ca);
             MCK(cudaGetLastError());
             MCK(launch_cylinder_sum<kCylQ>(
                 (int)qb, ca, dim3((unsigned)((nn + kSumWarps - 1) / kSumWarps), (unsigned)ca.nfb, (unsigned)nqc), st));
-            mp_cylinder_judge_kernel<<<judge_grid(ca.nfb, nqn), kSumWarps * 32, 0, st>>>(ca);
+            mp_cylinder_redo_kernel<<<dim3(kRedoCtas, (unsigned)ca.nfb), kSumWarps * 32, 0, st>>>(ca);
             MCK(cudaGetLastError());
-            mp_angle_kernel<false><<<grid_blocks(na2, 128, 16), 128, 0, st>>>(ca);
-            MCK(cudaGetLastError());
-            mp_cylinder_redo_kernel<<<redo_grid(nn, ca.nfb, nqn), kSumWarps * 32, 0, st>>>(ca);
-            MCK(cudaGetLastError());
-            launches += 6;
+            launches += 4;
         }
     }
     const size_t phase_launches = launches;
