@@ -189,6 +189,7 @@ int init_system(std::string& m, SystemState& s, const sass_plan_desc& d, int lg,
     s.nclass = d.nclass;
     s.na_pad = ((d.na + kAtomGranule - 1) / kAtomGranule) * kAtomGranule;
     s.lg = lg;
+    s.extent = d.precision == SASS_PRECISION_FP32 && d.scattering == SASS_SCATTERING_ALL;
     return build_system_tables(s, st, m);
 }
 

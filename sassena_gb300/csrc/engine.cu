@@ -234,8 +234,7 @@ int stage_system(SystemState& s, const float* coords, bool on_device, int precis
         }
     }
     memcpy(s.center, c, sizeof(c));
-    const bool bounded = precision == PREC_FP32;  // the gridded phase sum needs the extent
-    if (bounded) {
+    if (s.extent) {  // the gridded phase sum needs it
         ECK(s.rmax_word.ensure(sizeof(unsigned)));
         ECK(cudaMemsetAsync(s.rmax_word.p, 0, sizeof(unsigned), st));
     }
@@ -243,12 +242,12 @@ int stage_system(SystemState& s, const float* coords, bool on_device, int precis
     const bool rec = s.rec_ready && s.rec_map_ok;
     ECK(launch_stage(src, (int)s.nf, (int)s.na, (int)s.na_pad, c[0], c[1], c[2], precision == PREC_FP32,
                      s.xyz.as<float4>(), rec ? s.rec_inv.as<int>() : nullptr, (int)s.na_rec,
-                     rec ? s.xyz_rec.as<float4>() : nullptr, bounded ? s.rmax_word.as<unsigned>() : nullptr, st));
+                     rec ? s.xyz_rec.as<float4>() : nullptr, s.extent ? s.rmax_word.as<unsigned>() : nullptr, st));
     s.rmax = 0;
-    if (bounded) {
-        float r2 = 0.f;
-        ECK(cudaMemcpyAsync(&r2, s.rmax_word.p, sizeof(r2), cudaMemcpyDeviceToHost, st));
-        ECK(cudaStreamSynchronize(st));
+    float r2 = 0.f;
+    if (s.extent) ECK(cudaMemcpyAsync(&r2, s.rmax_word.p, sizeof(r2), cudaMemcpyDeviceToHost, st));
+    ECK(cudaStreamSynchronize(st));
+    if (s.extent) {
         // rounded up to 6 significant bits (and FP32's rounding of r^2), so that descriptors built
         // for one staging mostly fit the next
         int e = 0;
@@ -256,7 +255,6 @@ int stage_system(SystemState& s, const float* coords, bool on_device, int precis
         s.rmax = r2 > 0 ? std::ldexp(std::ceil(m * 64.0) / 64.0, e) : (r2 == 0 ? 1e-30 : INFINITY);
         if (!std::isfinite((double)r2)) s.rmax = INFINITY;
     }
-    ECK(cudaStreamSynchronize(st));
     s.staged = true;
     s.rec_valid = rec;
     s.mp_valid = false;

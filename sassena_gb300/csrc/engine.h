@@ -45,8 +45,9 @@ struct SystemState {
     size_t na = 0, nf = 0, na_pad = 0, nclass = 0;
     int lg = 0;  // padded FFT length 2^lg >= 2 nf
     double center[3] = {0, 0, 0};
-    // FP32 form: bound on |r| of the staged frames (rounded up to 6 bits; 0: not known, infinite:
-    // some coordinate is not finite)
+    // coherent FP32 form (`extent`): bound on |r| of the staged frames (rounded up to 6 bits; 0: not
+    // known, infinite: some coordinate is not finite)
+    bool extent = false;
     double rmax = 0;
     DevBuf rmax_word;
     DevBuf raw, xyz, cls, tw64, tw32, k64, k32;
