@@ -387,6 +387,7 @@ bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vect
 
 bool uniform_factors(const SystemState& s, const double* cf, size_t nq) {
     float lo = INFINITY, hi = 0.f;
+    double sum = 0;
     for (size_t c = 0; c < s.nclass; ++c) {
         const float b0 = (float)cf[c];
         for (size_t k = 0; k < nq; ++k)
@@ -394,9 +395,10 @@ bool uniform_factors(const SystemState& s, const double* cf, size_t nq) {
         if (s.class_atoms[c] && b0 != 0.f) {
             lo = std::min(lo, std::fabs(b0));
             hi = std::max(hi, std::fabs(b0));
+            sum += (double)s.class_atoms[c] * b0 * b0;
         }
     }
-    return hi <= 16.f * lo;
+    return hi <= 16.f * lo && (double)hi * hi * (double)s.na <= 16.0 * sum;
 }
 
 std::vector<std::pair<int, int>> arithmetic_runs(const std::vector<double>& lam, int min_len) {
@@ -1198,6 +1200,7 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         g.nq = (int)it.lam.size();
         g.G = gs.G;
         g.off = gs.off;
+        g.one_grid = it.uniform || s.nclass < 2;
         g.shell_off = (int)gshells.size();
         for (double l : it.lam) gshells.push_back(l * gs.h * 0.15915494309189533577);
         for (double l : it.lam) gshells.push_back(1.0 / grid_deconvolution(grid_set_, l * gs.h));

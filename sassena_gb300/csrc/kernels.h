@@ -214,6 +214,7 @@ struct GridSystem {
     int* konst;
     int na_rec, nf, nd, nclass, nq;
     int G, off;               // grid points; the point of projection 0
+    int one_grid;             // the class factors may weight the atoms (uniform_factors)
     int shell_off;            // of the system's [2][nq] shell constants
     int slice_atoms;          // most atoms summed in one grid (a multiple of 32)
 };

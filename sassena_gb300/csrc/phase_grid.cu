@@ -279,10 +279,10 @@ __global__ void __launch_bounds__(kGridWarps * 32, 4) phase_grid_kernel(const Gr
     }
 }
 
-// Per system: the transform table exp(i lam_k h g) / D, whether the class factors can weight the
-// atoms (then a slice is summed once): the same at all shells, finite, and within 16 of each other
-// so that no atom is lost in the grid's units; the atoms' weights per class in those units, the
-// unit itself (gw[nclass]) and the factors per class and shell.
+// Per system: the transform table exp(i lam_k h g) / D, whether the class factors weight the atoms
+// (then a slice is summed once), as uniform_factors decides on the host, and the same at all shells
+// and finite (one class: its factor is read here alone); the atoms' weights per class in grid
+// units, the unit itself (gw[nclass]) and the factors per class and shell.
 __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const double* __restrict__ shells) {
     const GridSystem s = systems[blockIdx.y];
     const int nk = (s.nq + kGridChunk - 1) / kGridChunk * kGridChunk;
@@ -304,10 +304,9 @@ __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const
     }
     if (blockIdx.x == 0) {
         __shared__ int differs;
-        __shared__ unsigned lo, hi;  // smallest and largest |factor| of the atoms' classes, as bits
+        __shared__ unsigned hi;  // largest |factor| of the atoms' classes, as bits
         if (threadIdx.x == 0) {
             differs = 0;
-            lo = 0x7f800000u;
             hi = 0u;
         }
         __syncthreads();
@@ -319,14 +318,11 @@ __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const
         }
         for (int i = threadIdx.x; i < s.na_rec / 32; i += blockDim.x) {
             const unsigned b = __float_as_uint(fabsf((float)s.cf[s.block_class[i] & 0xffff]));
-            if (b) {
-                atomicMin(&lo, b);
-                atomicMax(&hi, b);
-            }
+            if (b) atomicMax(&hi, b);
         }
         __syncthreads();
         const float bmax = hi ? __uint_as_float(hi) : 1.f;
-        const int konst = !differs && (!hi || bmax <= 16.f * __uint_as_float(lo));
+        const int konst = s.one_grid && !differs;
         // units per weight of 1: no sum of slice_atoms atoms reaches 2^31, no weight 2^22
         // times a power of two, so that the factors' products with it are exact: a rounding of
         // the scale is common to all atoms and counts four times in fq2

@@ -10,7 +10,7 @@ import torch
 import oracle
 from sassena_gb300 import abi
 
-from helpers import rel_err_sqt
+from helpers import cplx, rel_err_sqt
 from test_gpu_grid import BAR, case
 
 pytestmark = pytest.mark.gpu
@@ -100,3 +100,18 @@ def test_no_memory_for_the_sorted_copy(native_lib, shells):
             del hold
             torch.cuda.empty_cache()
         assert (got == ref).all()
+
+
+def test_one_large_factor(native_lib):
+    # One atom of 16 among 4,000 of 1. A weight is rounded to 9e-7 of the largest factor of its grid: by
+    # class, an amplitude is off by 1.35e-6 of its norm (and by 1e-6 for FP32's phases), of which S(q) takes
+    # 2 / sqrt(2) / sqrt(20 directions) = 5.3e-7 rms; in one grid the former is up to 16 times that.
+    w = system(4001, 20, 18, 20, 2, "random")
+    cls = np.zeros(w.na, dtype=np.int32)
+    cls[77] = 1
+    w = dataclasses.replace(w, atom_class=cls, class_factors=np.tile([1.0, 16.0], (w.nq, 1)))
+    sch = {}
+    got = abi.compute_workload(w, "fp32", schedule=sch)[0]
+    assert kernel(sch) == "gridded"
+    ref = cplx(reference(w))
+    assert np.sqrt(np.mean(np.abs(got / ref - 1) ** 2)) <= 1e-6
