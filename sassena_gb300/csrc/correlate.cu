@@ -573,6 +573,53 @@ __device__ __noinline__ void tail_lags(const FinalLaunch& a, const FinalEntry& e
     }
 }
 
+// The same in FP64: the transforms' rounding, 3e-16 of S(q, 0) at the first lags, is 5e-14 to 8e-14 at the
+// last of 250 frames, and with the phases in fixed point it was most of a row's error (3,000 atoms, 12
+// shells x 60 directions against 80-bit arithmetic: 2.0e-15 of the rows' norm, 4.5e-16 so; the FP64 phase
+// sum 1.3e-15). The FP64 pipe bounds it, so lags k and 7 - k of a shell have a CTA, of nine products a
+// series (all eight in one CTA: 25 us more than the spectrum's, 60 directions).
+constexpr int kTailCtas = kTailLags / 2;
+__device__ __noinline__ void tail_lags64(const FinalLaunch& a, const FinalEntry& e, const TailEntry& t, int pair, int nt) {
+    const int lag[2] = {pair, kTailLags - 1 - pair};  // lag nf - 1 - k
+    double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    int bad = 0;
+    for (int s = e.slot_begin + (int)threadIdx.x; s < e.slot_end; s += nt)
+        bad |= !isfinite(a.apart[s].x) || !isfinite(a.apart[s].y);
+    for (size_t v = threadIdx.x; v < t.nv; v += nt) {
+        const double2* x = t.A64 + v * e.nf;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const double2* y = x + e.nf - 1 - lag[h];
+            double2 z = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int i = 0; i <= lag[h]; ++i) {
+                const double2 p = x[i], q = y[i];
+                z.x = fma(q.x, p.x, fma(q.y, p.y, z.x));
+                z.y = fma(q.y, p.x, fma(-q.x, p.y, z.y));
+            }
+            acc[h] = cadd(acc[h], z);
+        }
+    }
+    bad = __syncthreads_or(bad);
+    __shared__ double2 part[32][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        for (int o = 16; o; o >>= 1) {
+            acc[h].x += __shfl_down_sync(0xffffffffu, acc[h].x, o);
+            acc[h].y += __shfl_down_sync(0xffffffffu, acc[h].y, o);
+        }
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][h] = acc[h];
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const int k = threadIdx.x ? lag[1] : lag[0];
+        double2 z = part[0][threadIdx.x];
+        for (int w = 1; w < nt / 32; ++w) z = cadd(z, part[w][threadIdx.x]);
+        const double f = (bad ? nan("") : 1.0) * e.inv_nm / (double)(k + 1);
+        e.fqt[e.nf - 1 - k] = make_double2(z.x * f, (a.conj_out ? -z.y : z.y) * f);
+    }
+}
+
 // fq and fq2 of a shell from its slots' partials, by one warp (by one thread, after the spectrum's
 // transform, 112 slots took half of the kernel: 48 -> 22 us for 10 shells of 256 bins).
 __device__ void mean_sums(const FinalLaunch& a, const FinalEntry& e) {
@@ -594,15 +641,20 @@ __device__ void mean_sums(const FinalLaunch& a, const FinalEntry& e) {
     }
 }
 
-// Two CTAs per shell: its spectrum or series, and beside it the means and the last lags.
+// Two CTAs per shell: its spectrum or series, and beside it the means and the last lags (with FP64 tails
+// two lags, and further CTAs for the others).
 template <int NT>
 __global__ void __launch_bounds__(NT) finalize_kernel(FinalLaunch a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const FinalEntry e = a.entries[blockIdx.x % a.nentries];
-    const TailEntry tail = a.tails ? a.tails[blockIdx.x % a.nentries] : TailEntry{nullptr, 0};
+    const TailEntry tail = a.tails ? a.tails[blockIdx.x % a.nentries] : TailEntry{nullptr, nullptr, 0};
     if (blockIdx.x >= a.nentries) {
-        if (threadIdx.x < 32) mean_sums(a, e);
-        if (tail.A) tail_lags(a, e, tail, NT);
+        const int role = (int)blockIdx.x / a.nentries - 1;
+        if (role == 0) {
+            if (threadIdx.x < 32) mean_sums(a, e);
+            if (tail.A) tail_lags(a, e, tail, NT);
+        }
+        if (tail.A64) tail_lags64(a, e, tail, role, NT);
         return;
     }
     const int nf = e.nf, ns = e.slot_end - e.slot_begin;
@@ -632,7 +684,7 @@ __global__ void __launch_bounds__(NT) finalize_kernel(FinalLaunch a) {
         }
         __syncthreads();
         dit_inverse<NT>(buf, a.tw, e.lg, a.lg_max - e.lg);
-        for (int t = threadIdx.x; t < nf - (tail.A ? kTailLags : 0); t += NT) {
+        for (int t = threadIdx.x; t < nf - (tail.A || tail.A64 ? kTailLags : 0); t += NT) {
             double f = (1.0 / ((double)L * (double)(nf - t))) * e.inv_nm;
             e.fqt[t] = make_double2(buf[t].x * f, sgn * buf[t].y * f);
         }
@@ -1975,7 +2027,7 @@ cudaError_t launch_finalize(const FinalLaunch& a, cudaStream_t st) {
     auto k = finalize_kernel<NT>;
     cudaError_t e = set_smem(k, sm);
     if (e != cudaSuccess) return e;
-    k<<<2 * a.nentries, NT, sm, st>>>(a);
+    k<<<(a.tails && a.tails64 ? 1 + kTailCtas : 2) * a.nentries, NT, sm, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -1298,8 +1298,9 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
             e.f32pair = corr_writes_f32_pairs(cfg.precision, cfg.dsp, lg_max_) ? 1 : 0;
             // from 128 frames on: below, the transforms' rounding stays under FP32's own
             TailEntry tail{};
-            if (f32 && coherent && autoc && s.nf >= 128) {
-                tail.A = static_cast<const float2*>(item_amp_[i]) + it.offs[sh] * s.nf;
+            if (coherent && autoc && s.nf >= 128) {
+                if (f32) tail.A = static_cast<const float2*>(item_amp_[i]) + it.offs[sh] * s.nf;
+                else tail.A64 = static_cast<const double2*>(item_amp_[i]) + it.offs[sh] * s.nf;
                 tail.nv = it.offs[sh + 1] - it.offs[sh];
                 tails_ = true;
             }
@@ -1667,6 +1668,7 @@ int Engine::enqueue(cudaStream_t st, std::string& err, cudaEvent_t* ev) {
     fl.entries = d_entries_;
     fl.nentries = nentries_;
     fl.tails = d_tails_;
+    fl.tails64 = !f32;
     fl.lg_max = lg_max_;
     fl.ppart = ppart_.as<double>();
     fl.apart = apart_.as<double2>();

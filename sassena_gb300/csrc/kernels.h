@@ -320,11 +320,12 @@ struct FinalEntry {
     double2* fq2;
 };
 
-// FP32 form: the series [nv][nf] of a shell whose last kTailLags lags are summed directly
-// (A nullptr: they come from the transforms like the others).
+// The series [nv][nf] of a shell whose last kTailLags lags are summed directly (A and A64 nullptr: they
+// come from the transforms like the others).
 constexpr int kTailLags = 8;
 struct TailEntry {
     const float2* A;
+    const double2* A64;  // FP64 form
     size_t nv;
 };
 
@@ -338,6 +339,7 @@ struct FinalLaunch {
     const double* a2part;
     const double2* tw;         // [L_max/2] FP64
     const TailEntry* tails;    // one per entry, or nullptr: none
+    int tails64;               // whether they are FP64 series
 };
 cudaError_t launch_finalize(const FinalLaunch& a, cudaStream_t st);
 
