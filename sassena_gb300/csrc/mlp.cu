@@ -91,12 +91,12 @@ __device__ __forceinline__ void mma_block(float (&d)[4], const __nv_bfloat16* A,
     }
 }
 
-__device__ void load_weights(Smem& s, const __nv_bfloat16* __restrict__ w, bool transposed) {
+__device__ void load_weights(Smem& s, const __nv_bfloat16* __restrict__ w) {
     for (int i = threadIdx.x; i < H * 4; i += NT) s.w1[i] = bf(w, OW1 + i);
     for (int i = threadIdx.x; i < H * H; i += NT) {
         const int r = i / H, c = i % H;
         s.w2[r * HP + c] = w[OW2 + i];
-        if (transposed) s.w2t[c * HP + r] = w[OW2 + i];
+        s.w2t[c * HP + r] = w[OW2 + i];
     }
     for (int i = threadIdx.x; i < H; i += NT) {
         s.b1[i] = bf(w, OB1 + i);
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(NT) mlp_train_kernel(const __nv_bfloat16* __re
                                                        double* __restrict__ lpart) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-    load_weights(s, w, true);
+    load_weights(s, w);
     const int j = threadIdx.x, warp = j >> 5, lane = j & 31, g = lane >> 2, t = lane & 3;
     float gw1[4] = {0, 0, 0, 0}, gb1 = 0, gb2 = 0, gw3 = 0, gb3 = 0;
     float gw2[2][16][4];  // dW2 rows 32 warp + 16 mt + (g, g + 8), columns 8 nt + 2t (+1)
