@@ -237,8 +237,8 @@ struct GridLaunch {
 };
 
 constexpr int kGridShellChunk = 8;
-// Atoms of one grid: the unit of its integers grows with them (rounding a weight to 9e-7 of the
-// largest factor at 4,096, to 3.5e-6 at 16,384). Slices are made no longer than the first; the
+// Atoms of one grid: the unit of its integers grows with them (rounding a weight to at most 1.1e-6 of
+// the largest factor at 4,096, to 4.4e-6 at 16,384). Slices are made no longer than the first; the
 // second is the limit (100,000 atoms, 64 frames, 200 x 2,000: 20 slices of 5,000 atoms 31.5 ms,
 // each as two grids 44).
 constexpr size_t kGridMaxSlice = 4096, kGridMaxSum = 16384;

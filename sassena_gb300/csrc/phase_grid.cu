@@ -22,9 +22,11 @@
 // The grid holds 32-bit integers: shared memory adds integers in place at one access per 32
 // lanes (FP32 adds are a read and a write, whose latency a warp also waits for between atoms), in
 // any order with the same result, and without the bias that small weights take when they are
-// added to a large FP32 sum. The unit is the largest sum a grid can reach over 2^31, so no cell
-// overflows; a grid of 4,096 atoms rounds each weight to 9e-7 of the largest
-// factor (6e-7 rms in A per atom).
+// added to a large FP32 sum. The unit is a power of two above the largest sum a grid can reach over
+// 2^31, so no cell overflows; a grid of 4,096 atoms rounds each weight to at most 1.1e-6 of the largest
+// factor, whatever that is (1e-6 where it is 1), which leaves 2.1e-6 rms in A per atom and unit of that factor at
+// most (1.35e-6 at small shells; tests/test_grid_unit.py). S(q,t) averages it over atoms and
+// directions: 3e-7 of a row, where the direct kernel's FP32 phases leave 3e-7 to 1e-6.
 //
 // Layout. A lane owns one (direction, frame) and a column of the grid in shared memory, [g][lane],
 // so the adds have no bank conflicts. The 32 lanes of a tile are 32 directions of one frame, or
