@@ -301,20 +301,6 @@ int product_of(std::string& m, const double* qv, bool on_device, const std::vect
     return SASS_OK;
 }
 
-// uniform_factors of nq rows of class factors; from the device only where there are classes to tell apart.
-int uniform_of(std::string& m, const SystemState& s, const double* cf, bool on_device, size_t nq, bool& uniform) {
-    std::vector<double> copy;
-    if (on_device) {
-        uniform = false;
-        if (!cf || s.nclass < 2) return SASS_OK;
-        copy.resize(nq * s.nclass);
-        CK(m, cudaMemcpy(copy.data(), cf, copy.size() * sizeof(double), cudaMemcpyDeviceToHost));
-        cf = copy.data();
-    }
-    uniform = uniform_factors(s, cf, nq);
-    return SASS_OK;
-}
-
 void fill_schedule(const EngineStats& s, sass_schedule* out) {
     memset(out, 0, sizeof(*out));
     out->terms = s.terms;
@@ -568,9 +554,7 @@ int sass_compute(sass_plan* p, size_t nq, const size_t* offs, const double* subv
             rc = product_of(p->msg, io_on_device ? d_qv + 3 * offs[i] : subvectors + 3 * offs[i], io_on_device != 0,
                             it.offs, it.lam, it.lam_base, it.umax);
             if (rc) return rc;
-            rc = uniform_of(p->msg, p->sys, io_on_device ? it.lam.empty() ? nullptr : d_cf + nclass * i : class_factors + nclass * i,
-                            io_on_device != 0, j - i, it.uniform);
-            if (rc) return rc;
+            if (!io_on_device) it.uniform = uniform_factors(p->sys, class_factors + nclass * i, j - i);
         }
         it.d_cf = d_cf + nclass * i;
         it.d_fqt = d_fqt + i * nf;
@@ -869,7 +853,7 @@ static std::vector<WorkItem> batch_items(sass_batch* b) {
         it.lam = b->lam[i];
         it.lam_base = b->lam_base[i];
         it.umax = b->umax[i];
-        it.uniform = b->uniform[i] != 0;
+        it.uniform = b->uniform[i];
         it.d_cf = b->cf.as<double>() + b->cf_off[i];
         it.d_fqt = reinterpret_cast<double2*>(b->out.as<double>() + b->fqt_off[i]);
         it.d_fq = reinterpret_cast<double2*>(b->out.as<double>() + b->fq_off[i]);

@@ -318,18 +318,26 @@ int set_system_classes(SystemState& s, const int32_t* cls, bool on_device, cudaS
     std::vector<int32_t> h(s.na_pad, -1);
     if (on_device) ECK(cudaMemcpy(h.data(), cls, s.na * sizeof(int32_t), cudaMemcpyDeviceToHost));
     else memcpy(h.data(), cls, s.na * sizeof(int32_t));
-    for (size_t j = 0; j < s.na; ++j)
-        if (h[j] < 0 || (size_t)h[j] >= s.nclass) {
-            err = "atom " + std::to_string(j) + " has class " + std::to_string(h[j]) + " outside [0," +
-                  std::to_string(s.nclass) + ")";
+    // atoms of each class, four counts in turn: one would wait for its own last store
+    std::vector<uint32_t> count(4 * s.nclass, 0);
+    uint32_t* const n = count.data();
+    const size_t nclass = s.nclass;
+    for (size_t j = 0; j < s.na; ++j) {
+        const int32_t c = h[j];
+        if (c < 0 || (size_t)c >= nclass) {
+            err = "atom " + std::to_string(j) + " has class " + std::to_string(c) + " outside [0," +
+                  std::to_string(nclass) + ")";
             return kErrArg;
         }
+        ++n[4 * (size_t)c + (j & 3)];
+    }
     ECK(s.cls.ensure(s.na_pad * sizeof(int32_t)));
     ECK(cudaMemcpyAsync(s.cls.p, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
     ECK(cudaStreamSynchronize(st));
     s.h_cls.assign(h.begin(), h.begin() + s.na);
-    s.class_atoms.assign(s.nclass, 0);
-    for (int32_t c : s.h_cls) ++s.class_atoms[c];
+    s.class_atoms.resize(s.nclass);
+    for (size_t c = 0; c < s.nclass; ++c)
+        s.class_atoms[c] = (size_t)count[4 * c] + count[4 * c + 1] + count[4 * c + 2] + count[4 * c + 3];
     s.classes_set = true;
     ++s.class_gen;
     s.rec_map_ok = s.rec_ready = s.rec_valid = false;
@@ -520,9 +528,9 @@ void choose_grid(const std::vector<WorkItem>& items, std::vector<char>& on, int&
         for (const GridLanes& g : grid_lanes(nd)) lanes += 1 << g.lgd;
         const double slice = (double)std::min(s.na, kGridMaxSlice);
         const double pad = (double)slots / (double)s.na, transform = nq * G / 1.5;
-        const double further = it.uniform ? 0.0 : (double)(classes - 1) * (2000.0 + 130.0 * nq + transform);
+        const double further = (double)(classes - 1) * (2000.0 + 130.0 * nq + transform) / (double)s.na * lanes / nd;
         const double base = grid_ctas(G, 4) < 3 ? 18.0 : grid_ctas(G, 4) < 4 ? 15.0 : 12.0;
-        const double grid = (base * pad + transform / slice + further / (double)s.na) * lanes / nd;
+        const double one = (base * pad + transform / slice) * lanes / nd;
         const auto runs = arithmetic_runs(it.lam, 3);
         double other = 4.5 * nq;
         if (s.nclass <= (size_t)kRecMaxClass && !runs.empty()) {
@@ -532,7 +540,15 @@ void choose_grid(const std::vector<WorkItem>& items, std::vector<char>& on, int&
                 other += ng * 1.18 * rec_group_cost(K) * pad * std::ceil(ng * nd / 32.0) * 32.0 / (ng * nd) - 4.5 * n;
             }
         }
-        if (grid > 0.9 * other) continue;
+        bool uniform = it.uniform != 0;
+        if (it.uniform < 0 && one <= 0.9 * other && one + further > 0.9 * other) {
+            // factors on the device, and the choice hangs on them: read here, when descriptors are built
+            std::vector<double> cf((size_t)nq * s.nclass);
+            if (cudaMemcpy(cf.data(), it.d_cf, cf.size() * sizeof(double), cudaMemcpyDeviceToHost) == cudaSuccess)
+                uniform = uniform_factors(s, cf.data(), nq);
+            else (void)cudaGetLastError();
+        }
+        if (one + (uniform ? 0.0 : further) > 0.9 * other) continue;
         on[i] = 1;
         any = true;
         if (grid_ctas(grid_shape(it, 1).G, 4) < 4) set = 0;
@@ -660,7 +676,7 @@ static std::vector<uint64_t> prepare_key(const EngineConfig& c, const std::vecto
         for (double l : it.lam) d(l);
         u((uint64_t)(int64_t)it.lam_base);
         d(it.umax);
-        u(it.uniform);
+        u((uint64_t)(int64_t)it.uniform);
         for (const void* q : {(const void*)it.d_qv, (const void*)it.d_cf, (const void*)it.d_fqt,
                               (const void*)it.d_fq, (const void*)it.d_fq2, (const void*)it.d_wsqrt,
                               (const void*)it.d_fqt_w, (const void*)it.d_fq_w, (const void*)it.d_fq2_w,
@@ -1200,10 +1216,10 @@ int Engine::prepare_full(const EngineConfig& cfg, const std::vector<WorkItem>& i
         g.nq = (int)it.lam.size();
         g.G = gs.G;
         g.off = gs.off;
-        g.one_grid = it.uniform || s.nclass < 2;
         g.shell_off = (int)gshells.size();
         for (double l : it.lam) gshells.push_back(l * gs.h * 0.15915494309189533577);
         for (double l : it.lam) gshells.push_back(1.0 / grid_deconvolution(grid_set_, l * gs.h));
+        for (size_t a : s.class_atoms) gshells.push_back((double)a);
         const int nk = (g.nq + kGridShellChunk - 1) / kGridShellChunk * kGridShellChunk;
         const int np = (g.off + 2 + 15) / 16 * 16, sidx = (int)gsys.size();
         grid_table_ = std::max(grid_table_, nk * np);

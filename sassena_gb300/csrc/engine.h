@@ -94,7 +94,7 @@ struct WorkItem {
     std::vector<double> lam;
     int lam_base = -1;
     double umax = 0;  // length of the longest base vector
-    bool uniform = false;          // uniform_factors of d_cf (false also where it is not known: one class)
+    int uniform = -1;              // uniform_factors of d_cf; -1: not known (factors on the device)
     const double* d_cf = nullptr;  // [nq][nclass]
     double2* d_fqt = nullptr;      // [nq][nf]
     double2* d_fq = nullptr;       // [nq]
@@ -145,7 +145,7 @@ void drop_prefetch(SystemState& s);
 bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vector<double>& lam, int& base,
                     double& umax);
 // Whether the gridded sum can weight the atoms of `s` by class factors cf [nq][nclass] (host) and so take
-// all classes in one grid: the same at all shells, finite, within 16 of each other, and the largest at
+// all classes in one grid, as grid_tables_kernel decides: the same at all shells, finite, within 16 of each other, and the largest at
 // most 4 times the root of their mean square over the atoms, since a weight is rounded to a fraction of
 // the largest (one atom of 16 among 4,000 of 1, 20 directions: S(q) off by 2e-6 rms, 3e-7 by class).
 bool uniform_factors(const SystemState& s, const double* cf, size_t nq);

@@ -214,8 +214,7 @@ struct GridSystem {
     int* konst;
     int na_rec, nf, nd, nclass, nq;
     int G, off;               // grid points; the point of projection 0
-    int one_grid;             // the class factors may weight the atoms (uniform_factors)
-    int shell_off;            // of the system's [2][nq] shell constants
+    int shell_off;            // of the system's [2][nq] shell constants and [nclass] atoms of each class
     int slice_atoms;          // most atoms summed in one grid (a multiple of 32)
 };
 
@@ -246,7 +245,7 @@ constexpr double kGridSigma[2] = {3.0, 4.0};  // grid points per half period at 
 // D(l) of the weights `set`; CTAs per SM for that many grid points and staged frames (0: too many)
 double grid_deconvolution(int set, double l);
 int grid_ctas(int grid_points, int ring_frames);
-// shells: per system [nq] lam_k h / 2 pi, then [nq] 1 / D(lam_k h)
+// shells: per system [nq] lam_k h / 2 pi, then [nq] 1 / D(lam_k h), then [nclass] atoms
 cudaError_t launch_grid_tables(const GridSystem* systems, int nsys, int max_points, const double* shells,
                                cudaStream_t st);
 cudaError_t launch_phase_grid(GridLaunch a, int grid_points, int ring_frames, cudaStream_t st);

@@ -282,9 +282,8 @@ __global__ void __launch_bounds__(kGridWarps * 32, 4) phase_grid_kernel(const Gr
 }
 
 // Per system: the transform table exp(i lam_k h g) / D, whether the class factors weight the atoms
-// (then a slice is summed once), as uniform_factors decides on the host, and the same at all shells
-// and finite (one class: its factor is read here alone); the atoms' weights per class in grid
-// units, the unit itself (gw[nclass]) and the factors per class and shell.
+// (then a slice is summed once; uniform_factors is the same rule, with its reasons); the atoms'
+// weights per class in grid units, the unit itself (gw[nclass]) and the factors per class and shell.
 __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const double* __restrict__ shells) {
     const GridSystem s = systems[blockIdx.y];
     const int nk = (s.nq + kGridChunk - 1) / kGridChunk * kGridChunk;
@@ -306,9 +305,11 @@ __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const
     }
     if (blockIdx.x == 0) {
         __shared__ int differs;
-        __shared__ unsigned hi;  // largest |factor| of the atoms' classes, as bits
+        __shared__ unsigned lo, hi;  // smallest and largest |factor| of the atoms' classes, as bits
+        __shared__ double sum, count;  // of their squares over the atoms; atoms
         if (threadIdx.x == 0) {
             differs = 0;
+            lo = 0x7f800000u;
             hi = 0u;
         }
         __syncthreads();
@@ -318,13 +319,32 @@ __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const
             s.facs[(size_t)c * s.nq + i / s.nclass] = b;
             if (!(b == b0) || isinf(b)) differs = 1;
         }
-        for (int i = threadIdx.x; i < s.na_rec / 32; i += blockDim.x) {
-            const unsigned b = __float_as_uint(fabsf((float)s.cf[s.block_class[i] & 0xffff]));
-            if (b) atomicMax(&hi, b);
+        if (threadIdx.x < 32) {
+            const double* atoms = lam + 2 * s.nq;
+            double sq = 0.0, n = 0.0;
+            for (int c = threadIdx.x; c < s.nclass; c += 32) {
+                if (atoms[c] == 0.0) continue;
+                const float b = fabsf((float)s.cf[c]);
+                n += atoms[c];
+                sq = fma(atoms[c], (double)b * (double)b, sq);
+                if (b != 0.f) {
+                    atomicMin(&lo, __float_as_uint(b));
+                    atomicMax(&hi, __float_as_uint(b));
+                }
+            }
+            for (int o = 16; o; o >>= 1) {
+                sq += __shfl_xor_sync(0xffffffffu, sq, o);
+                n += __shfl_xor_sync(0xffffffffu, n, o);
+            }
+            if (threadIdx.x == 0) {
+                sum = sq;
+                count = n;
+            }
         }
         __syncthreads();
         const float bmax = hi ? __uint_as_float(hi) : 1.f;
-        const int konst = s.one_grid && !differs;
+        const int konst = !differs && (!hi || (bmax <= 16.f * __uint_as_float(lo) &&
+                                               (double)bmax * (double)bmax * count <= 16.0 * sum));
         // units per weight of 1: no sum of slice_atoms atoms reaches 2^31, no weight 2^22
         // times a power of two, so that the factors' products with it are exact: a rounding of
         // the scale is common to all atoms and counts four times in fq2
