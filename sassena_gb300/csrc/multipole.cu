@@ -429,9 +429,11 @@ __device__ void cyl_bessel_row(int N, double x, double* out, size_t stride, cons
 // 500 atoms, the moment (12, 12) alone: 5e-6 of S(q, 0)), a class of factor 0 that holds the large
 // Bessel functions, the sine moments of atoms in one half plane. So the amplitudes of each (frame, q),
 // over all the moments asked for, are compared with the error expected of them, and where it is more
-// than 2^-47 of their norm the frame's angular functions are written as FP64 numbers and the sums taken
-// of those. One cluster of kRedoCtas CTAs a frame tests it and, where needed, does both. Ordinary calls have
-// none: 64 frames, 10 q, 441 moments 2.500 ms without the test, 2.504 so (2.53 with the three steps
+// than 2^-44 of their norm the frame's angular functions are written as FP64 numbers and the sums taken
+// of those. (The expectation takes the bounds as reached and is some eight times what comes out: single
+// moments of 100,000 atoms that pass it differ by 1.6e-14 of S(q, 0) from the FP64 sums, all 441 by 1.4e-15.
+// At 2^-47 a third of the frames of such a system would be summed again.)
+// One cluster of kRedoCtas CTAs a frame tests it and, where needed, does both. Ordinary calls have none: 64 frames, 10 q, 441 moments 2.500 ms without the test, 2.504 so (2.53 with the three steps
 // as kernels of their own). Of a column of 5,000 atoms, the 182 moments of |m| >= 8 are all summed again:
 // 1.7 ms without, 4.4 so, 5.9 with FP64 sums alone.
 constexpr int kRedoCtas = 8;
@@ -446,10 +448,13 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// One warp: the norm of the moments A[k * stride] against their expected error, 2^(e - 57) for each atom of
-// each moment, 2^e the largest product of two rows' bounds (a lane's share of the rows in `e`).
-// Amplitudes that are not finite stay so.
-__device__ __forceinline__ void mp_judge(const MpRedo& r, int fl, int q, int e, const double2* A, size_t stride,
+// 4^e, e kept where it and sums of it are FP64 numbers
+__device__ __forceinline__ double mp_pow4(int e) { return __hiloint2double((2 * min(max(e, -500), 500) + 1023) << 20, 0); }
+
+// One warp: the norm of the moments A[k * stride] against their expected error. `err2` is a lane's share of
+// the sum over moments of 4^e, 2^e the product of their rows' bounds, of which each atom's term is off by
+// 2^-57. Amplitudes that are not finite stay so.
+__device__ __forceinline__ void mp_judge(const MpRedo& r, int fl, int q, double err2, const double2* A, size_t stride,
                                          int nmom, int na) {
     const int lane = threadIdx.x & 31;
     double sum2 = 0.0;
@@ -458,11 +463,12 @@ __device__ __forceinline__ void mp_judge(const MpRedo& r, int fl, int q, int e, 
         const double2 v = A[k * stride];
         sum2 = fma(v.x, v.x, fma(v.y, v.y, sum2));
     }
-    for (int o = 16; o; o >>= 1) sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
-    e = __reduce_max_sync(0xffffffffu, e);
+    for (int o = 16; o; o >>= 1) {
+        sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
+        err2 += __shfl_xor_sync(0xffffffffu, err2, o);
+    }
     if (lane) return;
-    const double u = __hiloint2double((min(max(e - 57 + 47, -1022), 1024) + 1023) << 20, 0);  // 2^(e - 10)
-    const unsigned redo = u * u * nmom * na > sum2;
+    const unsigned redo = err2 * na > 67108864.0 * sum2;  // 4^(57 - 44)
     *r.at(fl, q) = redo;
     if (redo) atomicOr(r.at(fl, r.nq), 1u);
 }
@@ -721,12 +727,12 @@ __global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(kSumWarps * 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int q = w0; q < a.nq; q += wn) {
         const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q) * (a.L + 1);
-        int e = -4096;
+        double err2 = 0.0;
         for (int k = lane; k < a.npair; k += 32) {
-            const int l = a.pl[k];
-            e = max(e, mp_exponent(mx[l]) + 3 + (33 - __clz(2 * l + 1)) / 2);
+            const int l = a.pl[k], e = mp_exponent(mx[l]) + 3 + (33 - __clz(2 * l + 1)) / 2;
+            err2 = fma(mp_pow4(e), (double)(a.pmom[k + 1] - a.pmom[k]), err2);
         }
-        mp_judge(a.redo, fl, q, e, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
+        mp_judge(a.redo, fl, q, err2, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
     }
     cluster_barrier();
     if (*reinterpret_cast<volatile unsigned*>(a.redo.at(fl, a.nq)) == 0u) return;  // the same for the whole cluster
@@ -1028,9 +1034,10 @@ __global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(kSumWarps * 
     for (int q = w0; q < a.nq; q += wn) {
         const unsigned* mx = a.jmax + ((size_t)fl * a.nq + q) * (a.N + 3);
         const int xe = mp_exponent(max(mx[a.N + 1], mx[a.N + 2]));
-        int e = -4096;
-        for (int k = lane; k < a.nn; k += 32) e = max(e, mp_exponent(mx[a.ns[k]]) + xe + 2);
-        mp_judge(a.redo, fl, q, e, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
+        double err2 = 0.0;
+        for (int k = lane; k < a.nn; k += 32)
+            err2 = fma(mp_pow4(mp_exponent(mx[a.ns[k]]) + xe + 2), (double)(a.nmom0[k + 1] - a.nmom0[k]), err2);
+        mp_judge(a.redo, fl, q, err2, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
     }
     cluster_barrier();
     if (*reinterpret_cast<volatile unsigned*>(a.redo.at(fl, a.nq)) == 0u) return;  // the same for the whole cluster
