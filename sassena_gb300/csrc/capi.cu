@@ -554,7 +554,7 @@ int sass_compute(sass_plan* p, size_t nq, const size_t* offs, const double* subv
             rc = product_of(p->msg, io_on_device ? d_qv + 3 * offs[i] : subvectors + 3 * offs[i], io_on_device != 0,
                             it.offs, it.lam, it.lam_base, it.umax);
             if (rc) return rc;
-            if (!io_on_device) it.uniform = uniform_factors(p->sys, class_factors + nclass * i, j - i);
+            if (!io_on_device && !it.lam.empty()) it.uniform = uniform_factors(p->sys, class_factors + nclass * i, j - i);
         }
         it.d_cf = d_cf + nclass * i;
         it.d_fqt = d_fqt + i * nf;
@@ -641,7 +641,7 @@ int sass_autotune(sass_plan* p, size_t nq, const size_t* offs, const double* sub
         rc = product_of(p->msg, subvectors, false, items[0].offs, items[0].lam, items[0].lam_base,
                         items[0].umax);
         if (rc) return rc;
-        items[0].uniform = uniform_factors(p->sys, class_factors, nq);
+        if (!items[0].lam.empty()) items[0].uniform = uniform_factors(p->sys, class_factors, nq);
     }
     TuneChoice best;
     double ms = 0;

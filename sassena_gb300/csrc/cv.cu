@@ -312,7 +312,7 @@ int sass_compute_cv(sass_plan* p, sass_mlp* net, size_t nq, const double* qlen, 
         it.d_qv = p->qv.as<double>() + 3 * first;
         if (p->d.precision == SASS_PRECISION_FP32 && p->rec_k >= 0)
             detect_product(sv.data() + 3 * first, it.offs, it.lam, it.lam_base, it.umax);
-        it.uniform = uniform_factors(p->sys, class_factors, nq);
+        if (!it.lam.empty()) it.uniform = uniform_factors(p->sys, class_factors, nq);
         it.d_cf = p->cf.as<double>();
         it.d_fqt = o + row * nf;
         it.d_fq = o + ne * nf + row;

@@ -396,10 +396,12 @@ bool detect_product(const double* qv, const std::vector<size_t>& offs, std::vect
 bool uniform_factors(const SystemState& s, const double* cf, size_t nq) {
     float lo = INFINITY, hi = 0.f;
     double sum = 0;
+    for (size_t k = 0; k < nq; ++k)
+        for (size_t c = 0; c < s.nclass; ++c)
+            if (!((float)cf[k * s.nclass + c] == (float)cf[c])) return false;
     for (size_t c = 0; c < s.nclass; ++c) {
         const float b0 = (float)cf[c];
-        for (size_t k = 0; k < nq; ++k)
-            if (!((float)cf[k * s.nclass + c] == b0) || std::isinf(b0)) return false;
+        if (std::isinf(b0)) return false;
         if (s.class_atoms[c] && b0 != 0.f) {
             lo = std::min(lo, std::fabs(b0));
             hi = std::max(hi, std::fabs(b0));
@@ -527,7 +529,8 @@ void choose_grid(const std::vector<WorkItem>& items, std::vector<char>& on, int&
         double lanes = 0;
         for (const GridLanes& g : grid_lanes(nd)) lanes += 1 << g.lgd;
         const double slice = (double)std::min(s.na, kGridMaxSlice);
-        const double pad = (double)slots / (double)s.na, transform = nq * G / 1.5;
+        // padding of up to a tenth is in the costs as measured
+        const double pad = 10 * slots > 11 * s.na_pad ? (double)slots / (double)s.na : 1.0, transform = nq * G / 1.5;
         const double further = (double)(classes - 1) * (2000.0 + 130.0 * nq + transform) / (double)s.na * lanes / nd;
         const double base = grid_ctas(G, 4) < 3 ? 18.0 : grid_ctas(G, 4) < 4 ? 15.0 : 12.0;
         const double one = (base * pad + transform / slice) * lanes / nd;

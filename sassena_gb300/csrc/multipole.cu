@@ -454,7 +454,7 @@ __device__ __forceinline__ double mp_pow4(int e) { return __hiloint2double((2 * 
 // One warp: the norm of the moments A[k * stride] against their expected error. `err2` is a lane's share of
 // the sum over moments of 4^e, 2^e the product of their rows' bounds, of which each atom's term is off by
 // 2^-57. Amplitudes that are not finite stay so.
-__device__ __forceinline__ void mp_judge(const MpRedo& r, int fl, int q, double err2, const double2* A, size_t stride,
+__device__ __forceinline__ void mp_decide(const MpRedo& r, int fl, int q, double err2, const double2* A, size_t stride,
                                          int nmom, int na) {
     const int lane = threadIdx.x & 31;
     double sum2 = 0.0;
@@ -732,7 +732,7 @@ __global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(kSumWarps * 
             const int l = a.pl[k], e = mp_exponent(mx[l]) + 3 + (33 - __clz(2 * l + 1)) / 2;
             err2 = fma(mp_pow4(e), (double)(a.pmom[k + 1] - a.pmom[k]), err2);
         }
-        mp_judge(a.redo, fl, q, err2, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
+        mp_decide(a.redo, fl, q, err2, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
     }
     cluster_barrier();
     if (*reinterpret_cast<volatile unsigned*>(a.redo.at(fl, a.nq)) == 0u) return;  // the same for the whole cluster
@@ -895,8 +895,8 @@ constexpr double kMpSqrt2Pi = 2.50662827463100050242;
 // as mp_sphere_sum_kernel sums: a lane is an atom, a warp an order (or a part of one's atoms). The
 // tile's X words are shared; J and the angles are read once, straight from memory. X J is one
 // 58-bit product more, taken before the four sums' (18 of the 32-bit multiplications per J, 12 of
-// them in the sums). 5,000 atoms, 64 frames, 10 q, 41 orders: 8.0 ms with the basis before, 2.8 now
-// (1.0 here, 1.6 the Bessel rows).
+// them in the sums). 5,000 atoms, 64 frames, 10 q, 41 orders: 8.0 ms with the basis before, 2.7 now
+// (1.0 here, 1.5 the Bessel rows).
 template <int QB>
 __global__ void __launch_bounds__(kSumWarps * 32, 2) mp_cylinder_sum_kernel(MpCylinder a) {
     __shared__ int4 Xs[QB][kSumTile];
@@ -1037,7 +1037,7 @@ __global__ void __cluster_dims__(kRedoCtas, 1, 1) __launch_bounds__(kSumWarps * 
         double err2 = 0.0;
         for (int k = lane; k < a.nn; k += 32)
             err2 = fma(mp_pow4(mp_exponent(mx[a.ns[k]]) + xe + 2), (double)(a.nmom0[k + 1] - a.nmom0[k]), err2);
-        mp_judge(a.redo, fl, q, err2, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
+        mp_decide(a.redo, fl, q, err2, a.A + (size_t)q * a.nmom * a.nf + a.f0 + fl, a.nf, a.nmom, a.na);
     }
     cluster_barrier();
     if (*reinterpret_cast<volatile unsigned*>(a.redo.at(fl, a.nq)) == 0u) return;  // the same for the whole cluster

@@ -305,46 +305,47 @@ __global__ void grid_tables_kernel(const GridSystem* __restrict__ systems, const
     }
     if (blockIdx.x == 0) {
         __shared__ int differs;
-        __shared__ unsigned lo, hi;  // smallest and largest |factor| of the atoms' classes, as bits
+        __shared__ float lo, hi;       // smallest and largest |factor| of the atoms' classes
         __shared__ double sum, count;  // of their squares over the atoms; atoms
-        if (threadIdx.x == 0) {
-            differs = 0;
-            lo = 0x7f800000u;
-            hi = 0u;
-        }
+        if (threadIdx.x == 0) differs = 0;
         __syncthreads();
-        for (int i = threadIdx.x; i < s.nq * s.nclass; i += blockDim.x) {
-            const int c = i % s.nclass;
-            const float b = (float)s.cf[i], b0 = (float)s.cf[c];
-            s.facs[(size_t)c * s.nq + i / s.nclass] = b;
-            if (!(b == b0) || isinf(b)) differs = 1;
-        }
-        if (threadIdx.x < 32) {
+        if (threadIdx.x >= 32) {
+            for (int i = threadIdx.x - 32; i < s.nq * s.nclass; i += blockDim.x - 32) {
+                const int c = i % s.nclass;
+                const float b = (float)s.cf[i], b0 = (float)s.cf[c];
+                s.facs[(size_t)c * s.nq + i / s.nclass] = b;
+                if (!(b == b0) || isinf(b)) differs = 1;
+            }
+        } else {
             const double* atoms = lam + 2 * s.nq;
             double sq = 0.0, n = 0.0;
+            unsigned mn = 0x7f800000u, mx = 0u;
             for (int c = threadIdx.x; c < s.nclass; c += 32) {
-                if (atoms[c] == 0.0) continue;
-                const float b = fabsf((float)s.cf[c]);
-                n += atoms[c];
-                sq = fma(atoms[c], (double)b * (double)b, sq);
+                const double na = atoms[c];
+                const float b = na > 0.0 ? fabsf((float)s.cf[c]) : 0.f;
+                n += na;
+                sq = fma(na, (double)b * (double)b, sq);
                 if (b != 0.f) {
-                    atomicMin(&lo, __float_as_uint(b));
-                    atomicMax(&hi, __float_as_uint(b));
+                    mn = min(mn, __float_as_uint(b));
+                    mx = max(mx, __float_as_uint(b));
                 }
             }
+            mn = __reduce_min_sync(0xffffffffu, mn);
+            mx = __reduce_max_sync(0xffffffffu, mx);
             for (int o = 16; o; o >>= 1) {
                 sq += __shfl_xor_sync(0xffffffffu, sq, o);
                 n += __shfl_xor_sync(0xffffffffu, n, o);
             }
             if (threadIdx.x == 0) {
+                lo = __uint_as_float(mn);
+                hi = __uint_as_float(mx);
                 sum = sq;
                 count = n;
             }
         }
         __syncthreads();
-        const float bmax = hi ? __uint_as_float(hi) : 1.f;
-        const int konst = !differs && (!hi || (bmax <= 16.f * __uint_as_float(lo) &&
-                                               (double)bmax * (double)bmax * count <= 16.0 * sum));
+        const float bmax = hi != 0.f ? hi : 1.f;
+        const int konst = !differs && (hi == 0.f || (bmax <= 16.f * lo && (double)bmax * (double)bmax * count <= 16.0 * sum));
         // units per weight of 1: no sum of slice_atoms atoms reaches 2^31, no weight 2^22
         // times a power of two, so that the factors' products with it are exact: a rounding of
         // the scale is common to all atoms and counts four times in fq2
