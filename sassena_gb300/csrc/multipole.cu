@@ -1385,12 +1385,13 @@ extern "C" int sass_multipole_compute(sass_plan* p, int type, size_t nq, const d
         // as many q-vectors at a time as the basis of one frame has room for (all, but for very
         // large systems)
         const size_t per_q = na_pad * (N + 3) * sizeof(double), angles = na_pad * nn * sizeof(int4);
-        // The basis stays with the plan, so no more of it than fills the GPU: 2 GiB, frames in even parts
-        // (5,000 atoms, 512 frames, 10 q, 41 orders: 10 GB 20.3 ms, 2 GiB 20.5)
-        const size_t cap = std::min(budget, (size_t)2 << 30);
+        // The basis stays with the plan, so no more of it than fills the GPU: 4 GiB, frames in even parts, each
+        // of which costs about 0.2 ms of its kernels' ends (10,000 atoms, 1,024 frames, 20 q, 41 orders: 16 GB
+        // 148 ms, 4 GiB 151, 2 GiB 157; as many frames as make whole waves of the contraction's CTAs: no gain)
+        const size_t cap = std::min(budget, (size_t)4 << 30);
         const size_t nqm = std::max<size_t>(1, std::min<size_t>(nq, cap > angles ? (cap - angles) / per_q : 1));
         const size_t most = std::max<size_t>(1, std::min<size_t>({nf, cap / (nqm * per_q + angles), (size_t)65535}));  // grid y
-        const size_t nfb = (nf + (nf + most - 1) / most - 1) / ((nf + most - 1) / most);
+        const size_t parts = (nf + most - 1) / most, nfb = (nf + parts - 1) / parts;
         MCK(p->mp_Jb.ensure(nfb * nqm * per_q));
         MCK(p->mp_Yc.ensure(nfb * angles));
         MCK(p->mp_ycf.ensure(nfb * (nqm * (N + 4) + 1) * sizeof(unsigned)));  // jmax and the redo words
