@@ -231,7 +231,8 @@ int sass_frame_center(const sass_plan* plan, double* center3);
  * exp(i q_k u.r) from shell to shell with a three-term recurrence: two reduced sin/cos
  * pairs per atom for up to `shells_per_lane` shells. 0 = automatic (default): the gridded
  * kernel where the shells share a direction set, at any spacing, and it costs less, else the
- * recurrence; -1 = off (neither); else one of 4, 8, 12, 16, 20, 24, 32 (the recurrence alone).
+ * recurrence (and the direct kernel where their class-sorted copy of the frames finds no
+ * memory); -1 = off (neither); else one of 4, 8, 12, 16, 20, 24, 32 (the recurrence alone).
  * FP64 plans ignore it. */
 int sass_set_shell_recurrence(sass_plan* plan, int shells_per_lane);
 
