@@ -4,7 +4,10 @@ alone, which the transforms' (times NF / (NF - tau)) does not meet."""
 import numpy as np
 import pytest
 
+import oracle
 from sassena_gb300 import abi, synth
+
+from test_gpu_multipole import case, check
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +38,11 @@ def test_last_lags(native_lib, nf, nm, method, precision, bar):
     w = synth.small("all", "autocorrelate", seed=nf, na=40, nf=nf, nq=2, nm=nm)
     got, lags = products(w, precision, method)
     assert (np.abs(got[:, -8:] - lags).max(axis=1) <= bar * np.abs(got[:, 0])).all()
+
+
+@pytest.mark.parametrize("kind", ["sphere", "cylinder"])
+@pytest.mark.parametrize("method", ["fftw", "direct"])
+def test_last_lags_of_multipole_amplitudes(native_lib, kind, method):
+    w, q = case(7, na=30, nf=150, nq=2)
+    moments = oracle.sphere_moments(4) if kind == "sphere" else oracle.cylinder_moments(4)
+    check(w, q, kind, moments, method=method)
